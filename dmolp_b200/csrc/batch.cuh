@@ -25,6 +25,8 @@ struct Inst {
     int64_t narcs;   // arcs of the instance
     int32_t nv, k;
     int32_t maxdeg, ibits, dbits, symmetric;
+    int64_t cbase;    // its first kept label count
+    int32_t cstride;  // 16-bit counts per vertex (min(k, 32) rounded up to 8); 0 = no kept counts
 };
 
 struct Out {
@@ -37,7 +39,9 @@ struct Args {
     const int32_t *col;
     int32_t *label, *newlab, *cstamp;
     int32_t *ndiff;  // neighbours with another label, exact at every iteration start
-    int32_t *l_cand, *l_bnd, *l_act, *l_win0, *l_win1;  // per-instance slices at vbase
+    int32_t *l_bnd, *l_win0, *l_win1;  // per-instance slices at vbase
+    uint64_t *rec0, *rec1;             // selection records, per-instance slices at vbase
+    uint16_t *cnt;                     // kept label counts, per-instance slices at cbase
     const Inst *inst;
     const int32_t *order;
     int ninst;
@@ -73,27 +77,102 @@ struct P1Args {
     const int32_t *col;
     int32_t *label;
     const Inst *inst;
-    const int32_t *order;
-    int ninst;
     int *next;
-    const int32_t *hubs;       // per graph, local ids in the reference's hub order
-    const int64_t *hstart;     // [ninst + 1]
-    const int32_t *first;      // [ninst] first seed (local id)
-    const int32_t *first_hub;  // [ninst] its index in the graph's hub list, or -1
-    uint8_t *hub_used, *cov, *seedm, *sel;
+    const int32_t *hubs;    // per graph, local ids in the reference's hub order (descending degree)
+    const int64_t *hstart;  // [ninst + 1]
+    const int32_t *first;   // [ninst] first seed (local id)
+    uint8_t *cov;
     int32_t *claim;
-    int32_t *l_front0, *l_front1, *l_claim, *l_act0, *l_act1;  // per-graph slices at vbase
-    int32_t *seeds_out;                                        // [ninst][kBatchMaxK]
+    int32_t *l_front0, *l_front1, *l_sel;  // per-graph slices at vbase
+    uint64_t *rec0, *rec1;                 // selection records, per-graph slices at vbase
+    int32_t *seeds_out;                    // [ninst][kBatchMaxK]
     P1Out *out;
-    const uint8_t *only;  // [ninst] or null: run only the graphs flagged 1
     int theta;
 };
 
-void launch_p1(const P1Args &a, int grid, cudaStream_t s);
+// Teams: the batch's graphs, in `order` (largest first), are run by clusters of 16, 8, 4 and 2 CTAs and by
+// single CTAs; n[j] graphs by teams of kMaxTeam >> j.
+constexpr int kMaxTeam = 16;
+constexpr int kTeamClasses = 5;
+struct TeamPlan {
+    int n[kTeamClasses];
+};
+
+// Side streams on which the classes of a plan run next to each other (the plan's first class runs on the
+// stream itself): open() makes them wait for what is on the stream, close() makes the stream wait for them.
+struct Fork {
+    cudaStream_t side[kTeamClasses - 1];
+    cudaEvent_t begin, end[kTeamClasses - 1];
+    static int lead(const TeamPlan &p) {
+        int j = 0;
+        while (j < kTeamClasses - 1 && p.n[j] == 0) ++j;
+        return j;
+    }
+    cudaStream_t stream(const TeamPlan &p, int j, cudaStream_t s) const { return j == lead(p) ? s : side[j - 1]; }
+    void open(const TeamPlan &p, cudaStream_t s) const {
+        bool first = true;
+        for (int j = lead(p) + 1; j < kTeamClasses; ++j) {
+            if (p.n[j] == 0) continue;
+            if (first) cudaEventRecord(begin, s);
+            first = false;
+            cudaStreamWaitEvent(side[j - 1], begin, 0);
+        }
+    }
+    void close(const TeamPlan &p, cudaStream_t s) const {
+        for (int j = lead(p) + 1; j < kTeamClasses; ++j) {
+            if (p.n[j] == 0) continue;
+            cudaEventRecord(end[j - 1], side[j - 1]);
+            cudaStreamWaitEvent(s, end[j - 1], 0);
+        }
+    }
+};
+
+// Whether clusters of c CTAs of the kernel can run, and how many at once.
+template <typename K>
+bool max_clusters(K kernel, int c, int nt, int *n) {
+    if (c > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)c;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)c);
+    cfg.blockDim = dim3((unsigned)nt);
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(n, kernel, &cfg) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
+// n clusters of c CTAs (max_clusters has been asked for this kernel and c).
+template <typename K, typename... A>
+cudaError_t launch_cluster(K kernel, int n, int c, int nt, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)c;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(n * c));
+    cfg.blockDim = dim3((unsigned)nt);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+int p1_threads();
+int p1_max_team();
+void launch_p1(const P1Args &a, const int32_t *order, int grid, const TeamPlan &plan, const Fork &f, cudaStream_t s);
 
 int occupancy(int nt, int td);
-bool launch(const Args &a, int nt, int td, int grid, cudaStream_t s);
-void prepare(const int64_t *off, int32_t *col, Inst *inst, int ninst, int *next, int *err, int grid, cudaStream_t s);
+int max_team(int nt, int td);  // the largest cluster the device can run, 1 if none
+bool launch(const Args &a, int nt, int td, int grid, const TeamPlan &plan, const Fork &f, cudaStream_t s);
+void prepare(const int64_t *off, int32_t *col, Inst *inst, int ninst, int64_t nv, int64_t narcs, int *err, int grid,
+             cudaStream_t s);
 
 }  // namespace batch
 }  // namespace dmolp

@@ -23,6 +23,7 @@ struct dmolp_batch {
     int device = 0, num_sms = 148;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    Fork fork{};
     bool has_graph = false;
     int ninst = 0;
     int64_t nv = 0, narcs = 0;
@@ -32,6 +33,7 @@ struct dmolp_batch {
     int32_t *order = nullptr, *saved = nullptr;
     int *err = nullptr;
     std::vector<Inst> h_inst;
+    std::vector<int32_t> h_order;
     std::vector<Out> h_out;
     std::vector<long long> h_counts;
     bool tuned = false;
@@ -42,7 +44,7 @@ struct dmolp_batch {
     std::vector<int64_t> h_vstart;
     bool have_hubs = false;
     P1Args p1{};
-    uint8_t *p1_only = nullptr;
+    int32_t *p1_order = nullptr;  // the flagged graphs of a masked run, largest first
     std::vector<P1Out> h_p1;
 };
 
@@ -100,6 +102,30 @@ int bsync(dmolp_batch *b) {
         if (r_) return r_;   \
     } while (0)
 
+// How many CTAs work on each graph of `order` (largest first): with `slots` CTAs resident at once, a graph deserves its share of the
+// batch's work (arcs + vertices) of them, rounded down to a power of two, up again above 1.4 times that, and at
+// most one CTA per nt vertices (a thread with less than a vertex only adds barriers).  So a batch of thousands
+// of like graphs runs one CTA per graph, and a small batch, or a graph far larger than the others, spreads
+// over the chip.
+TeamPlan team_sizes(const std::vector<Inst> &inst, const std::vector<int32_t> &order, int slots, int nt, int most) {
+    TeamPlan plan{};
+    double total = 0;
+    for (int32_t i : order) total += (double)(inst[i].narcs + inst[i].nv);
+    int last = most;  // the order is by work: team sizes never grow along it
+    for (int32_t i : order) {
+        const Inst &I = inst[i];
+        const double share = total > 0 ? (double)(I.narcs + I.nv) * slots / total : 1.0;
+        int c = 1, j = kTeamClasses - 1;
+        while (2 * c <= last && share > 1.4 * c && (int64_t)I.nv > (int64_t)c * nt) {
+            c *= 2;
+            --j;
+        }
+        last = c;
+        ++plan.n[j];
+    }
+    return plan;
+}
+
 // Capture (once per shape and configuration) and launch the batch.
 int run_graph(dmolp_batch *b, const dmolp_batch_tuning &t, const dmolp_lp_config &cfg) {
     const int occ = occupancy(t.block_threads, t.thread_row_max);
@@ -114,9 +140,11 @@ int run_graph(dmolp_batch *b, const dmolp_batch_tuning &t, const dmolp_lp_config
         a.mode = cfg.mode;
         a.iters = cfg.iterations;
         a.cap = cfg.cap;
+        const TeamPlan plan = team_sizes(b->h_inst, b->h_order, b->num_sms * bps, t.block_threads,
+                                         max_team(t.block_threads, t.thread_row_max));
         cudaGraph_t g = nullptr;
         BCUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-        const bool ok = launch(a, t.block_threads, t.thread_row_max, grid, b->stream);
+        const bool ok = launch(a, t.block_threads, t.thread_row_max, grid, plan, b->fork, b->stream);
         cudaError_t e = cudaStreamEndCapture(b->stream, &g);
         if (!ok) {
             if (g) cudaGraphDestroy(g);
@@ -197,9 +225,14 @@ int dmolp_batch_create(int device, dmolp_batch **out) {
     dmolp_batch *b = new dmolp_batch();
     b->device = device;
     cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, device);
-    if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess) {
-        delete b;
+    bool ok = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) == cudaSuccess &&
+              cudaEventCreate(&b->ev0) == cudaSuccess && cudaEventCreate(&b->ev1) == cudaSuccess &&
+              cudaEventCreateWithFlags(&b->fork.begin, cudaEventDisableTiming) == cudaSuccess;
+    for (int j = 0; j < kTeamClasses - 1 && ok; ++j)
+        ok = cudaStreamCreateWithFlags(&b->fork.side[j], cudaStreamNonBlocking) == cudaSuccess &&
+             cudaEventCreateWithFlags(&b->fork.end[j], cudaEventDisableTiming) == cudaSuccess;
+    if (!ok) {
+        dmolp_batch_destroy(b);
         return fail(DMOLP_ERR_CUDA, "stream / event creation failed");
     }
     *out = b;
@@ -209,11 +242,16 @@ int dmolp_batch_create(int device, dmolp_batch **out) {
 int dmolp_batch_destroy(dmolp_batch *b) {
     if (!b) return DMOLP_OK;
     cudaSetDevice(b->device);
-    cudaStreamSynchronize(b->stream);
+    if (b->stream) cudaStreamSynchronize(b->stream);
     free_all(b);
-    cudaEventDestroy(b->ev0);
-    cudaEventDestroy(b->ev1);
-    cudaStreamDestroy(b->stream);
+    for (int j = 0; j < kTeamClasses - 1; ++j) {
+        if (b->fork.end[j]) cudaEventDestroy(b->fork.end[j]);
+        if (b->fork.side[j]) cudaStreamDestroy(b->fork.side[j]);
+    }
+    if (b->fork.begin) cudaEventDestroy(b->fork.begin);
+    if (b->ev0) cudaEventDestroy(b->ev0);
+    if (b->ev1) cudaEventDestroy(b->ev1);
+    if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return DMOLP_OK;
 }
@@ -240,9 +278,11 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
     BCUDA(cudaStreamSynchronize(b->stream));
     free_all(b);
     Args &a = b->a;
-    int32_t *label = nullptr, *newlab = nullptr, *cstamp = nullptr, *ndiff = nullptr, *lc = nullptr, *lb = nullptr, *la = nullptr,
-            *w0 = nullptr, *w1 = nullptr, *col = nullptr, *order = nullptr, *saved = nullptr;
+    int32_t *label = nullptr, *newlab = nullptr, *cstamp = nullptr, *ndiff = nullptr, *lb = nullptr, *w0 = nullptr, *w1 = nullptr,
+            *col = nullptr, *order = nullptr, *saved = nullptr;
     int64_t *off = nullptr;
+    uint64_t *rec0 = nullptr, *rec1 = nullptr;
+    uint16_t *cnt = nullptr;
     Inst *inst = nullptr;
     Out *out = nullptr;
     long long *counts = nullptr;
@@ -254,12 +294,12 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
     BTRY(balloc(b, &newlab, nv));
     BTRY(balloc(b, &cstamp, nv));
     BTRY(balloc(b, &ndiff, nv));
-    BTRY(balloc(b, &lc, nv));
     BTRY(balloc(b, &lb, nv));
-    BTRY(balloc(b, &la, nv));
     BTRY(balloc(b, &w0, nv));
     BTRY(balloc(b, &w1, nv));
     BTRY(balloc(b, &saved, nv));
+    BTRY(balloc(b, &rec0, nv));
+    BTRY(balloc(b, &rec1, nv));
     BTRY(balloc(b, &inst, ninst));
     BTRY(balloc(b, &order, ninst));
     BTRY(balloc(b, &out, ninst));
@@ -267,12 +307,10 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
     BTRY(balloc(b, &lt, kMaxIter + 1));
     BTRY(balloc(b, &rt, kMaxIter + 1));
     BTRY(balloc(b, &ctr, 4));
-    uint8_t *cov = nullptr, *seedm = nullptr, *selm = nullptr;
+    uint8_t *cov = nullptr;
     int32_t *claim = nullptr, *seeds_out = nullptr;
     P1Out *p1out = nullptr;
     BTRY(balloc(b, &cov, nv));
-    BTRY(balloc(b, &seedm, nv));
-    BTRY(balloc(b, &selm, nv));
     BTRY(balloc(b, &claim, nv));
     BTRY(balloc(b, &seeds_out, (size_t)ninst * kBatchMaxK));
     BTRY(balloc(b, &p1out, ninst));
@@ -283,7 +321,10 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
         I.nv = (int32_t)(vstart[i + 1] - vstart[i]);
         I.narcs = offsets[vstart[i + 1]] - offsets[vstart[i]];
         I.k = parts[i];
-        I.maxdeg = I.ibits = I.dbits = I.symmetric = 0;
+        I.maxdeg = I.ibits = I.dbits = 0;
+        I.symmetric = 1;  // until an arc without its reverse is met
+        I.cbase = 0;
+        I.cstride = 0;
     }
     // largest instances first: the persistent CTAs take them in this order
     std::vector<int32_t> ord(ninst);
@@ -310,7 +351,7 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
     BCUDA(cudaMemsetAsync(cstamp, 0, nv * sizeof(int32_t), s));
     BCUDA(cudaMemsetAsync(ndiff, 0, nv * sizeof(int32_t), s));
     BCUDA(cudaMemsetAsync(ctr, 0, 4 * sizeof(int), s));
-    prepare(off, col, inst, ninst, ctr, ctr + 2, b->num_sms * 4, s);
+    prepare(off, col, inst, ninst, nv, narcs, ctr + 2, b->num_sms * 8, s);
     BTRY(bsync(b));
     int h_err = 0;
     BCUDA(cudaMemcpy(&h_err, ctr + 2, sizeof(int), cudaMemcpyDeviceToHost));
@@ -319,17 +360,33 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
         return fail(DMOLP_ERR_ARG, "instance " + std::to_string(h_err - 1) + ": neighbour id outside its graph");
     }
     BCUDA(cudaMemcpy(hi.data(), inst, ninst * sizeof(Inst), cudaMemcpyDeviceToHost));
+    // key widths, and a slice of kept label counts for every graph whose decisions can use them: symmetric,
+    // degrees in 16 bits
+    int64_t ncnt = 0;
+    for (Inst &I : hi) {
+        int ib = 1, db = 1;
+        while (ib < 62 && (int64_t(1) << ib) <= (int64_t)(I.nv > 0 ? I.nv - 1 : 0)) ++ib;
+        while (db < 62 && (int64_t(1) << db) <= (int64_t)I.maxdeg) ++db;
+        I.ibits = ib;
+        I.dbits = db;
+        I.cbase = ncnt;
+        I.cstride = I.symmetric && I.maxdeg < 65536 ? (std::min(I.k, 32) + 7) & ~7 : 0;
+        ncnt += (int64_t)I.cstride * I.nv;
+    }
+    BTRY(balloc(b, &cnt, ncnt));
+    BCUDA(cudaMemcpy(inst, hi.data(), ninst * sizeof(Inst), cudaMemcpyHostToDevice));
     a.off = off;
     a.col = col;
     a.label = label;
     a.newlab = newlab;
     a.cstamp = cstamp;
     a.ndiff = ndiff;
-    a.l_cand = lc;
     a.l_bnd = lb;
-    a.l_act = la;
     a.l_win0 = w0;
     a.l_win1 = w1;
+    a.rec0 = rec0;
+    a.rec1 = rec1;
+    a.cnt = cnt;
     a.inst = inst;
     a.order = order;
     a.ninst = ninst;
@@ -344,6 +401,7 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
     b->saved = saved;
     b->err = ctr + 2;
     b->h_inst = hi;
+    b->h_order = ord;
     b->h_out.assign(ninst, Out());
     b->h_counts.assign((size_t)ninst * 2 * kBatchMaxK, 0);
     b->ninst = ninst;
@@ -355,25 +413,21 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
     for (int64_t v = 0; v < nv; ++v) b->h_deg[v] = (int32_t)(offsets[v + 1] - offsets[v]);
     b->h_vstart.assign(vstart, vstart + ninst + 1);
     b->have_hubs = false;
-    b->p1_only = nullptr;
+    b->p1_order = nullptr;
     P1Args &q = b->p1;
     q = P1Args();
     q.off = off;
     q.col = col;
     q.label = label;
     q.inst = inst;
-    q.order = order;
-    q.ninst = ninst;
     q.next = ctr + 3;
     q.cov = cov;
-    q.seedm = seedm;
-    q.sel = selm;
     q.claim = claim;
     q.l_front0 = w0;
     q.l_front1 = w1;
-    q.l_claim = lb;
-    q.l_act0 = lc;
-    q.l_act1 = la;
+    q.l_sel = lb;
+    q.rec0 = rec0;
+    q.rec1 = rec1;
     q.seeds_out = seeds_out;
     q.out = p1out;
     b->h_p1.assign(ninst, P1Out());
@@ -507,7 +561,7 @@ int dmolp_batch_phase1(dmolp_batch *b, int theta, const uint8_t *only, int32_t *
     if (!b->have_hubs) {
         // hub lists and first seeds per graph, in the reference's order (init.cpp:139-187)
         std::vector<std::vector<int>> hubs(n);
-        std::vector<int32_t> first(n, 0), first_hub(n, -1);
+        std::vector<int32_t> first(n, 0);
 #pragma omp parallel for schedule(dynamic, 1)
         for (int i = 0; i < n; ++i) {
             const int64_t v0 = b->h_vstart[i], v1 = b->h_vstart[i + 1];
@@ -519,43 +573,42 @@ int dmolp_batch_phase1(dmolp_batch *b, int theta, const uint8_t *only, int32_t *
                 if (d > f.second || (d == f.second && (int)v < f.second)) f = std::make_pair((int)v, d);
             }
             first[i] = f.first < 0 ? 0 : f.first;
-            auto it = std::find(hubs[i].begin(), hubs[i].end(), f.first);
-            first_hub[i] = it == hubs[i].end() ? -1 : (int32_t)(it - hubs[i].begin());
         }
         std::vector<int64_t> hstart(n + 1, 0);
         for (int i = 0; i < n; ++i) hstart[i + 1] = hstart[i] + (int64_t)hubs[i].size();
         std::vector<int32_t> flat(std::max<int64_t>(1, hstart[n]));
         for (int i = 0; i < n; ++i) std::copy(hubs[i].begin(), hubs[i].end(), flat.begin() + hstart[i]);
-        int32_t *dh = nullptr, *df = nullptr, *dfh = nullptr;
+        int32_t *dh = nullptr, *df = nullptr;
         int64_t *dhs = nullptr;
-        uint8_t *used = nullptr;
         BTRY(balloc(b, &dh, flat.size()));
         BTRY(balloc(b, &dhs, n + 1));
         BTRY(balloc(b, &df, n));
-        BTRY(balloc(b, &dfh, n));
-        BTRY(balloc(b, &used, flat.size()));
         BCUDA(cudaMemcpyAsync(dh, flat.data(), flat.size() * sizeof(int32_t), cudaMemcpyHostToDevice, b->stream));
         BCUDA(cudaMemcpyAsync(dhs, hstart.data(), (n + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, b->stream));
         BCUDA(cudaMemcpyAsync(df, first.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, b->stream));
-        BCUDA(cudaMemcpyAsync(dfh, first_hub.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, b->stream));
         BTRY(bsync(b));
         q.hubs = dh;
         q.hstart = dhs;
         q.first = df;
-        q.first_hub = dfh;
-        q.hub_used = used;
         b->have_hubs = true;
     }
     q.theta = theta;
-    q.only = nullptr;
+    const int32_t *order = b->order;
+    std::vector<int32_t> picked;
     if (only) {
-        if (!b->p1_only) BTRY(balloc(b, &b->p1_only, n));
-        BCUDA(cudaMemcpyAsync(b->p1_only, only, n, cudaMemcpyHostToDevice, b->stream));
-        q.only = b->p1_only;
+        for (int32_t i : b->h_order)
+            if (only[i]) picked.push_back(i);
+        if (!b->p1_order) BTRY(balloc(b, &b->p1_order, n));
+        if (!picked.empty())
+            BCUDA(cudaMemcpyAsync(b->p1_order, picked.data(), picked.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
+                                  b->stream));
+        order = b->p1_order;
     }
+    const int slots = b->num_sms * 2;
+    const TeamPlan plan = team_sizes(b->h_inst, only ? picked : b->h_order, slots, p1_threads(), p1_max_team());
     BCUDA(cudaMemsetAsync(q.out, 0, n * sizeof(P1Out), b->stream));
     BCUDA(cudaEventRecord(b->ev0, b->stream));
-    launch_p1(q, std::max(1, std::min(n, b->num_sms * 2)), b->stream);
+    launch_p1(q, order, slots, plan, b->fork, b->stream);
     BCUDA(cudaGetLastError());
     BCUDA(cudaEventRecord(b->ev1, b->stream));
     BCUDA(cudaMemcpyAsync(b->h_p1.data(), q.out, n * sizeof(P1Out), cudaMemcpyDeviceToHost, b->stream));

@@ -1,94 +1,96 @@
-// Batched boundary label propagation: thousands of independent partition instances in one persistent
-// launch, replayed from a captured CUDA graph.
+// Batched boundary label propagation: thousands of independent partition instances in a few persistent
+// launches, replayed from a captured CUDA graph.
 //
 // Each instance is one graph of the batch (its vertices are a contiguous range of the batch's union CSR)
-// with its own part count k <= 64.  A CTA takes the next instance from a global queue (largest first) and
-// runs the whole phase-2 loop of src/phase2/phase2.cpp:256-449 on it -- penalties, candidate marking,
-// boundary test, per-label window selection, decisions, incremental cut / balance update, stopping rules --
-// with block barriers between the steps, then takes the next instance.  The per-instance arithmetic is the
-// single-graph path's: the same penalties (warp_penalties), the same selection keys (degree ascending, or
-// max-degree minus degree when RE > 1, then the vertex's id within its graph), the same decision rule and
-// tie order, so every instance ends bit-identical to a single-graph run of the same graph and labels.
+// with its own part count k <= 64.  A team of C CTAs -- one CTA, or a thread-block cluster of 2 to 16 --
+// runs the whole phase-2 loop of src/phase2/phase2.cpp:256-449 on it: penalties, candidate marking, boundary
+// test, per-label window selection, decisions, incremental cut / balance update, stopping rules, with a
+// barrier of the team between the steps.  The per-instance arithmetic is the single-graph path's: the same
+// penalties (warp_penalties), the same selection keys (degree ascending, or max-degree minus degree when
+// RE > 1, then the vertex's id within its graph), the same decision rule and tie order, so every instance
+// ends bit-identical to a single-graph run of the same graph and labels.
 //
-// Work inside a CTA is scheduled per warp: a warp takes 32 list entries; rows of at most TD arcs are walked
-// by their own lane, longer rows (and vertices whose own label is not scored) by the whole warp, one after
-// another.  The window selection is an MSD radix select over the instance's boundary list with 6-bit
-// digits and one shared-memory histogram of k x 64 counters.  Block size NT, the thread-row limit TD and
-// the number of resident CTAs per SM are the autotuned shape.
+// Why teams: an iteration is a chain of short steps, each bound by the latency of its gathers (L2, ~700
+// cycles), so a graph's time is its vertices per thread times that chain.  With one CTA per graph a batch
+// took as long as its largest graph on one SM while the others idled; the host gives each graph CTAs in
+// proportion to its share of the batch (batch_cabi.cu, team_sizes).  Phase 2 of 64 mixed graphs (2.2 M
+// vertices, 27 M arcs, the largest 195 K vertices): 98 -> 4.3 ms; of 512 graphs of 1 K to 10 K vertices,
+// where most teams are one CTA: 6.7 -> 3.0 ms, from the three points below.
+//
+// Counters the team shares (list lengths, the cut's change) live in the first CTA's shared memory and are
+// reached through distributed shared memory; histograms and part counts are kept per CTA and summed over
+// the team where they are read.  Work inside a team is scheduled per warp: a warp takes 32 list entries;
+// rows of at most TD arcs are walked by their own lane (eight ids in flight), longer rows by the whole warp,
+// one after another.
+//
+//  * Candidates are not listed: marking stores stamps (no atomics), and one coalesced scan over the graph's
+//    vertices does candidacy, the boundary test and the first histogram of the selection.
+//  * The selection is an MSD radix select with 6-bit digits over records (part, key) of 8 bytes, so no pass
+//    gathers labels or degrees; each pass scatters the records that stay open and counts their next digit.
+//  * Decisions of symmetric graphs with at most 32 scored labels read kept label counts (16 bits per label
+//    and vertex, built by the first statistics pass and updated from the movers): a vertex costs one row of
+//    at most 64 bytes instead of a gather per arc.  Other graphs recount from the arcs.
+//
+// Block size NT, the thread-row limit TD and the number of resident CTAs per SM are the autotuned shape.
+#include <cooperative_groups.h>
+
 #include <cfloat>
 
 #include "batch.cuh"
 #include "lp_device.cuh"
+#include "team.cuh"
 
 namespace dmolp {
 namespace batch {
 namespace {
 
-constexpr int kDigitBits = 6;
-constexpr int kDigits = 1 << kDigitBits;
+constexpr int kCountRow = 32;  // statistics: rows of at most this many arcs are counted by one lane
+constexpr int kScanU = 4;      // vertices per lane and step of the boundary scan
+
+// Counters the team shares (in the first CTA's shared memory), by iteration parity.
+struct Shared {
+    int nbnd, nwin, nmov;
+    int nact[kMaxPass];
+    unsigned long long te_cand, te_sel;
+    long long dcut;
+};
 
 template <int NT>
 struct Smem {
-    long long vc[kBatchMaxK], intra[kBatchMaxK];
+    long long vc[kBatchMaxK], intra[kBatchMaxK];    // this CTA's share: the sum over the team is the count
+    long long tvc[kBatchMaxK], tintra[kBatchMaxK];  // the sums at the iteration's start
     double tpen[kBatchMaxK], RE[kBatchMaxK];
     int bcnt[kBatchMaxK], need[kBatchMaxK], below[kBatchMaxK], keep[kBatchMaxK];
-    int hist[kBatchMaxK * kDigits];
+    union {
+        int hist[2][kBatchMaxK * kDigits];  // zero between selections
+        unsigned int bytes[8][NT];          // statistics: byte counters of 32 labels per thread
+    };
     int whist[NT / 32][kBatchMaxK];
-    int ncand, nbnd, nwin, nmov, nact[2], open, bad, inst;
-    unsigned long long te_cand, te_sel, arcs, visits;
-    long long cut_arcs, dcut;
+    Shared sh[2];
+    long long cut_arcs;
+    int bad, inst;
+    unsigned long long arcs, visits;
 };
 
-__device__ __forceinline__ int warp_push(int *ctr, bool pred) {
-    const int lane = threadIdx.x & 31;
-    const unsigned m = __ballot_sync(DMOLP_FULL_MASK, pred);
-    int base = 0;
-    if (lane == 0 && m) base = atomicAdd(ctr, __popc(m));
-    base = __shfl_sync(DMOLP_FULL_MASK, base, 0);
-    return base + __popc(m & ((1u << lane) - 1));
-}
-
-// Visit the n vertices vid(i), i in [0, n).  Every thread of the block calls it.  small(active, v, s, e) is
-// called by all lanes of a warp (active marks the lanes that own a short row); rows with is_big(v, s, e)
-// are passed one by one to wide(v, s, e), called by the whole warp.
-template <typename Vid, typename Big, typename Small, typename Wide>
-__device__ __forceinline__ void visit(const Args &a, int n, Vid vid, Big is_big, Small small, Wide wide) {
-    const int lane = threadIdx.x & 31;
-    for (int i0 = (int)(threadIdx.x & ~31u); i0 < n; i0 += blockDim.x) {
-        const int i = i0 + lane;
-        int v = -1;
-        int64_t s = 0, e = 0;
-        if (i < n) {
-            v = vid(i);
-            s = a.off[v];
-            e = a.off[v + 1];
-        }
-        const bool big = v >= 0 && is_big(v, s, e);
-        small(v >= 0 && !big, v, s, e);
-        unsigned m = __ballot_sync(DMOLP_FULL_MASK, big);
-        while (m) {
-            const int l = __ffs(m) - 1;
-            m &= m - 1;
-            wide(__shfl_sync(DMOLP_FULL_MASK, v, l), __shfl_sync(DMOLP_FULL_MASK, s, l),
-                 __shfl_sync(DMOLP_FULL_MASK, e, l));
-        }
-    }
-}
-
-__device__ __forceinline__ long long block_sum_into(long long x, long long *dst) {
+__device__ __forceinline__ void warp_sum_into(long long x, long long *dst) {
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(DMOLP_FULL_MASK, x, o);
     if ((threadIdx.x & 31) == 0 && x) atomicAdd((unsigned long long *)dst, (unsigned long long)x);
-    return x;
 }
 
-// Label counts and same-label / cut arcs of the instance's current labels (phase2.cpp:55-117, 214-253).
-template <int NT, int TD>
-__device__ void full_stats(const Args &a, const Inst &I, Smem<NT> &sm) {
-    const int lane = threadIdx.x & 31;
+// Label counts and same-label / cut arcs of the instance's current labels (phase2.cpp:55-117, 214-253), each
+// CTA's share into its own counters; with keep_counts also the label counts of every vertex's row.  The
+// team's barriers before (zeroed counters) and after are the caller's.
+template <int NT, int TD, typename Tm>
+__device__ void full_stats(const Args &a, const Inst &I, const Tm &tm, Smem<NT> &sm, bool keep_counts, int eff) {
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int words = I.cstride >> 1;  // 32-bit words of a count row
+    unsigned int *const cw = reinterpret_cast<unsigned int *>(a.cnt + I.cbase);
+    unsigned char *const mine = reinterpret_cast<unsigned char *>(&sm.bytes[0][threadIdx.x]);
+    constexpr int kByteRow = NT * 4;  // bytes between a thread's consecutive counter words
     long long cut = 0;
     int bad = 0;
-    visit(a, I.nv, [&](int i) { return (int)I.vbase + i; },
-          [&](int, int64_t s, int64_t e) { return e - s > TD; },
+    visit(a.off, tm, I.nv, [&](int i) { return (int)I.vbase + i; },
+          [&](int, int64_t s, int64_t e) { return e - s > (keep_counts ? kCountRow : TD); },
           [&](bool act, int v, int64_t s, int64_t e) {
               if (!act) return;
               const int lv = a.label[v];
@@ -96,269 +98,307 @@ __device__ void full_stats(const Args &a, const Inst &I, Smem<NT> &sm) {
                   bad = 1;
                   return;
               }
-              int same = 0, diff = 0;
-              for (int64_t j = s; j < e; ++j) {
-                  const int lu = a.label[__ldg(a.col + j)];
-                  same += lu == lv;
-                  diff += lu != lv;
+              if (keep_counts)
+#pragma unroll
+                  for (int w = 0; w < 8; ++w) sm.bytes[w][threadIdx.x] = 0u;
+              int same = 0;
+              const int deg = (int)(e - s);
+              for (int j = 0; j < deg; j += 8) {
+                  int l[8];
+#pragma unroll
+                  for (int q = 0; q < 8; ++q) l[q] = j + q < deg ? a.label[__ldg(a.col + s + j + q)] : -1;
+#pragma unroll
+                  for (int q = 0; q < 8; ++q) {
+                      same += l[q] == lv;
+                      if (keep_counts && (unsigned)l[q] < (unsigned)eff) mine[(l[q] >> 2) * kByteRow + (l[q] & 3)] += 1;
+                  }
               }
               atomicAdd((unsigned long long *)&sm.vc[lv], 1ull);
               if (same) atomicAdd((unsigned long long *)&sm.intra[lv], (unsigned long long)same);
-              cut += diff;
-              a.ndiff[v] = diff;
+              cut += deg - same;
+              a.ndiff[v] = deg - same;
+              if (keep_counts) {
+                  uint2 *const row = reinterpret_cast<uint2 *>(cw + (size_t)(v - (int)I.vbase) * words);
+                  for (int w = 0; w < words / 2; ++w) {  // four byte counters -> four 16-bit counts
+                      const unsigned int x = sm.bytes[w][threadIdx.x];
+                      row[w] = make_uint2(__byte_perm(x, 0, 0x4140), __byte_perm(x, 0, 0x4342));
+                  }
+              }
           },
           [&](int v, int64_t s, int64_t e) {
               const int lv = a.label[v];
-              int same = 0, diff = 0;
-              warp_row(a.col, s, e, lane, [&](int u) {
-                  const int lu = a.label[u];
-                  same += lu == lv;
-                  diff += lu != lv;
-              }, [] { return false; });
-              for (int o = 16; o > 0; o >>= 1) {
-                  same += __shfl_xor_sync(DMOLP_FULL_MASK, same, o);
-                  diff += __shfl_xor_sync(DMOLP_FULL_MASK, diff, o);
+              int *h = sm.whist[wib];
+              if (keep_counts) {
+                  h[lane] = 0;
+                  __syncwarp();
               }
-              if (lane == 0) {
-                  if ((unsigned)lv >= (unsigned)I.k) {
-                      bad = 1;
-                  } else {
-                      atomicAdd((unsigned long long *)&sm.vc[lv], 1ull);
-                      if (same) atomicAdd((unsigned long long *)&sm.intra[lv], (unsigned long long)same);
-                      cut += diff;
-                      a.ndiff[v] = diff;
-                  }
+              int same = 0;
+              warp_row_wide(a.col, s, e, lane, [&](int u) { return a.label[u]; }, [&](int, int lu) {
+                  same += lu == lv;
+                  if (keep_counts && (unsigned)lu < (unsigned)eff) atomicAdd(&h[lu], 1);
+              }, [] { return false; });
+              for (int o = 16; o > 0; o >>= 1) same += __shfl_xor_sync(DMOLP_FULL_MASK, same, o);
+              const int diff = (int)(e - s) - same;
+              if ((unsigned)lv >= (unsigned)I.k) {
+                  bad = 1;
+              } else if (lane == 0) {
+                  atomicAdd((unsigned long long *)&sm.vc[lv], 1ull);
+                  if (same) atomicAdd((unsigned long long *)&sm.intra[lv], (unsigned long long)same);
+                  cut += diff;
+                  a.ndiff[v] = diff;
+              }
+              if (keep_counts) {
+                  __syncwarp();
+                  if (lane < words)
+                      cw[(size_t)(v - (int)I.vbase) * words + lane] =
+                          (unsigned int)h[2 * lane] | ((unsigned int)h[2 * lane + 1] << 16);
+                  __syncwarp();
               }
           });
-    block_sum_into(cut, &sm.cut_arcs);
-    if (__any_sync(DMOLP_FULL_MASK, bad) && lane == 0) sm.bad = 1;
+    warp_sum_into(cut, tm.first(&sm.cut_arcs));
+    if (__any_sync(DMOLP_FULL_MASK, bad) && lane == 0) *tm.first(&sm.bad) = 1;
 }
 
-// Selection key of a boundary vertex (as the single-graph path's sel_key, with the id inside its graph).
-__device__ __forceinline__ uint64_t key_of(const Inst &I, bool desc, int deg, int v) {
-    const uint64_t dk = desc ? (uint64_t)(I.maxdeg - deg) : (uint64_t)deg;
-    return (dk << I.ibits) | (uint64_t)(v - (int)I.vbase);
-}
-
-template <int NT, int TD>
-__device__ void run_instance(const Args &a, const int ii, Smem<NT> &sm) {
+template <int NT, int TD, typename Tm>
+__device__ void run_instance(const Args &a, const int ii, const Tm &tm, Smem<NT> &sm) {
     const Inst I = a.inst[ii];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int k = I.k;
+    const int k = I.k, vb = (int)I.vbase;
     const int eff = a.cap == DMOLP_LP_CAP_FULL ? k : (k < 32 ? k : 32);
+    const bool counts = I.cstride > 0 && eff <= 32;  // kept label counts (symmetric, 16-bit degrees)
+    const int words = I.cstride >> 1;
+    unsigned int *const cw = reinterpret_cast<unsigned int *>(a.cnt + I.cbase);
     const int stamp0 = *a.stamp_base;
-    int32_t *const cand = a.l_cand + I.vbase, *const bnd = a.l_bnd + I.vbase;
-    int32_t *const act[2] = {a.l_cand + I.vbase, a.l_act + I.vbase};  // cand is dead once bnd is built
+    uint64_t *const rec[2] = {a.rec0 + I.vbase, a.rec1 + I.vbase};
     int32_t *const win[2] = {a.l_win0 + I.vbase, a.l_win1 + I.vbase};
-    int32_t *const mov = a.l_bnd + I.vbase;  // bnd is dead once the window is selected
-    const int npass_raw = (I.dbits + I.ibits + kDigitBits - 1) / kDigitBits;
-    const int npass = npass_raw > 0 ? npass_raw : 1;
+    int32_t *const mov = a.l_bnd + I.vbase;
+    const int kbits = I.dbits + I.ibits;
+    const int npass = (kbits + kDigitBits - 1) / kDigitBits > 0 ? (kbits + kDigitBits - 1) / kDigitBits : 1;
     const int top = npass * kDigitBits;
+    const bool packed = kbits <= kOwnShift;
+    const uint64_t idmask = (uint64_t(1) << I.ibits) - 1;
+    // the part of a record (its label does not change before the movers apply)
+    auto part_of = [&](uint64_t r) {
+        return packed ? (int)(r >> kOwnShift) : a.label[vb + (int)(r & idmask)];
+    };
 
-    for (int p = threadIdx.x; p < k; p += blockDim.x) sm.vc[p] = sm.intra[p] = 0;
+    for (int p = threadIdx.x; p < kBatchMaxK; p += NT) sm.vc[p] = sm.intra[p] = 0;
     if (threadIdx.x == 0) {
         sm.cut_arcs = 0;
         sm.bad = 0;
+        sm.arcs = sm.visits = 0;
     }
-    __syncthreads();
-    full_stats<NT, TD>(a, I, sm);
-    __syncthreads();
+    if (threadIdx.x < 2) sm.sh[threadIdx.x] = Shared();
+    tm.sync();
+    full_stats<NT, TD>(a, I, tm, sm, counts, eff);
+    tm.sync();
+    for (int i = threadIdx.x; i < 2 * kBatchMaxK * kDigits; i += NT) (&sm.hist[0][0])[i] = 0;  // (was byte counters)
+    long long cut_arcs = *tm.first(&sm.cut_arcs);
     Out o;
-    o.edge_cut = sm.cut_arcs >> 1;
+    o.edge_cut = cut_arcs >> 1;
     o.te = o.arcs = o.visits = 0;
     o.iterations = o.stop_reason = o.changes = 0;
-    o.status = (sm.bad || (sm.cut_arcs & 1)) ? DMOLP_ERR_BAD_LABELS : DMOLP_OK;
+    o.status = (*tm.first(&sm.bad) || (cut_arcs & 1)) ? DMOLP_ERR_BAD_LABELS : DMOLP_OK;
     const int max_iter = a.mode == DMOLP_LP_MODE_REF ? kMaxIter : a.iters;
     long long prev_cut = o.edge_cut;
     int conv = 0;
     unsigned long long te_prev_next = (unsigned long long)I.narcs;
     int nprev = I.nv;
+    unsigned long long arcs = 0, visits = 0;
     for (int t = 1; o.status == DMOLP_OK && t <= max_iter; ++t) {
         const int st = stamp0 + t;
-        // ---- penalties (phase2.cpp:158-209) and per-iteration counters ----
-        if (wib == 0)
-            warp_penalties(k, [&](int p) { return sm.vc[p]; }, [&](int p) { return sm.intra[p] / 2; }, a.logtab[t],
-                           sm.RE, sm.tpen, nullptr);
-        for (int p = threadIdx.x; p < k; p += blockDim.x) sm.bcnt[p] = 0;
-        for (int i = threadIdx.x; i < k * kDigits; i += blockDim.x) sm.hist[i] = 0;
-        if (threadIdx.x == 32) {
-            sm.ncand = sm.nbnd = sm.nwin = sm.nmov = 0;
-            sm.te_cand = sm.te_sel = 0;
-            sm.dcut = 0;
+        Shared *const sh = tm.first(&sm.sh[t & 1]);
+        // ---- penalties (phase2.cpp:158-209), by every CTA from the team's counts ----
+        for (int p = threadIdx.x; p < k; p += NT) {
+            long long x = 0, y = 0;
+            for (int r = 0; r < tm.size(); ++r) {
+                x += *tm.at(&sm.vc[p], r);
+                y += *tm.at(&sm.intra[p], r);
+            }
+            sm.tvc[p] = x;
+            sm.tintra[p] = y;
+            sm.bcnt[p] = 0;
         }
         __syncthreads();
+        if (wib == 0)
+            warp_penalties(k, [&](int p) { return sm.tvc[p]; }, [&](int p) { return sm.tintra[p] / 2; }, a.logtab[t],
+                           sm.RE, sm.tpen, nullptr);
         const unsigned long long te_prev = te_prev_next;
-        unsigned long long arcs = 0, visits = 0;
         // ---- candidates = previous window and its neighbours (gpu_lp_boundary.cu:196-214) ----
         if (t > 1) {
             const int32_t *prev = win[(t - 1) & 1];
-            auto mark = [&](int u) {
-                if (a.cstamp[u] != st && atomicExch(&a.cstamp[u], st) != st) cand[atomicAdd(&sm.ncand, 1)] = u;
-            };
-            visit(a, nprev, [&](int i) { return prev[i]; }, [&](int, int64_t s, int64_t e) { return e - s > TD; },
+            visit(a.off, tm, nprev, [&](int i) { return prev[i]; }, [&](int, int64_t s, int64_t e) { return e - s > TD; },
                   [&](bool act, int v, int64_t s, int64_t e) {
                       if (!act) return;
+                      a.cstamp[v] = st;
+                      const int deg = (int)(e - s);
+                      for (int j = 0; j < deg; j += 8) {
+                          int u[8];
+#pragma unroll
+                          for (int q = 0; q < 8; ++q) u[q] = j + q < deg ? __ldg(a.col + s + j + q) : -1;
+#pragma unroll
+                          for (int q = 0; q < 8; ++q)
+                              if (u[q] >= 0) a.cstamp[u[q]] = st;
+                      }
                       ++visits;
-                      mark(v);
-                      for (int64_t j = s; j < e; ++j) mark(__ldg(a.col + j));
-                      arcs += (unsigned long long)(e - s);
+                      arcs += (unsigned long long)deg;
                   },
                   [&](int v, int64_t s, int64_t e) {
                       if (lane == 0) {
+                          a.cstamp[v] = st;
                           ++visits;
-                          mark(v);
                           arcs += (unsigned long long)(e - s);
                       }
-                      warp_row(a.col, s, e, lane, mark, [] { return false; });
+                      warp_row(a.col, s, e, lane, [&](int u) { a.cstamp[u] = st; }, [] { return false; });
                   });
-            __syncthreads();
+            tm.sync();
+        } else {
+            __syncthreads();  // the penalties
         }
-        // ---- boundary test: a neighbour with another label (gpu_lp_boundary.cu:216-236), i.e. ndiff > 0 ----
+        // ---- boundary test over all vertices: a candidate with a neighbour of another label
+        //      (gpu_lp_boundary.cu:216-236), i.e. ndiff > 0; its record and first digit ----
+        if (tm.is_first() && threadIdx.x == 0) sm.sh[(t + 1) & 1] = Shared();  // last read before this barrier
         {
-            const int n = t == 1 ? I.nv : sm.ncand;
             unsigned long long tec = 0;
-            for (int i0 = (int)(threadIdx.x & ~31u); i0 < n; i0 += blockDim.x) {
-                const int i = i0 + lane;
-                bool isb = false;
-                int own = 0, v = 0;
-                if (i < n) {
-                    v = t == 1 ? (int)I.vbase + i : cand[i];
-                    tec += (unsigned long long)(a.off[v + 1] - a.off[v]);
-                    ++visits;
-                    if (a.ndiff[v] > 0) {
-                        isb = true;
-                        own = a.label[v];
-                    }
+            for (int i0 = tm.warp() * 32 * kScanU; i0 < I.nv; i0 += tm.threads() * kScanU) {
+                int deg[kScanU], nd[kScanU], own[kScanU];
+                bool isb[kScanU];
+#pragma unroll
+                for (int q = 0; q < kScanU; ++q) {
+                    const int i = i0 + q * 32 + lane;
+                    const bool in = i < I.nv;
+                    const int v = vb + (in ? i : 0);
+                    isb[q] = in && (t == 1 || a.cstamp[v] == st);
+                    deg[q] = (int)(a.off[v + 1] - a.off[v]);
+                    nd[q] = a.ndiff[v];
+                    own[q] = a.label[v];
                 }
-                const int slot = warp_push(&sm.nbnd, isb);
-                if (isb) {
-                    bnd[slot] = v;
-                    atomicAdd(&sm.bcnt[own], 1);
+                unsigned m[kScanU];
+                int tot = 0;
+#pragma unroll
+                for (int q = 0; q < kScanU; ++q) {
+                    if (isb[q]) {
+                        tec += (unsigned long long)deg[q];
+                        ++visits;
+                    }
+                    isb[q] = isb[q] && nd[q] > 0;
+                    m[q] = __ballot_sync(DMOLP_FULL_MASK, isb[q]);
+                    tot += __popc(m[q]);
+                }
+                int base = 0;
+                if (lane == 0 && tot) base = atomicAdd(&sh->nbnd, tot);
+                base = __shfl_sync(DMOLP_FULL_MASK, base, 0);
+#pragma unroll
+                for (int q = 0; q < kScanU; ++q) {
+                    if (isb[q]) {
+                        const int p = own[q];
+                        const uint64_t dk = sm.RE[p] > 1.0 ? (uint64_t)(I.maxdeg - deg[q]) : (uint64_t)deg[q];
+                        const uint64_t key = (dk << I.ibits) | (uint64_t)(i0 + q * 32 + lane);
+                        rec[0][base + __popc(m[q] & ((1u << lane) - 1))] =
+                            packed ? key | ((uint64_t)p << kOwnShift) : key;
+                        atomicAdd(&sm.bcnt[p], 1);
+                        atomicAdd(&sm.hist[0][p * kDigits + (int)((key >> (top - kDigitBits)) & (kDigits - 1))], 1);
+                    }
+                    base += __popc(m[q]);
                 }
             }
             tec = warp_sum_u64(tec);
-            if (lane == 0 && tec) atomicAdd(&sm.te_cand, tec);
+            if (lane == 0 && tec) atomicAdd(&sh->te_cand, tec);
         }
-        __syncthreads();
+        tm.sync();
         // ---- per label keep ceil(e^(-t/5) * n_p) (gpu_lp_boundary.cu:238-300) ----
         {
             const double ratio = a.ratiotab[t];
-            for (int p = threadIdx.x; p < k; p += blockDim.x) {
-                const int n = sm.bcnt[p];
+            for (int p = threadIdx.x; p < k; p += NT) {
+                int n = 0;
+                for (int r = 0; r < tm.size(); ++r) n += *tm.at(&sm.bcnt[p], r);
                 const int m = (int)ceil(__dmul_rn(ratio, (double)n));
                 sm.need[p] = m > n ? n : m;
             }
         }
-        int32_t *const wout = win[t & 1];
         __syncthreads();
-        int nlist = sm.nbnd;
-        const int32_t *list = bnd;
+        int32_t *const wout = win[t & 1];
+        int nlist = sh->nbnd;
         for (int pass = 0; pass < npass; ++pass) {
             const int shift = top - kDigitBits * (pass + 1);
-            // histogram of the digit over the records of open labels
-            for (int i0 = (int)(threadIdx.x & ~31u); i0 < nlist; i0 += blockDim.x) {
-                const int i = i0 + lane;
-                int bin = -(lane + 1);
-                if (i < nlist) {
-                    const int v = list[i];
-                    const int p = a.label[v];
-                    if (sm.need[p] > 0) {
-                        const int deg = (int)(a.off[v + 1] - a.off[v]);
-                        bin = p * kDigits + (int)((key_of(I, sm.RE[p] > 1.0, deg, v) >> shift) & (kDigits - 1));
-                    }
-                }
-                const unsigned m = __match_any_sync(DMOLP_FULL_MASK, bin);
-                if (bin >= 0 && lane == __ffs(m) - 1) atomicAdd(&sm.hist[bin], __popc(m));
-            }
-            if (threadIdx.x == 0) {
-                sm.open = 0;
-                sm.nact[pass & 1] = 0;
-            }
-            __syncthreads();
-            // per label: the digit where the running count crosses need (warp per label, 2 bins per lane)
-            for (int p = wib; p < k; p += NT / 32) {
-                int *h = sm.hist + p * kDigits;
-                const int c0 = h[2 * lane], c1 = h[2 * lane + 1];
-                h[2 * lane] = 0;
-                h[2 * lane + 1] = 0;
-                const int sum = c0 + c1;
-                int incl = sum;
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(DMOLP_FULL_MASK, incl, o);
-                    if (lane >= o) incl += y;
-                }
-                const int total = __shfl_sync(DMOLP_FULL_MASK, incl, 31);
-                const int nd = sm.need[p];
-                __syncwarp();
-                if (nd <= 0) {
-                    if (lane == 0) {
-                        sm.below[p] = 0;
-                        sm.keep[p] = -1;
-                    }
-                } else if (nd >= total) {
-                    if (lane == 0) {
-                        sm.below[p] = kDigits;
-                        sm.keep[p] = -1;
-                        sm.need[p] = 0;
-                    }
-                } else {
-                    const int ex0 = incl - sum, in0 = ex0 + c0, in1 = in0 + c1;
-                    int d = -1, r = 0, cnt = 0;
-                    if (ex0 < nd && nd <= in0) {
-                        d = 2 * lane;
-                        r = nd - ex0;
-                        cnt = c0;
-                    } else if (in0 < nd && nd <= in1) {
-                        d = 2 * lane + 1;
-                        r = nd - in0;
-                        cnt = c1;
-                    }
-                    if (d >= 0) {
-                        if (r == cnt) {
-                            sm.below[p] = d + 1;
-                            sm.keep[p] = -1;
-                            sm.need[p] = 0;
-                        } else {
-                            sm.below[p] = d;
-                            sm.keep[p] = d;
-                            sm.need[p] = r;
-                            atomicAdd(&sm.open, 1);
-                        }
-                    }
-                }
-            }
-            __syncthreads();
-            // records below the digit are selected; records on it stay for the next digit
-            int32_t *const nxt = act[pass & 1];
-            for (int i0 = (int)(threadIdx.x & ~31u); i0 < nlist; i0 += blockDim.x) {
+            cut_digit(tm, k, sm.hist[pass & 1], sm.need, sm.below, sm.keep);
+            tm.sync();
+            const bool open = any_open(k, sm.keep);
+            // records below the digit are selected; records on it stay, counted by their next digit
+            for (int i = threadIdx.x; i < k * kDigits; i += NT) sm.hist[pass & 1][i] = 0;
+            const uint64_t *const list = rec[pass & 1];
+            uint64_t *const nxt = rec[(pass + 1) & 1];
+            for (int i0 = tm.warp() * 32; i0 < nlist; i0 += tm.threads()) {
                 const int i = i0 + lane;
                 bool take = false, keep = false;
-                int v = 0;
+                uint64_t r = 0;
+                int p = 0;
                 if (i < nlist) {
-                    v = list[i];
-                    const int p = a.label[v];
-                    const int deg = (int)(a.off[v + 1] - a.off[v]);
-                    const int d = (int)((key_of(I, sm.RE[p] > 1.0, deg, v) >> shift) & (kDigits - 1));
+                    r = list[i];
+                    p = part_of(r);
+                    const int d = (int)((r >> shift) & (kDigits - 1));
                     take = d < sm.below[p];
                     keep = d == sm.keep[p];
                 }
-                const int ws = warp_push(&sm.nwin, take);
-                if (take) wout[ws] = v;
-                const int ks = warp_push(&sm.nact[pass & 1], keep);
-                if (keep) nxt[ks] = v;
+                const int ws = warp_push(&sh->nwin, take);
+                if (take) wout[ws] = vb + (int)(r & idmask);
+                const int ks = warp_push(&sh->nact[pass], keep);
+                if (keep) {
+                    nxt[ks] = r;
+                    atomicAdd(&sm.hist[(pass + 1) & 1][p * kDigits + (int)((r >> (shift - kDigitBits)) & (kDigits - 1))],
+                              1);
+                }
             }
-            __syncthreads();
-            if (sm.open == 0) break;
-            list = nxt;
-            nlist = sm.nact[pass & 1];
-            __syncthreads();  // nact of the next pass is reset by thread 0 only after everyone read it
+            tm.sync();
+            if (!open) break;
+            nlist = sh->nact[pass];
         }
-        const int nwin = sm.nwin;
+        const int nwin = sh->nwin;
         // ---- decisions for the window (boundaryLPKernel_unified, gpu_lp_boundary.cu:327-427) ----
-        {
-            unsigned long long tes = 0;
+        unsigned long long tes = 0;
+        if (counts) {
+            for (int i0 = tm.warp() * 32; i0 < nwin; i0 += tm.threads()) {
+                const int i = i0 + lane;
+                int nl = -1, v = 0;
+                if (i < nwin) {
+                    v = wout[i];
+                    const int own = a.label[v];
+                    tes += (unsigned long long)(a.off[v + 1] - a.off[v]);
+                    ++visits;
+                    const uint4 *const row = reinterpret_cast<const uint4 *>(cw + (size_t)(v - vb) * words);
+                    double best = -DBL_MAX;
+                    int bkey = 0x7fffffff, blab = -1, own_cnt = -1;
+                    for (int c0 = 0; c0 < eff; c0 += 8) {
+                        const uint4 x = row[c0 >> 3];
+                        const unsigned int w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) {
+                            const int c = c0 + q;
+                            const int n = (int)((w[q >> 1] >> (16 * (q & 1))) & 0xffffu);
+                            if (c == own) own_cnt = n;
+                            if (c < eff && (n > 0 || own >= eff)) {
+                                const double sc = n > 0 ? __dmul_rn((double)n, sm.tpen[c]) : 0.0;
+                                const int key = tiekey(c);
+                                if (better(sc, key, best, bkey)) {
+                                    best = sc;
+                                    bkey = key;
+                                    blab = c;
+                                }
+                            }
+                        }
+                    }
+                    const double own_raw = own < eff ? (double)own_cnt : -1e300;
+                    if (blab >= 0 && best > own_raw && blab != own) nl = blab;
+                }
+                const int slot = warp_push(&sh->nmov, nl >= 0);
+                if (nl >= 0) {
+                    a.newlab[v] = nl;
+                    mov[slot] = v;
+                }
+            }
+        } else {
             int *h = sm.whist[wib];
-            visit(a, nwin, [&](int i) { return wout[i]; },
+            visit(a.off, tm, nwin, [&](int i) { return wout[i]; },
                   [&](int v, int64_t s, int64_t e) { return e - s > TD || a.label[v] >= eff; },
                   [&](bool act, int v, int64_t s, int64_t e) {
                       int nl = -1;
@@ -393,7 +433,7 @@ __device__ void run_instance(const Args &a, const int ii, Smem<NT> &sm) {
                           }
                           if (blab >= 0 && best > (double)own_cnt && blab != own) nl = blab;
                       }
-                      const int slot = warp_push(&sm.nmov, nl >= 0);
+                      const int slot = warp_push(&sh->nmov, nl >= 0);
                       if (nl >= 0) {
                           a.newlab[v] = nl;
                           mov[slot] = v;
@@ -403,13 +443,9 @@ __device__ void run_instance(const Args &a, const int ii, Smem<NT> &sm) {
                       const int own = a.label[v];
                       for (int c = lane; c < eff; c += 32) h[c] = 0;
                       __syncwarp();
-                      for (int64_t j0 = s; j0 < e; j0 += 32) {
-                          const int64_t j = j0 + lane;
-                          const int lu = j < e ? a.label[__ldg(a.col + j)] : -1;
-                          const bool ok = (unsigned)lu < (unsigned)eff;
-                          const unsigned m = __match_any_sync(DMOLP_FULL_MASK, ok ? lu : -(lane + 1));
-                          if (ok && lane == __ffs(m) - 1) atomicAdd(&h[lu], __popc(m));
-                      }
+                      warp_row_wide(a.col, s, e, lane, [&](int u) { return a.label[u]; }, [&](int, int lu) {
+                          if ((unsigned)lu < (unsigned)eff) atomicAdd(&h[lu], 1);
+                      }, [] { return false; });
                       __syncwarp();
                       double best;
                       int blab;
@@ -423,23 +459,22 @@ __device__ void run_instance(const Args &a, const int ii, Smem<NT> &sm) {
                           const int nl = best > own_raw ? blab : own;
                           if (nl != own) {
                               a.newlab[v] = nl;
-                              mov[atomicAdd(&sm.nmov, 1)] = v;
+                              mov[atomicAdd(&sh->nmov, 1)] = v;
                           }
                       }
                   });
-            tes = warp_sum_u64(tes);
-            if (lane == 0 && tes) atomicAdd(&sm.te_sel, tes);
         }
-        __syncthreads();
-        const int nmov = sm.nmov;
-        // ---- incremental cut / balance update from the movers (symmetric graphs) ----
+        tes = warp_sum_u64(tes);
+        if (lane == 0 && tes) atomicAdd(&sh->te_sel, tes);
+        tm.sync();
+        const int nmov = sh->nmov;
+        // ---- incremental cut / balance / count update from the movers (symmetric graphs) ----
         if (I.symmetric && nmov > 0) {
             long long dcut = 0;
             // cut / intra counts, and the differently-labelled neighbour counts: arc (u,v) seen from u, arc
-            // (v,u) from v when u stays (a moving u updates v's count from its own row)
-            auto upd = [&](int v, int u, long long &dc, long long &in_c, long long &out_a, int &dv) {
-                const int a0 = a.label[v], c = a.newlab[v];
-                const int lo = a.label[u], nu = a.newlab[u];
+            // (v,u) from v when u stays (a moving u updates v's count from its own row); the kept counts of u
+            // lose v's old label and gain its new one.  a0 -> c: v's labels; lo, nu: u's label and its new one
+            auto upd = [&](int u, int lo, int nu, int a0, int c, long long &dc, int &in_c, int &out_a, int &dv) {
                 const int ln = nu >= 0 ? nu : lo;
                 const int w = nu >= 0 ? 1 : 2;
                 dc += w * ((int)(c != ln) - (int)(a0 != lo));
@@ -448,53 +483,76 @@ __device__ void run_instance(const Args &a, const int ii, Smem<NT> &sm) {
                 const int du = (int)(ln != c) - (int)(lo != a0);
                 if (du) atomicAdd(&a.ndiff[u], du);
                 if (nu < 0) dv += (int)(c != lo) - (int)(a0 != lo);
+                if (counts) {  // 16-bit halves: the sums end non-negative, so borrows between them cancel
+                    unsigned int *const row = cw + (size_t)(u - vb) * words;
+                    const unsigned int minus = (unsigned int)-(1 << (16 * (a0 & 1))), plus = 1u << (16 * (c & 1));
+                    if ((a0 >> 1) == (c >> 1)) {
+                        atomicAdd(&row[c >> 1], minus + plus);
+                    } else {
+                        if (a0 < eff) atomicAdd(&row[a0 >> 1], minus);
+                        if (c < eff) atomicAdd(&row[c >> 1], plus);
+                    }
+                }
             };
-            visit(a, nmov, [&](int i) { return mov[i]; }, [&](int, int64_t s, int64_t e) { return e - s > TD; },
+            visit(a.off, tm, nmov, [&](int i) { return mov[i]; }, [&](int, int64_t s, int64_t e) { return e - s > TD; },
                   [&](bool act, int v, int64_t s, int64_t e) {
                       if (!act) return;
-                      long long in_c = 0, out_a = 0;
-                      int dv = 0;
-                      for (int64_t j = s; j < e; ++j) upd(v, __ldg(a.col + j), dcut, in_c, out_a, dv);
+                      const int a0 = a.label[v], c = a.newlab[v], deg = (int)(e - s);
+                      int in_c = 0, out_a = 0, dv = 0;
+                      for (int j = 0; j < deg; j += 4) {
+                          int u[4], lo[4], nu[4];
+#pragma unroll
+                          for (int q = 0; q < 4; ++q) u[q] = j + q < deg ? __ldg(a.col + s + j + q) : -1;
+#pragma unroll
+                          for (int q = 0; q < 4; ++q) {
+                              lo[q] = u[q] >= 0 ? a.label[u[q]] : 0;
+                              nu[q] = u[q] >= 0 ? a.newlab[u[q]] : 0;
+                          }
+#pragma unroll
+                          for (int q = 0; q < 4; ++q)
+                              if (u[q] >= 0) upd(u[q], lo[q], nu[q], a0, c, dcut, in_c, out_a, dv);
+                      }
                       if (dv) atomicAdd(&a.ndiff[v], dv);
-                      arcs += (unsigned long long)(e - s);
+                      arcs += (unsigned long long)deg;
                       ++visits;
-                      const int a0 = a.label[v], c = a.newlab[v];
                       atomicAdd((unsigned long long *)&sm.vc[a0], (unsigned long long)-1ll);
                       atomicAdd((unsigned long long *)&sm.vc[c], 1ull);
                       if (in_c) atomicAdd((unsigned long long *)&sm.intra[c], (unsigned long long)in_c);
-                      if (out_a) atomicAdd((unsigned long long *)&sm.intra[a0], (unsigned long long)-out_a);
+                      if (out_a) atomicAdd((unsigned long long *)&sm.intra[a0], (unsigned long long)-(long long)out_a);
                   },
                   [&](int v, int64_t s, int64_t e) {
-                      long long in_c = 0, out_a = 0, dc = 0;
-                      int dv = 0;
-                      warp_row(a.col, s, e, lane, [&](int u) { upd(v, u, dc, in_c, out_a, dv); }, [] { return false; });
-                      for (int o = 16; o > 0; o >>= 1) {
-                          in_c += __shfl_xor_sync(DMOLP_FULL_MASK, in_c, o);
-                          out_a += __shfl_xor_sync(DMOLP_FULL_MASK, out_a, o);
-                          dv += __shfl_xor_sync(DMOLP_FULL_MASK, dv, o);
+                      const int a0 = a.label[v], c = a.newlab[v];
+                      long long dc = 0;
+                      int in_c = 0, out_a = 0, dv = 0;
+                      warp_row(a.col, s, e, lane,
+                               [&](int u) { upd(u, a.label[u], a.newlab[u], a0, c, dc, in_c, out_a, dv); },
+                               [] { return false; });
+                      for (int o2 = 16; o2 > 0; o2 >>= 1) {
+                          in_c += __shfl_xor_sync(DMOLP_FULL_MASK, in_c, o2);
+                          out_a += __shfl_xor_sync(DMOLP_FULL_MASK, out_a, o2);
+                          dv += __shfl_xor_sync(DMOLP_FULL_MASK, dv, o2);
                       }
-                      if (lane == 0 && dv) atomicAdd(&a.ndiff[v], dv);
                       dcut += dc;
                       if (lane == 0) {
+                          if (dv) atomicAdd(&a.ndiff[v], dv);
                           arcs += (unsigned long long)(e - s);
                           ++visits;
-                          const int a0 = a.label[v], c = a.newlab[v];
                           atomicAdd((unsigned long long *)&sm.vc[a0], (unsigned long long)-1ll);
                           atomicAdd((unsigned long long *)&sm.vc[c], 1ull);
                           if (in_c) atomicAdd((unsigned long long *)&sm.intra[c], (unsigned long long)in_c);
-                          if (out_a) atomicAdd((unsigned long long *)&sm.intra[a0], (unsigned long long)-out_a);
+                          if (out_a) atomicAdd((unsigned long long *)&sm.intra[a0], (unsigned long long)-(long long)out_a);
                       }
                   });
-            block_sum_into(dcut, &sm.dcut);
+            warp_sum_into(dcut, &sh->dcut);
         }
-        __syncthreads();
+        tm.sync();
         // ---- movers take their labels ----
-        for (int i = threadIdx.x; i < nmov; i += blockDim.x) {
+        for (int i = tm.thread(); i < nmov; i += tm.threads()) {
             const int v = mov[i];
             a.label[v] = a.newlab[v];
             a.newlab[v] = -1;
         }
-        // ---- stopping rules (phase2.cpp:305-415) ----
+        // ---- stopping rules (phase2.cpp:305-415), by every thread alike ----
         bool stats = true;
         int stop = 0;
         if (nwin == 0) {
@@ -504,24 +562,16 @@ __device__ void run_instance(const Args &a, const int ii, Smem<NT> &sm) {
             stats = false;
             stop = 2;
         }
+        long long ca = cut_arcs + sh->dcut;
+        const unsigned long long te_cand = sh->te_cand, te_sel = sh->te_sel;
         if (stats && !I.symmetric) {  // no reverse arcs to update from: recount
-            __syncthreads();
-            for (int p = threadIdx.x; p < k; p += blockDim.x) sm.vc[p] = sm.intra[p] = 0;
-            if (threadIdx.x == 0) {
-                sm.cut_arcs = 0;
-                sm.dcut = 0;
-            }
-            __syncthreads();
-            full_stats<NT, TD>(a, I, sm);
+            for (int p = threadIdx.x; p < k; p += NT) sm.vc[p] = sm.intra[p] = 0;
+            if (threadIdx.x == 0) sm.cut_arcs = 0;
+            tm.sync();
+            full_stats<NT, TD>(a, I, tm, sm, false, eff);
+            tm.sync();
+            ca = *tm.first(&sm.cut_arcs);
         }
-        arcs = warp_sum_u64(arcs);
-        visits = warp_sum_u64(visits);
-        if (lane == 0) {
-            atomicAdd(&sm.arcs, arcs);
-            atomicAdd(&sm.visits, visits);
-        }
-        __syncthreads();
-        const long long ca = sm.cut_arcs + sm.dcut;
         if (stats) {
             if (ca & 1) {
                 o.status = DMOLP_ERR_BAD_LABELS;
@@ -535,46 +585,65 @@ __device__ void run_instance(const Args &a, const int ii, Smem<NT> &sm) {
                 prev_cut = cur;
                 if (a.mode == DMOLP_LP_MODE_REF && conv >= 10) stop = 3;
             }
+            cut_arcs = ca;
         }
-        o.te += te_prev + sm.te_cand + sm.te_sel + (stats ? (unsigned long long)I.narcs : 0ull);
+        o.te += te_prev + te_cand + te_sel + (stats ? (unsigned long long)I.narcs : 0ull);
         o.changes += nmov;
         o.iterations = t;
-        te_prev_next = sm.te_sel;
+        te_prev_next = te_sel;
         nprev = nwin;
-        __syncthreads();  // every thread has read this iteration's shared counters
-        if (threadIdx.x == 0 && stats) sm.cut_arcs = ca;
         if (stop) {
             o.stop_reason = stop;
             break;
         }
     }
-    __syncthreads();
-    o.edge_cut = prev_cut;
-    o.arcs = sm.arcs;
-    o.visits = sm.visits;
-    if (threadIdx.x == 0) a.out[ii] = o;
-    long long *cnt = a.counts + (size_t)ii * 2 * kBatchMaxK;
-    for (int p = threadIdx.x; p < kBatchMaxK; p += blockDim.x) {
-        cnt[p] = p < k ? sm.vc[p] : 0;
-        cnt[kBatchMaxK + p] = p < k ? sm.intra[p] / 2 : 0;
+    arcs = warp_sum_u64(arcs);
+    visits = warp_sum_u64(visits);
+    if (lane == 0) {
+        atomicAdd(tm.first(&sm.arcs), arcs);
+        atomicAdd(tm.first(&sm.visits), visits);
     }
-    __syncthreads();
+    tm.sync();
+    if (tm.is_first()) {
+        o.edge_cut = prev_cut;
+        o.arcs = sm.arcs;
+        o.visits = sm.visits;
+        if (threadIdx.x == 0) a.out[ii] = o;
+        long long *cnt = a.counts + (size_t)ii * 2 * kBatchMaxK;
+        for (int p = threadIdx.x; p < kBatchMaxK; p += NT) {
+            long long x = 0, y = 0;
+            for (int r = 0; p < k && r < tm.size(); ++r) {
+                x += *tm.at(&sm.vc[p], r);
+                y += *tm.at(&sm.intra[p], r);
+            }
+            cnt[p] = x;
+            cnt[kBatchMaxK + p] = y / 2;
+        }
+    }
+    tm.sync();  // no CTA leaves, or starts on another graph, while its counters are read
 }
 
+// One CTA per graph: persistent CTAs take the graphs order[0, n) from a queue.
 template <int NT, int TD>
-__global__ void __launch_bounds__(NT, 1024 / NT) k_batch_lp(Args a) {
+__global__ void __launch_bounds__(NT, 1024 / NT) k_batch_lp(Args a, const int32_t *order, int n) {
     __shared__ Smem<NT> sm;
+    const CtaTeam<NT> tm;
     for (;;) {
-        if (threadIdx.x == 0) {
-            sm.inst = atomicAdd(a.next, 1);
-            sm.arcs = 0;
-            sm.visits = 0;
-        }
+        if (threadIdx.x == 0) sm.inst = atomicAdd(a.next, 1);
         __syncthreads();
         const int q = sm.inst;
-        if (q >= a.ninst) break;
-        run_instance<NT, TD>(a, a.order[q], sm);
+        __syncthreads();  // every thread has read it before it is rewritten
+        if (q >= n) break;
+        run_instance<NT, TD>(a, order[q], tm, sm);
     }
+}
+
+// One cluster per graph: cluster c runs order[c].
+template <int NT, int TD>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_batch_lp_team(Args a, const int32_t *order) {
+    __shared__ Smem<NT> sm;
+    const ClusterTeam<NT> tm;
+    run_instance<NT, TD>(a, order[blockIdx.x / tm.size()], tm, sm);
 }
 
 __global__ void k_batch_begin(int *next, int *stamp_base) {
@@ -582,78 +651,93 @@ __global__ void k_batch_begin(int *next, int *stamp_base) {
     *stamp_base += kStampStride;
 }
 
-// Per instance: local neighbour ids -> union ids (with range check), maximum degree, key widths, and
-// whether every row is sorted and every arc has its reverse (binary search in the neighbour's row).
-__global__ void k_batch_prepare(const int64_t *off, int32_t *col, Inst *inst, int ninst, int *next, int *err) {
-    __shared__ int s_i, s_maxdeg, s_unsym, s_bad;
-    for (;;) {
-        if (threadIdx.x == 0) {
-            s_i = atomicAdd(next, 1);
-            s_maxdeg = 0;
-            s_unsym = 0;
-            s_bad = 0;
-        }
-        __syncthreads();
-        const int i = s_i;
-        if (i >= ninst) break;
-        Inst I = inst[i];
-        const int64_t v0 = I.vbase, v1 = I.vbase + I.nv;
-        for (int64_t v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
-            const int64_t s = off[v], e = off[v + 1];
-            atomicMax(&s_maxdeg, (int)(e - s));
-            for (int64_t j = s; j < e; ++j) {
-                const int u = col[j];
-                if ((unsigned)u >= (unsigned)I.nv) s_bad = 1;
-                else col[j] = u + (int)v0;
-            }
-        }
-        __syncthreads();
-        for (int64_t v = v0 + threadIdx.x; v < v1 && !s_bad; v += blockDim.x) {
-            const int64_t s = off[v], e = off[v + 1];
-            int prev = -1;
-            bool sorted = true;
-            for (int64_t j = s; j < e; ++j) {
-                const int u = col[j];
-                sorted &= u > prev;
-                prev = u;
-            }
-            if (!sorted) {
-                s_unsym = 1;
-                continue;
-            }
-            for (int64_t j = s; j < e; ++j) {
-                const int u = col[j];
-                int64_t lo = off[u], hi = off[u + 1];
-                while (lo < hi) {
-                    const int64_t mid = (lo + hi) >> 1;
-                    if (col[mid] < (int)v) lo = mid + 1;
-                    else hi = mid;
-                }
-                if (lo >= off[u + 1] || col[lo] != (int)v) {
-                    s_unsym = 1;
-                    break;
-                }
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            if (s_bad) atomicExch(err, i + 1);
-            I.maxdeg = s_maxdeg;
-            int ib = 1, db = 1;
-            while (ib < 62 && (int64_t(1) << ib) <= (int64_t)(I.nv > 0 ? I.nv - 1 : 0)) ++ib;
-            while (db < 62 && (int64_t(1) << db) <= (int64_t)s_maxdeg) ++db;
-            I.ibits = ib;
-            I.dbits = db;
-            I.symmetric = !s_unsym && !s_bad;
-            inst[i] = I;
-        }
-        __syncthreads();
+// ------------------------------------------------------------------------------------ upload
+// The row of arc j: the last v with off[v] <= j.
+__device__ __forceinline__ int64_t row_of(const int64_t *off, int64_t nv, int64_t j) {
+    int64_t lo = 0, hi = nv;  // off[lo] <= j < off[hi]
+    while (hi - lo > 1) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (off[mid] <= j) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// The instance of vertex v: the last one whose first vertex is <= v (empty instances before it share it).
+__device__ __forceinline__ int inst_of(const Inst *inst, int ninst, int64_t v) {
+    int lo = 0, hi = ninst;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (inst[mid].vbase <= v) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// The three passes of an upload's check run over all arcs (or vertices) of the batch alike, whatever the
+// graphs' sizes and degrees: each thread finds its arc's row and graph by bisection.  One block per graph
+// and one thread per row, as before, took 3.9 s for one skewed graph of a million vertices.
+// Local neighbour ids -> union ids, with the range check (err: 1 + an instance with a bad id).
+__global__ void k_batch_ids(const int64_t *off, int32_t *col, const Inst *inst, int ninst, int64_t nv, int64_t narcs,
+                            int *err) {
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < narcs; j += (int64_t)gridDim.x * blockDim.x) {
+        const int i = inst_of(inst, ninst, row_of(off, nv, j));
+        const int u = col[j];
+        if ((unsigned)u >= (unsigned)inst[i].nv) atomicMax(err, i + 1);
+        else col[j] = u + (int)inst[i].vbase;
     }
 }
 
-template <int NT, int TD>
-void launch_variant(const Args &a, int grid, cudaStream_t s) {
-    k_batch_lp<NT, TD><<<grid, NT, 0, s>>>(a);
+// Whether every row is strictly increasing and every arc has its reverse (bisection in the neighbour's row).
+__global__ void k_batch_symmetric(const int64_t *off, const int32_t *col, Inst *inst, int ninst, int64_t nv,
+                                  int64_t narcs, const int *err) {
+    if (*err) return;
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < narcs; j += (int64_t)gridDim.x * blockDim.x) {
+        const int v = (int)row_of(off, nv, j);
+        const int u = col[j];
+        bool bad = j > off[v] && col[j - 1] >= u;
+        if (!bad) {
+            const int64_t ue = off[u + 1];
+            int64_t lo = off[u], hi = ue;
+            while (lo < hi) {
+                const int64_t mid = (lo + hi) >> 1;
+                if (col[mid] < v) lo = mid + 1;
+                else hi = mid;
+            }
+            bad = lo >= ue || col[lo] != v;
+        }
+        if (bad) inst[inst_of(inst, ninst, v)].symmetric = 0;
+    }
+}
+
+// Largest degree per instance: one atomic per warp where its vertices share the instance.
+__global__ void k_batch_maxdeg(const int64_t *off, Inst *inst, int ninst, int64_t nv) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t v0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~int64_t(31); v0 < nv;
+         v0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t v = v0 + lane < nv ? v0 + lane : nv - 1;
+        const int i = inst_of(inst, ninst, v), deg = (int)(off[v + 1] - off[v]);
+        if (__all_sync(DMOLP_FULL_MASK, i == __shfl_sync(DMOLP_FULL_MASK, i, 0))) {
+            const int m = __reduce_max_sync(DMOLP_FULL_MASK, deg);
+            if (lane == 0) atomicMax(&inst[i].maxdeg, m);
+        } else {
+            atomicMax(&inst[i].maxdeg, deg);
+        }
+    }
+}
+
+// f(kernel, cluster kernel) for the variant (nt, td); false when there is none.
+template <typename F>
+bool with_variant(int nt, int td, F f) {
+#define DMOLP_VARIANT(NT_, TD_)                                     \
+    if (nt == NT_ && td == TD_) {                                   \
+        f(k_batch_lp<NT_, TD_>, k_batch_lp_team<NT_, TD_>);         \
+        return true;                                                \
+    }
+    DMOLP_VARIANT(256, 8) DMOLP_VARIANT(256, 16) DMOLP_VARIANT(512, 8) DMOLP_VARIANT(512, 16) DMOLP_VARIANT(1024, 8)
+    DMOLP_VARIANT(1024, 16)
+#undef DMOLP_VARIANT
+    return false;
 }
 
 }  // namespace
@@ -661,28 +745,43 @@ void launch_variant(const Args &a, int grid, cudaStream_t s) {
 int occupancy(int nt, int td) {
     int n = 0;
     cudaError_t e = cudaSuccess;
-#define DMOLP_OCC(NT_, TD_) \
-    if (nt == NT_ && td == TD_) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_batch_lp<NT_, TD_>, NT_, 0);
-    DMOLP_OCC(256, 8) DMOLP_OCC(256, 16) DMOLP_OCC(512, 8) DMOLP_OCC(512, 16) DMOLP_OCC(1024, 8) DMOLP_OCC(1024, 16)
-#undef DMOLP_OCC
+    with_variant(nt, td, [&](auto one, auto) { e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, one, nt, 0); });
     return e == cudaSuccess ? n : 0;
 }
 
-bool launch(const Args &a, int nt, int td, int grid, cudaStream_t s) {
-    k_batch_begin<<<1, 1, 0, s>>>(a.next, a.stamp_base);
-#define DMOLP_LAUNCH(NT_, TD_)              \
-    if (nt == NT_ && td == TD_) {           \
-        launch_variant<NT_, TD_>(a, grid, s); \
-        return true;                        \
-    }
-    DMOLP_LAUNCH(256, 8) DMOLP_LAUNCH(256, 16) DMOLP_LAUNCH(512, 8) DMOLP_LAUNCH(512, 16) DMOLP_LAUNCH(1024, 8)
-    DMOLP_LAUNCH(1024, 16)
-#undef DMOLP_LAUNCH
-    return false;
+int max_team(int nt, int td) {
+    int best = 1;
+    with_variant(nt, td, [&](auto, auto team) {
+        for (int c = kMaxTeam; c > 1 && best == 1; c >>= 1) {
+            int n = 0;
+            if (max_clusters(team, c, nt, &n) && n > 0) best = c;
+        }
+    });
+    return best;
 }
 
-void prepare(const int64_t *off, int32_t *col, Inst *inst, int ninst, int *next, int *err, int grid, cudaStream_t s) {
-    k_batch_prepare<<<grid, 256, 0, s>>>(off, col, inst, ninst, next, err);
+bool launch(const Args &a, int nt, int td, int grid, const TeamPlan &plan, const Fork &f, cudaStream_t s) {
+    k_batch_begin<<<1, 1, 0, s>>>(a.next, a.stamp_base);
+    return with_variant(nt, td, [&](auto one, auto team) {
+        f.open(plan, s);
+        const int32_t *order = a.order;
+        for (int j = 0, c = kMaxTeam; c > 1; ++j, c >>= 1) {  // the largest graphs first
+            if (plan.n[j] > 0) launch_cluster(team, plan.n[j], c, nt, f.stream(plan, j, s), a, order);
+            order += plan.n[j];
+        }
+        const int n1 = plan.n[kTeamClasses - 1];
+        if (n1 > 0) one<<<grid < n1 ? grid : n1, nt, 0, f.stream(plan, kTeamClasses - 1, s)>>>(a, order, n1);
+        f.close(plan, s);
+    });
+}
+
+void prepare(const int64_t *off, int32_t *col, Inst *inst, int ninst, int64_t nv, int64_t narcs, int *err, int grid,
+             cudaStream_t s) {
+    if (narcs > 0) {
+        k_batch_ids<<<grid, 256, 0, s>>>(off, col, inst, ninst, nv, narcs, err);
+        k_batch_symmetric<<<grid, 256, 0, s>>>(off, col, inst, ninst, nv, narcs, err);
+    }
+    if (nv > 0) k_batch_maxdeg<<<grid, 256, 0, s>>>(off, inst, ninst, nv);
 }
 
 }  // namespace batch
