@@ -18,6 +18,7 @@ std::vector<int> hubs_of(const std::vector<int32_t> &degree);
 namespace batch {
 
 constexpr int kBatchMaxK = DMOLP_BATCH_MAX_K;
+constexpr int kLongRow = 256;      // the per-vertex network kernels give longer rows a block each
 constexpr int kStampStride = 512;  // > the longest run (kMaxIter iterations)
 
 struct Inst {
@@ -51,20 +52,6 @@ struct Args {
     const double *logtab, *ratiotab;
     int mode, iters, cap;
 };
-
-// What the other device modules (the learned proposal) need of a resident batch.
-struct View {
-    const int64_t *off;
-    const int32_t *col;
-    int32_t *label;
-    const Inst *inst;
-    const int32_t *order;
-    int ninst;
-    int64_t nv, narcs;
-    cudaStream_t stream;
-    int num_sms, device;
-};
-bool view(dmolp_batch *b, View *v);  // false when nothing is uploaded
 
 // Batched phase 1 (batch_p1.cu).
 struct P1Out {
@@ -127,9 +114,31 @@ struct Fork {
     }
 };
 
+// What the other device modules (the learned proposal) need of a resident batch.
+struct View {
+    const int64_t *off;
+    const int32_t *col;
+    int32_t *label;
+    const Inst *inst;
+    const int32_t *order;
+    const int32_t *longrow;  // [nlong] vertices of more than kLongRow arcs
+    int ninst, nlong;
+    int64_t nv, narcs;
+    cudaStream_t stream;
+    int num_sms, device;
+    const std::vector<Inst> *h_inst;      // the same table and order on the host
+    const std::vector<int32_t> *h_order;
+    const std::vector<int32_t> *h_longrow;  // ascending
+    const Fork *fork;
+};
+bool view(dmolp_batch *b, View *v);  // false when nothing is uploaded
+
+// CTAs per graph of `order` (batch_cabi.cu).
+TeamPlan team_sizes(const std::vector<Inst> &inst, const std::vector<int32_t> &order, int slots, int nt, int most);
+
 // Whether clusters of c CTAs of the kernel can run, and how many at once.
 template <typename K>
-bool max_clusters(K kernel, int c, int nt, int *n) {
+bool max_clusters(K kernel, int c, int nt, int *n, size_t smem = 0) {
     if (c > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
         return false;
@@ -141,6 +150,7 @@ bool max_clusters(K kernel, int c, int nt, int *n) {
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.gridDim = dim3((unsigned)c);
     cfg.blockDim = dim3((unsigned)nt);
+    cfg.dynamicSmemBytes = smem;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     if (cudaOccupancyMaxActiveClusters(n, kernel, &cfg) == cudaSuccess) return true;
@@ -150,7 +160,7 @@ bool max_clusters(K kernel, int c, int nt, int *n) {
 
 // n clusters of c CTAs (max_clusters has been asked for this kernel and c).
 template <typename K, typename... A>
-cudaError_t launch_cluster(K kernel, int n, int c, int nt, cudaStream_t s, A... args) {
+cudaError_t launch_cluster_smem(K kernel, int n, int c, int nt, size_t smem, cudaStream_t s, A... args) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeClusterDimension;
@@ -158,10 +168,15 @@ cudaError_t launch_cluster(K kernel, int n, int c, int nt, cudaStream_t s, A... 
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.gridDim = dim3((unsigned)(n * c));
     cfg.blockDim = dim3((unsigned)nt);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <typename K, typename... A>
+cudaError_t launch_cluster(K kernel, int n, int c, int nt, cudaStream_t s, A... args) {
+    return launch_cluster_smem(kernel, n, c, nt, 0, s, args...);
 }
 
 int p1_threads();
@@ -171,8 +186,8 @@ void launch_p1(const P1Args &a, const int32_t *order, int grid, const TeamPlan &
 int occupancy(int nt, int td);
 int max_team(int nt, int td);  // the largest cluster the device can run, 1 if none
 bool launch(const Args &a, int nt, int td, int grid, const TeamPlan &plan, const Fork &f, cudaStream_t s);
-void prepare(const int64_t *off, int32_t *col, Inst *inst, int ninst, int64_t nv, int64_t narcs, int *err, int grid,
-             cudaStream_t s);
+void prepare(const int64_t *off, int32_t *col, Inst *inst, int ninst, int64_t nv, int64_t narcs, int *err,
+             int32_t *longrow, int *nlong, int grid, cudaStream_t s);
 
 }  // namespace batch
 }  // namespace dmolp

@@ -30,10 +30,11 @@ struct dmolp_batch {
     std::vector<void *> allocations;
     Args a{};
     Inst *inst = nullptr;
-    int32_t *order = nullptr, *saved = nullptr;
+    int32_t *order = nullptr, *saved = nullptr, *longrow = nullptr;
+    int nlong = 0;
     int *err = nullptr;
     std::vector<Inst> h_inst;
-    std::vector<int32_t> h_order;
+    std::vector<int32_t> h_order, h_longrow;
     std::vector<Out> h_out;
     std::vector<long long> h_counts;
     bool tuned = false;
@@ -102,30 +103,6 @@ int bsync(dmolp_batch *b) {
         if (r_) return r_;   \
     } while (0)
 
-// How many CTAs work on each graph of `order` (largest first): with `slots` CTAs resident at once, a graph deserves its share of the
-// batch's work (arcs + vertices) of them, rounded down to a power of two, up again above 1.4 times that, and at
-// most one CTA per nt vertices (a thread with less than a vertex only adds barriers).  So a batch of thousands
-// of like graphs runs one CTA per graph, and a small batch, or a graph far larger than the others, spreads
-// over the chip.
-TeamPlan team_sizes(const std::vector<Inst> &inst, const std::vector<int32_t> &order, int slots, int nt, int most) {
-    TeamPlan plan{};
-    double total = 0;
-    for (int32_t i : order) total += (double)(inst[i].narcs + inst[i].nv);
-    int last = most;  // the order is by work: team sizes never grow along it
-    for (int32_t i : order) {
-        const Inst &I = inst[i];
-        const double share = total > 0 ? (double)(I.narcs + I.nv) * slots / total : 1.0;
-        int c = 1, j = kTeamClasses - 1;
-        while (2 * c <= last && share > 1.4 * c && (int64_t)I.nv > (int64_t)c * nt) {
-            c *= 2;
-            --j;
-        }
-        last = c;
-        ++plan.n[j];
-    }
-    return plan;
-}
-
 // Capture (once per shape and configuration) and launch the batch.
 int run_graph(dmolp_batch *b, const dmolp_batch_tuning &t, const dmolp_lp_config &cfg) {
     const int occ = occupancy(t.block_threads, t.thread_row_max);
@@ -192,6 +169,30 @@ void balance(const long long *vc, const long long *ec, int k, double *vb, double
 
 namespace dmolp {
 namespace batch {
+// How many CTAs work on each graph of `order` (largest first): with `slots` CTAs resident at once, a graph deserves its share of the
+// batch's work (arcs + vertices) of them, rounded down to a power of two, up again above 1.4 times that, and at
+// most one CTA per nt vertices (a thread with less than a vertex only adds barriers).  So a batch of thousands
+// of like graphs runs one CTA per graph, and a small batch, or a graph far larger than the others, spreads
+// over the chip.
+TeamPlan team_sizes(const std::vector<Inst> &inst, const std::vector<int32_t> &order, int slots, int nt, int most) {
+    TeamPlan plan{};
+    double total = 0;
+    for (int32_t i : order) total += (double)(inst[i].narcs + inst[i].nv);
+    int last = most;  // the order is by work: team sizes never grow along it
+    for (int32_t i : order) {
+        const Inst &I = inst[i];
+        const double share = total > 0 ? (double)(I.narcs + I.nv) * slots / total : 1.0;
+        int c = 1, j = kTeamClasses - 1;
+        while (2 * c <= last && share > 1.4 * c && (int64_t)I.nv > (int64_t)c * nt) {
+            c *= 2;
+            --j;
+        }
+        last = c;
+        ++plan.n[j];
+    }
+    return plan;
+}
+
 bool view(dmolp_batch *b, View *v) {
     if (!b || !b->has_graph) return false;
     v->off = b->a.off;
@@ -199,12 +200,18 @@ bool view(dmolp_batch *b, View *v) {
     v->label = b->a.label;
     v->inst = b->inst;
     v->order = b->order;
+    v->longrow = b->longrow;
+    v->nlong = b->nlong;
     v->ninst = b->ninst;
     v->nv = b->nv;
     v->narcs = b->narcs;
     v->stream = b->stream;
     v->num_sms = b->num_sms;
     v->device = b->device;
+    v->h_inst = &b->h_inst;
+    v->h_order = &b->h_order;
+    v->h_longrow = &b->h_longrow;
+    v->fork = &b->fork;
     return true;
 }
 }  // namespace batch
@@ -306,7 +313,9 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
     BTRY(balloc(b, &counts, (size_t)ninst * 2 * kBatchMaxK));
     BTRY(balloc(b, &lt, kMaxIter + 1));
     BTRY(balloc(b, &rt, kMaxIter + 1));
-    BTRY(balloc(b, &ctr, 4));
+    BTRY(balloc(b, &ctr, 5));
+    int32_t *longrow = nullptr;
+    BTRY(balloc(b, &longrow, narcs / kLongRow + 1));
     uint8_t *cov = nullptr;
     int32_t *claim = nullptr, *seeds_out = nullptr;
     P1Out *p1out = nullptr;
@@ -350,8 +359,8 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
     BCUDA(cudaMemsetAsync(newlab, 0xff, nv * sizeof(int32_t), s));
     BCUDA(cudaMemsetAsync(cstamp, 0, nv * sizeof(int32_t), s));
     BCUDA(cudaMemsetAsync(ndiff, 0, nv * sizeof(int32_t), s));
-    BCUDA(cudaMemsetAsync(ctr, 0, 4 * sizeof(int), s));
-    prepare(off, col, inst, ninst, nv, narcs, ctr + 2, b->num_sms * 8, s);
+    BCUDA(cudaMemsetAsync(ctr, 0, 5 * sizeof(int), s));
+    prepare(off, col, inst, ninst, nv, narcs, ctr + 2, longrow, ctr + 4, b->num_sms * 8, s);
     BTRY(bsync(b));
     int h_err = 0;
     BCUDA(cudaMemcpy(&h_err, ctr + 2, sizeof(int), cudaMemcpyDeviceToHost));
@@ -399,6 +408,11 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
     b->inst = inst;
     b->order = order;
     b->saved = saved;
+    b->longrow = longrow;
+    BCUDA(cudaMemcpy(&b->nlong, ctr + 4, sizeof(int), cudaMemcpyDeviceToHost));
+    b->h_longrow.resize(b->nlong);
+    BCUDA(cudaMemcpy(b->h_longrow.data(), longrow, b->nlong * sizeof(int32_t), cudaMemcpyDeviceToHost));
+    std::sort(b->h_longrow.begin(), b->h_longrow.end());
     b->err = ctr + 2;
     b->h_inst = hi;
     b->h_order = ord;

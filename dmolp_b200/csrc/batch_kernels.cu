@@ -710,8 +710,9 @@ __global__ void k_batch_symmetric(const int64_t *off, const int32_t *col, Inst *
     }
 }
 
-// Largest degree per instance: one atomic per warp where its vertices share the instance.
-__global__ void k_batch_maxdeg(const int64_t *off, Inst *inst, int ninst, int64_t nv) {
+// Largest degree per instance (one atomic per warp where its vertices share the instance), and the list of
+// rows longer than kLongRow.
+__global__ void k_batch_degrees(const int64_t *off, Inst *inst, int ninst, int64_t nv, int32_t *longrow, int *nlong) {
     const int lane = threadIdx.x & 31;
     for (int64_t v0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~int64_t(31); v0 < nv;
          v0 += (int64_t)gridDim.x * blockDim.x) {
@@ -723,6 +724,9 @@ __global__ void k_batch_maxdeg(const int64_t *off, Inst *inst, int ninst, int64_
         } else {
             atomicMax(&inst[i].maxdeg, deg);
         }
+        const bool lg = v0 + lane < nv && deg > kLongRow;
+        const int at = warp_push(nlong, lg);
+        if (lg) longrow[at] = (int)v;
     }
 }
 
@@ -775,13 +779,13 @@ bool launch(const Args &a, int nt, int td, int grid, const TeamPlan &plan, const
     });
 }
 
-void prepare(const int64_t *off, int32_t *col, Inst *inst, int ninst, int64_t nv, int64_t narcs, int *err, int grid,
-             cudaStream_t s) {
+void prepare(const int64_t *off, int32_t *col, Inst *inst, int ninst, int64_t nv, int64_t narcs, int *err,
+             int32_t *longrow, int *nlong, int grid, cudaStream_t s) {
     if (narcs > 0) {
         k_batch_ids<<<grid, 256, 0, s>>>(off, col, inst, ninst, nv, narcs, err);
         k_batch_symmetric<<<grid, 256, 0, s>>>(off, col, inst, ninst, nv, narcs, err);
     }
-    if (nv > 0) k_batch_maxdeg<<<grid, 256, 0, s>>>(off, inst, ninst, nv);
+    if (nv > 0) k_batch_degrees<<<grid, 256, 0, s>>>(off, inst, ninst, nv, longrow, nlong);
 }
 
 }  // namespace batch

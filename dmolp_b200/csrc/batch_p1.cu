@@ -60,30 +60,6 @@ struct P1Smem {
 
 __device__ __forceinline__ int deg_of(const P1Args &a, int v) { return (int)(a.off[v + 1] - a.off[v]); }
 
-// Maximum of a 64-bit key over the team (every thread passes its own; the result in every thread).
-template <typename Tm>
-__device__ __forceinline__ unsigned long long team_max(unsigned long long x, const Tm &tm, P1Smem &sm) {
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long y = __shfl_xor_sync(DMOLP_FULL_MASK, x, o);
-        x = y > x ? y : x;
-    }
-    if ((threadIdx.x & 31) == 0) sm.wbest[threadIdx.x >> 5] = x;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long r = 0;
-        for (int i = 0; i < kP1Threads / 32; ++i) r = sm.wbest[i] > r ? sm.wbest[i] : r;
-        sm.cbest = r;
-    }
-    tm.sync();
-    unsigned long long r = 0;
-    for (int c = 0; c < tm.size(); ++c) {
-        const unsigned long long y = *tm.at(&sm.cbest, c);
-        r = y > r ? y : r;
-    }
-    tm.sync();  // cbest may be rewritten
-    return r;
-}
-
 __device__ __forceinline__ bool is_seed(const P1Smem &sm, int n, int v) {
     bool s = false;
     for (int q = 0; q < n; ++q) s |= sm.seeds[q] == v;
@@ -218,7 +194,7 @@ __device__ void run_p1(const P1Args &a, int ii, const Tm &tm, P1Smem &sm) {
                     ((unsigned long long)(unsigned)deg_of(a, vb + v) << 32) | (0xffffffffull - (unsigned)v);
                 key = c > key ? c : key;
             }
-            key = team_max(key, tm, sm);
+            key = team_max<kP1Threads>(key, tm, sm.wbest, &sm.cbest);
             if (key == 0) break;  // every vertex is a seed
             add_seed(vb + (int)(0xffffffffull - (key & 0xffffffffull)));
         }

@@ -40,6 +40,7 @@ struct GemmArgs {
     int ldo;
     float *out_f32;
     int ldo32;
+    const int64_t *off;  // kBwdData: columns >= kHidden are divided by the row's degree
     float *out_w;
     int *err;
     uint32_t polls;  // polls of the MMA completion barrier before the GEMM gives up (then: err, TMEM freed)
@@ -48,14 +49,25 @@ struct GemmArgs {
 // One launch of the tensor-core GEMM: N = output tile width, KT = K tile.
 void gemm(const GemmArgs &g, int n, int kt, int num_sms, cudaStream_t s);
 
-void agg_fwd(const int64_t *off, const int32_t *col, int nv, __nv_bfloat16 *buf, int C, int num_sms, cudaStream_t s);
-void agg_bwd(const int64_t *off, const int32_t *col, int nv, const float *dC, const __nv_bfloat16 *Hbuf, int ldh,
-             __nv_bfloat16 *G, float *db, int num_sms, cudaStream_t s);
+void agg_fwd(const batch::View &b, __nv_bfloat16 *buf, int C);
+void agg_bwd(const batch::View &b, const float *dC, const __nv_bfloat16 *Hbuf, int ldh, __nv_bfloat16 *G, float *db);
 void loss(const int64_t *off, const int32_t *col, int nv, const float *Z, const int32_t *target, double inv_arcs,
           __nv_bfloat16 *G, float *db, double *loss_sum, int num_sms, cudaStream_t s);
 void grad_out(const float *dZ, int nv, __nv_bfloat16 *G, float *db, int num_sms, cudaStream_t s);
 void adam(float *p, const float *g, float *m, float *v, int n, float lr, int step, cudaStream_t s);
 void cast_weights(const float *params, __nv_bfloat16 *const W[3], __nv_bfloat16 *const Wt[3], cudaStream_t s);
+
+// A work unit of the walk: n <= kChunkV consecutive vertices of one graph, or (n = 0) the long row of v0.
+constexpr int kChunkV = 256;
+struct Chunk {
+    int v0, n, inst;
+};
+
+// A vertex's row and its distance to the nearest anchor so far.
+struct __align__(16) SearchRow {
+    int64_t start;
+    int len, dist;
+};
 
 struct FeatWork {
     const int64_t *off;
@@ -63,32 +75,33 @@ struct FeatWork {
     const batch::Inst *inst;
     int ninst;
     int nv;
-    int32_t *vinst, *dist, *mind, *front0, *front1, *cnt;  // cnt[4]
-    unsigned long long *akey;                              // [ninst]
-    int32_t *anchor;                                       // [kAnchors * ninst]
-    int32_t *ecc;                                          // [ninst]
-    float *P0, *Q0, *P1, *Q1;                              // [nv * 8]
-    double *stats;                                         // [ninst * 16]
-    float *Xf;                                             // [nv * 16] features before rounding
-    __nv_bfloat16 *X;                                      // [nv * ldx] bf16 input of layer 1
+    int32_t *vinst;                           // [nv]
+    SearchRow *row, *front0, *front1, *huge;  // [nv] search state; frontiers and long rows in per-graph slices
+    int *next;                                // the teams' queue
+    int32_t *anchor;                          // [kAnchors * ninst]
+    int32_t *ecc;                             // [ninst]
+    Chunk *chunks;                            // [nv / kChunkV + ninst + the batch's long rows]
+    float *P0, *Q0, *P1, *Q1;                 // [nv * 8]
+    double *stats;                            // [ninst * 16]
+    float *Xf;                                // [nv * 16] features before rounding
+    __nv_bfloat16 *X;                         // [nv * ldx] bf16 input of layer 1
     int ldx;
 };
-int features(const FeatWork &w, int num_sms, cudaStream_t s);  // returns a CUDA error code (0 = ok)
-void features_to_input(const float *Xf, int nv, __nv_bfloat16 *X, int ldx, cudaStream_t s);
+int features(const FeatWork &w, const batch::View &b, cudaStream_t s);  // returns a CUDA error code (0 = ok)
+void features_to_input(const float *Xf, int nv, __nv_bfloat16 *X, int ldx, int num_sms, cudaStream_t s);
 
 struct DecodeWork {
     const batch::Inst *inst;
-    const int32_t *order;
-    int ninst;
-    const float *Z;  // [nv * 16] proposal coordinates (first 8 columns used)
-    float *Y;        // [nv * 4] principal coordinates (work)
+    const float *Z;     // [nv * 16] proposal coordinates (first 8 columns used)
+    uint64_t *key;      // [nv] work
     int32_t *label;
-    int32_t *l0, *l1;  // [nv] each
-    int32_t *status;   // [ninst]
+    int32_t *l0, *l1;   // [nv] each: work
+    int32_t *status;    // [ninst]
     int *next;
-    const uint8_t *skip;  // [ninst] or null: graphs left alone (status 2, labels untouched)
 };
-void decode(const DecodeWork &w, int grid, cudaStream_t s);
+// The graphs of `order` (host and device copies, largest first).  Returns a CUDA error code (0 = ok).
+int decode(const DecodeWork &w, const std::vector<int32_t> &order, const int32_t *d_order, const batch::View &b,
+           cudaStream_t s);
 void coords(const float *Xf, const float *Z, int nv, float *P, int num_sms, cudaStream_t s);
 void gate_scores(const float *Z, const int32_t *vinst, int nv, double *score, int num_sms, cudaStream_t s);
 void gate_grad(const float *g, const int32_t *vinst, int nv, float *dZ, int num_sms, cudaStream_t s);

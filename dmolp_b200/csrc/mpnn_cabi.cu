@@ -57,15 +57,17 @@ struct dmolp_mpnn {
     std::vector<void *> fixed;
     // per-batch workspace
     int64_t cap_nv = -1;
-    int cap_inst = -1;
+    int cap_inst = -1, cap_long = -1;
     bool cap_train = false;
     std::vector<void *> ws;
     __nv_bfloat16 *C1 = nullptr, *C2 = nullptr, *C3 = nullptr, *G = nullptr, *G3 = nullptr;
-    float *Z3 = nullptr, *dC = nullptr, *Xf = nullptr, *Pc = nullptr, *Y = nullptr;
-    int32_t *vinst = nullptr, *dist = nullptr, *mind = nullptr, *f0 = nullptr, *f1 = nullptr, *cnt = nullptr;
-    unsigned long long *akey = nullptr;
+    float *Z3 = nullptr, *dC = nullptr, *Xf = nullptr, *Pc = nullptr;
+    int32_t *vinst = nullptr;
+    int *next_feat = nullptr;
+    Chunk *chunks = nullptr;
     int32_t *anchor = nullptr, *ecc = nullptr, *status = nullptr, *target = nullptr, *dl0 = nullptr, *dl1 = nullptr;
-    uint8_t *skip = nullptr;  // [ninst] graphs the decoder leaves to phase 1
+    int32_t *dorder = nullptr;  // [ninst] graphs of a decoder call, largest first
+    uint64_t *key = nullptr;
     int *next = nullptr;
     float *P0 = nullptr, *Q0 = nullptr, *P1 = nullptr, *Q1 = nullptr;
     double *stats = nullptr, *gscore = nullptr;
@@ -93,12 +95,14 @@ void free_ws(dmolp_mpnn *m) {
     m->ws.clear();
     m->cap_nv = -1;
     m->cap_inst = -1;
+    m->cap_long = -1;
     m->have_z = false;
 }
 
 // Workspace for a batch of nv vertices and ninst graphs (reallocated only when it must grow).
 int ensure_ws(dmolp_mpnn *m, const batch::View &b, bool train) {
-    if (b.nv <= m->cap_nv && b.ninst <= m->cap_inst && (!train || m->cap_train)) return DMOLP_OK;
+    if (b.nv <= m->cap_nv && b.ninst <= m->cap_inst && b.nlong <= m->cap_long && (!train || m->cap_train))
+        return DMOLP_OK;
     cudaStreamSynchronize(b.stream);
     free_ws(m);
     const size_t n = (size_t)b.nv;
@@ -109,23 +113,19 @@ int ensure_ws(dmolp_mpnn *m, const batch::View &b, bool train) {
     MTRY(alloc_into(o, &m->Z3, n * 16));
     MTRY(alloc_into(o, &m->Xf, n * 16));
     MTRY(alloc_into(o, &m->Pc, n * 16));
-    MTRY(alloc_into(o, &m->Y, n * 4));
+    MTRY(alloc_into(o, &m->key, n));
     MTRY(alloc_into(o, &m->G3, n * 16));
     MTRY(alloc_into(o, &m->vinst, n));
-    MTRY(alloc_into(o, &m->dist, n));
-    MTRY(alloc_into(o, &m->mind, n));
-    MTRY(alloc_into(o, &m->f0, n));
-    MTRY(alloc_into(o, &m->f1, n));
     MTRY(alloc_into(o, &m->dl0, n));
     MTRY(alloc_into(o, &m->dl1, n));
     MTRY(alloc_into(o, &m->target, n));
-    MTRY(alloc_into(o, &m->cnt, 4));
+    MTRY(alloc_into(o, &m->next_feat, 1));
     MTRY(alloc_into(o, &m->next, 1));
-    MTRY(alloc_into(o, &m->akey, b.ninst));
+    MTRY(alloc_into(o, &m->chunks, n / kChunkV + b.ninst + b.nlong));
     MTRY(alloc_into(o, &m->anchor, (size_t)kAnchors * b.ninst));
     MTRY(alloc_into(o, &m->ecc, b.ninst));
     MTRY(alloc_into(o, &m->status, b.ninst));
-    MTRY(alloc_into(o, &m->skip, b.ninst));
+    MTRY(alloc_into(o, &m->dorder, b.ninst));
     MTRY(alloc_into(o, &m->stats, (size_t)16 * b.ninst));
     MTRY(alloc_into(o, &m->gscore, b.ninst));
     MTRY(alloc_into(o, &m->ggrad, b.ninst));
@@ -139,6 +139,7 @@ int ensure_ws(dmolp_mpnn *m, const batch::View &b, bool train) {
     }
     m->cap_nv = b.nv;
     m->cap_inst = b.ninst;
+    m->cap_long = b.nlong;
     m->cap_train = train;
     return DMOLP_OK;
 }
@@ -175,7 +176,7 @@ GemmArgs base_args(dmolp_mpnn *m, int rows) {
 void run_forward(dmolp_mpnn *m, const batch::View &b) {
     const int nv = (int)b.nv;
     cudaStream_t s = b.stream;
-    agg_fwd(b.off, b.col, nv, m->C1, kIn, b.num_sms, s);
+    agg_fwd(b, m->C1, kIn);
     __nv_bfloat16 *in[3] = {m->C1, m->C2, m->C3};
     __nv_bfloat16 *out[2] = {m->C2, m->C3};
     for (int l = 0; l < 3; ++l) {
@@ -197,7 +198,7 @@ void run_forward(dmolp_mpnn *m, const batch::View &b) {
             g.ldo32 = kOut;
         }
         gemm(g, kN[l], l == 0 ? 32 : 64, b.num_sms, s);
-        if (l < 2) agg_fwd(b.off, b.col, nv, out[l], kHidden, b.num_sms, s);
+        if (l < 2) agg_fwd(b, out[l], kHidden);
     }
     m->have_z = true;
 }
@@ -234,8 +235,9 @@ void run_backward(dmolp_mpnn *m, const batch::View &b) {
         d.nb = kK[l];
         d.out_f32 = m->dC;
         d.ldo32 = 2 * kHidden;
+        d.off = b.off;
         gemm(d, 2 * kHidden, kN[l] == 16 ? 16 : 64, b.num_sms, s);
-        agg_bwd(b.off, b.col, nv, m->dC, C[l], kK[l], m->G, m->grads + kOffB[l - 1], b.num_sms, s);
+        agg_bwd(b, m->dC, C[l], kK[l], m->G, m->grads + kOffB[l - 1]);
         Gin = m->G;
         ldg = kHidden;
     }
@@ -341,12 +343,13 @@ int dmolp_mpnn_features(dmolp_mpnn *m, dmolp_batch *b, float *features) {
     w.ninst = v.ninst;
     w.nv = (int)v.nv;
     w.vinst = m->vinst;
-    w.dist = m->dist;
-    w.mind = m->mind;
-    w.front0 = m->f0;
-    w.front1 = m->f1;
-    w.cnt = m->cnt;
-    w.akey = m->akey;
+    // the walk's buffers (32 bytes per vertex each) hold the anchor search's before it starts
+    w.row = reinterpret_cast<SearchRow *>(m->P1);
+    w.front0 = reinterpret_cast<SearchRow *>(m->P0);
+    w.front1 = reinterpret_cast<SearchRow *>(m->Q0);
+    w.huge = reinterpret_cast<SearchRow *>(m->Q1);
+    w.next = m->next_feat;
+    w.chunks = m->chunks;
     w.anchor = m->anchor;
     w.ecc = m->ecc;
     w.P0 = m->P0;
@@ -357,7 +360,7 @@ int dmolp_mpnn_features(dmolp_mpnn *m, dmolp_batch *b, float *features) {
     w.Xf = m->Xf;
     w.X = m->C1;
     w.ldx = 2 * kIn;
-    const int e = mpnn::features(w, v.num_sms, v.stream);
+    const int e = mpnn::features(w, v, v.stream);
     if (e) return fail(DMOLP_ERR_CUDA, std::string("features: ") + cudaGetErrorString((cudaError_t)e));
     if (features)
         MCUDA(cudaMemcpyAsync(features, m->Xf, (size_t)v.nv * 16 * sizeof(float), cudaMemcpyDeviceToHost, v.stream));
@@ -371,7 +374,7 @@ int dmolp_mpnn_set_features(dmolp_mpnn *m, dmolp_batch *b, const float *features
     if (!features) return fail(DMOLP_ERR_ARG, "null features");
     MTRY(ensure_ws(m, v, m->cap_train));
     MCUDA(cudaMemcpyAsync(m->Xf, features, (size_t)v.nv * 16 * sizeof(float), cudaMemcpyHostToDevice, v.stream));
-    features_to_input(m->Xf, (int)v.nv, m->C1, 2 * kIn, v.stream);
+    features_to_input(m->Xf, (int)v.nv, m->C1, 2 * kIn, v.num_sms, v.stream);
     m->have_z = false;
     return sync_check(m, v.stream, "set_features");
 }
@@ -442,25 +445,29 @@ static int decode_impl(dmolp_mpnn *m, dmolp_batch *b, const float *embedding, co
     else if (!m->have_z)
         return fail(DMOLP_ERR_STATE, "run forward first or pass an embedding");
     coords(m->Xf, m->Z3, (int)v.nv, m->Pc, v.num_sms, v.stream);
-    DecodeWork w;
-    w.inst = v.inst;
-    w.order = v.order;
-    w.ninst = v.ninst;
-    w.Z = m->Pc;
-    w.Y = m->Y;
-    w.label = v.label;
-    w.l0 = m->dl0;
-    w.l1 = m->dl1;
-    w.status = m->status;
-    w.next = m->next;
-    w.skip = nullptr;
-    if (skip_host) {
-        MCUDA(cudaMemcpyAsync(m->skip, skip_host, v.ninst, cudaMemcpyHostToDevice, v.stream));
-        w.skip = m->skip;
+    std::vector<int32_t> order;
+    for (int32_t i : *v.h_order)
+        if (!skip_host || !skip_host[i]) order.push_back(i);
+    if (!order.empty()) {
+        MCUDA(cudaMemcpyAsync(m->dorder, order.data(), order.size() * sizeof(int32_t), cudaMemcpyHostToDevice, v.stream));
+        DecodeWork w;
+        w.inst = v.inst;
+        w.Z = m->Pc;
+        w.key = m->key;
+        w.label = v.label;
+        w.l0 = m->dl0;
+        w.l1 = m->dl1;
+        w.status = m->status;
+        w.next = m->next;
+        const int e = decode(w, order, m->dorder, v, v.stream);
+        if (e) return fail(DMOLP_ERR_CUDA, std::string("decode: ") + cudaGetErrorString((cudaError_t)e));
     }
-    decode(w, std::max(1, std::min(v.ninst, v.num_sms * 2)), v.stream);
     if (status) MCUDA(cudaMemcpyAsync(status, m->status, v.ninst * sizeof(int32_t), cudaMemcpyDeviceToHost, v.stream));
-    return sync_check(m, v.stream, "decode");
+    MTRY(sync_check(m, v.stream, "decode"));
+    if (status && skip_host)  // the gate prefers phase-1 seeding: nothing was decoded
+        for (int i = 0; i < v.ninst; ++i)
+            if (skip_host[i]) status[i] = 2;
+    return DMOLP_OK;
 }
 
 int dmolp_mpnn_decode(dmolp_mpnn *m, dmolp_batch *b, const float *embedding, int32_t *status) {

@@ -14,6 +14,7 @@ template <int NT>
 struct CtaTeam {
     __device__ __forceinline__ constexpr int size() const { return 1; }
     __device__ __forceinline__ constexpr bool is_first() const { return true; }
+    __device__ __forceinline__ constexpr int rank_of() const { return 0; }
     __device__ __forceinline__ int thread() const { return threadIdx.x; }
     __device__ __forceinline__ constexpr int threads() const { return NT; }
     __device__ __forceinline__ int warp() const { return threadIdx.x >> 5; }
@@ -39,6 +40,7 @@ struct ClusterTeam {
           rank((int)cooperative_groups::this_cluster().block_rank()) {}
     __device__ __forceinline__ int size() const { return n; }
     __device__ __forceinline__ bool is_first() const { return rank == 0; }
+    __device__ __forceinline__ int rank_of() const { return rank; }
     __device__ __forceinline__ int warp() const { return (int)(threadIdx.x >> 5) * n + rank; }
     __device__ __forceinline__ int threads() const { return NT * n; }
     __device__ __forceinline__ int thread() const { return warp() * 32 + (int)(threadIdx.x & 31); }
@@ -61,6 +63,32 @@ __device__ __forceinline__ int warp_push(int *ctr, bool pred) {
     if (lane == 0 && m) base = atomicAdd(ctr, __popc(m));
     base = __shfl_sync(DMOLP_FULL_MASK, base, 0);
     return base + __popc(m & ((1u << lane) - 1));
+}
+
+// Maximum of a 64-bit key over the team (every thread passes its own; the result in every thread).  Two
+// barriers of the team; wbest[NT / 32] and cbest are the CTA's scratch.
+template <int NT, typename Tm>
+__device__ __forceinline__ unsigned long long team_max(unsigned long long x, const Tm &tm, unsigned long long *wbest,
+                                                       unsigned long long *cbest) {
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long y = __shfl_xor_sync(DMOLP_FULL_MASK, x, o);
+        x = y > x ? y : x;
+    }
+    if ((threadIdx.x & 31) == 0) wbest[threadIdx.x >> 5] = x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long r = 0;
+        for (int i = 0; i < NT / 32; ++i) r = wbest[i] > r ? wbest[i] : r;
+        *cbest = r;
+    }
+    tm.sync();
+    unsigned long long r = 0;
+    for (int c = 0; c < tm.size(); ++c) {
+        const unsigned long long y = *tm.at(cbest, c);
+        r = y > r ? y : r;
+    }
+    tm.sync();  // cbest may be rewritten
+    return r;
 }
 
 // Visit the n vertices vid(i), i in [0, n).  Every thread of the team calls it.  small(active, v, s, e) is
