@@ -21,6 +21,7 @@ constexpr int kDecSmall = 32;    // LP decisions: rows of at most 32 arcs are co
 constexpr int kDecSmallK = 64;   // ... when at most 64 labels are scored (byte counters in shared memory)
 constexpr int kLargeDeg = 4096;  // deg > 4096: one block walks the row
 constexpr int kChunk = 4096;     // row chunk of the window-marking kernel
+constexpr int kP1Piece = 512;    // phase 1: longer rows are split into pieces of this many arcs
 constexpr int kHotMax = 16384;   // LP gathers: labels of up to this many highest-degree vertices per block
 constexpr int kHubChunk = 2048;  // row chunk of the decisions of deg > kLargeDeg vertices
 
@@ -128,9 +129,8 @@ struct Buffers {
     int *dtcnt = nullptr;                // [2 * kDegSelMaxK] tail records per label (by iteration parity)
     uint64_t *dlkey = nullptr;           // [nv] keys of the selection warps' lists (labels in active[0])
     uint64_t *dtkey = nullptr;           // [nv] keys of the selection's tail segments
-    int32_t *need = nullptr;             // [MAX_K]
-    int32_t *sel_below = nullptr;        // [MAX_K]
-    int32_t *keep_digit = nullptr;       // [MAX_K]
+    int32_t *need = nullptr;             // [MAX_K] phase-1 seeds
+    int32_t *sel_below = nullptr;        // [MAX_K] phase-1 frontier per part, odd rounds (even: npart)
     int32_t *npart = nullptr;            // [MAX_K] records per segment
     unsigned long long *vc = nullptr;    // [MAX_K] vertex counts
     unsigned long long *intra = nullptr; // [MAX_K] intra-part arcs
@@ -147,9 +147,8 @@ struct Buffers {
     // phase 1 scratch
     uint8_t *covered = nullptr;          // [nv]
     int32_t *hubs = nullptr;             // [nv]
-    uint8_t *hub_used = nullptr;         // [nv]
     int32_t *claim = nullptr;            // [nv] (aliases stamp)
-    unsigned long long *best = nullptr;  // [1] packed hub argmax
+    unsigned long long *best = nullptr;  // [2] packed hub argmax, by seed parity
     int *p1cnt = nullptr;                // [8] phase-1 counters
     unsigned long long *p1te = nullptr;  // [1]
     int *flag = nullptr;                 // [1] scratch flag (symmetry check)

@@ -268,7 +268,6 @@ size_t layout(dmolp_ctx *c, char *base, int64_t nv, int64_t narcs, const size_t 
     ALLOC(b.dtkey, n);
     ALLOC(b.need, DMOLP_MAX_K);
     ALLOC(b.sel_below, DMOLP_MAX_K);
-    ALLOC(b.keep_digit, DMOLP_MAX_K);
     ALLOC(b.npart, DMOLP_MAX_K);
     ALLOC(b.vc, DMOLP_MAX_K);
     ALLOC(b.intra, DMOLP_MAX_K);
@@ -284,8 +283,7 @@ size_t layout(dmolp_ctx *c, char *base, int64_t nv, int64_t narcs, const size_t 
     ALLOC(b.rec, kMaxIter);
     ALLOC(b.covered, n);
     ALLOC(b.hubs, n);
-    ALLOC(b.hub_used, n);
-    ALLOC(b.best, 1);
+    ALLOC(b.best, 2);
     ALLOC(b.p1cnt, 8);
     ALLOC(b.p1te, 1);
     ALLOC(b.flag, 1);
@@ -330,7 +328,7 @@ int graph_alloc(dmolp_ctx *c, int64_t nv, int64_t narcs, int64_t maxdeg, int64_t
     c->dbits = bits_for(maxdeg);
     c->rbits = bits_for(maxraw);
     for (int i = 0; i < 3; ++i) c->nb[i] = (int)nbc[i];
-    c->chunk_cap = narcs / kChunk + 2;
+    c->chunk_cap = narcs / (kP1Piece / 2) + 2;  // pieces of the rows above kP1Piece arcs (more than the chunks)
     c->hubq_cap = narcs / kHubChunk + nbc[2] + 2;
     const size_t nball[3] = {(size_t)nbc[0], (size_t)nbc[1], (size_t)nbc[2]};
     const size_t need = layout(c, nullptr, nv, narcs, nball);
@@ -926,23 +924,17 @@ static int find_seeds_impl(dmolp_ctx *c, int k, int first, const std::vector<int
     seeds.push_back(first);
     if (hubs.empty() || k <= 1) return DMOLP_OK;
     DMOLP_CUDA(cudaMemcpyAsync(b.hubs, hubs.data(), hubs.size() * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
-    DMOLP_CUDA(cudaMemsetAsync(b.hub_used, 0, hubs.size(), c->stream));
     DMOLP_CUDA(cudaMemsetAsync(b.covered, 0, (size_t)nv, c->stream));
-    auto fi = std::find(hubs.begin(), hubs.end(), first);
-    if (fi != hubs.end()) DMOLP_CUDA(cudaMemsetAsync(b.hub_used + (fi - hubs.begin()), 1, 1, c->stream));
-    size_t balls = 0;
-    for (int p = 1; p < k; ++p) {  // seed.cpp:206-226
-        for (; balls < seeds.size(); ++balls) p1_mark_ball(c, seeds[balls]);
-        p1_hub_argmax(c, (int64_t)hubs.size());
-        unsigned long long best = 0;
-        DMOLP_CUDA(cudaMemcpyAsync(&best, b.best, sizeof(best), cudaMemcpyDeviceToHost, c->stream));
-        int st = sync(c);
-        if (st) return st;
-        if (best == 0) break;
-        const int64_t idx = (int64_t)(0xffffffffu - (unsigned)(best & 0xffffffffull));
-        seeds.push_back(hubs[idx]);
-        DMOLP_CUDA(cudaMemsetAsync(b.hub_used + idx, 1, 1, c->stream));
-    }
+    DMOLP_CUDA(cudaMemsetAsync(b.best, 0, 2 * sizeof(unsigned long long), c->stream));
+    DMOLP_CUDA(cudaMemsetAsync(b.p1cnt, 0, 8 * sizeof(int), c->stream));
+    p1_find_seeds(c, k, first, (int64_t)hubs.size());
+    std::vector<int> out(k);
+    int cnt[8];
+    DMOLP_CUDA(cudaMemcpyAsync(out.data(), b.need, (size_t)k * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    DMOLP_CUDA(cudaMemcpyAsync(cnt, b.p1cnt, sizeof(cnt), cudaMemcpyDeviceToHost, c->stream));
+    const int st = check_waits(c);
+    if (st) return st;
+    seeds.assign(out.begin(), out.begin() + cnt[6]);
     return DMOLP_OK;
 }
 
@@ -988,34 +980,12 @@ static void complete_seeds(dmolp_ctx *c, int k, const std::vector<int> &hubs, st
 static int expand_impl(dmolp_ctx *c, int k, int theta, const std::vector<int32_t> &seedk, int *rounds_out) {
     Buffers &b = c->b;
     const int64_t nv = c->nv;
-    p1_init_labels(c);
-    DMOLP_CUDA(cudaMemsetAsync(b.psize, 0, DMOLP_MAX_K * sizeof(long long), c->stream));
-    DMOLP_CUDA(cudaMemsetAsync(b.npart, 0, DMOLP_MAX_K * sizeof(int32_t), c->stream));
-    DMOLP_CUDA(cudaMemsetAsync(b.p1cnt, 0, 8 * sizeof(int), c->stream));
-    // the seeds go through the need[] buffer as staging (k ints)
+    *rounds_out = 0;
+    if (nv <= 0) return DMOLP_OK;
     DMOLP_CUDA(cudaMemcpyAsync(b.need, seedk.data(), k * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
-    p1_set_seeds(c, b.need, k);
-    int cur = 0, rounds = 0;
-    std::vector<long long> psize(k);
-    while (nv > 0) {
-        int cnt[8];
-        DMOLP_CUDA(cudaMemcpyAsync(cnt, b.p1cnt, sizeof(cnt), cudaMemcpyDeviceToHost, c->stream));
-        DMOLP_CUDA(cudaMemcpyAsync(psize.data(), b.psize, k * sizeof(long long), cudaMemcpyDeviceToHost, c->stream));
-        int st = sync(c);
-        if (st) return st;
-        if (cnt[3] >= nv) break;
-        if (cnt[0] == 0) {  // every frontier empty: all unlabelled vertices go to the smallest part
-            int best = 0;
-            for (int p = 1; p < k; ++p)
-                if (psize[p] < psize[best]) best = p;
-            p1_fallback(c, best, cur);
-        }
-        p1_round(c, k, theta, cur);
-        cur ^= 1;
-        ++rounds;
-    }
-    *rounds_out = rounds;
-    return DMOLP_OK;
+    p1_grow(c, k, theta);
+    DMOLP_CUDA(cudaMemcpyAsync(rounds_out, b.p1cnt + 5, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    return check_waits(c);
 }
 
 static int check_seed_args(dmolp_ctx *c, int k) {
@@ -1059,7 +1029,7 @@ int dmolp_expand_partitions(dmolp_ctx *c, int k, int theta, const int32_t *seeds
     int r = 0;
     st = expand_impl(c, k, theta, seedk, &r);
     if (rounds) *rounds = r;
-    return st ? st : check_waits(c);
+    return st;
 }
 
 int dmolp_phase1(dmolp_ctx *c, int k, int theta, int32_t *seeds_out, int64_t *vertex_counts, int64_t *edge_counts,
@@ -1145,7 +1115,7 @@ int dmolp_phase1(dmolp_ctx *c, int k, int theta, int32_t *seeds_out, int64_t *ve
     }
     if (info) *info = inf;
     if (bad) return fail(DMOLP_ERR_BAD_LABELS, "phase 1 left a label outside [0,k)");
-    return check_waits(c);
+    return DMOLP_OK;
 }
 
 int dmolp_lp_run(dmolp_ctx *c, int k, const dmolp_lp_config *cfg, dmolp_lp_result *res, dmolp_lp_record *records,

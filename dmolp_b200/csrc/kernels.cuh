@@ -16,16 +16,15 @@ std::vector<int> hubs_from_degrees(const int32_t *degree, int64_t nv);
 // find_first_seed's (vertex, degree) over that order, its id-vs-degree tie test included.
 std::pair<int, int> first_seed_of(const int32_t *degree, int64_t nv);
 
-// ---- segmented radix select (select_kernels.cu) ----
-// Records i < *n_dev carry a segment seg[i] in [0,nseg) (or -1: an empty slot, ignored) and a 64-bit key
-// whose top bit is below `keybits`; keys are unique.  For every segment p, marks sel[i] = 1 on the need[p] records with the
-// smallest keys (need[] is consumed).  sel[] must be zero on entry.  `stopped` (may be null) turns the
-// launches into no-ops once it is non-zero.
+// ---- window selection (select_kernels.cu) ----
+// Records i < cnt->npos carry a segment bown[i] in [0,nseg) (or -1: an empty slot, ignored) and a 64-bit key
+// bkey[i] whose top bit is below `keybits`; keys are unique.  `stopped` (may be null) turns the launch into a no-op
+// once it is non-zero.
 // The LP window straight out of the selection: the key of a selected record slot holds its vertex and
 // degree (key = (dk << ibits) | v, dk = maxdeg - deg when RE[label] > 1, else deg; label = its segment);
 // v is stamped sstamp[v] = t, appended to win / nwin and to its decision-class list dec[c] / ndec[c], and
 // its degree added to *te.  The segments' needs are min(n, ceil(*ratio * n)) for n = npart[seg] (the
-// reference's ceil(e^(-t/5) n), gpu_lp_boundary.cu:244) instead of the need[] argument.
+// reference's ceil(e^(-t/5) n), gpu_lp_boundary.cu:244).
 struct SplitArgs {
     const double *RE;
     const int32_t *npart;
@@ -41,11 +40,11 @@ struct SplitArgs {
 };
 // first_hist_ready: the writer of the records has already added every record's first digit (bits
 // [select_first_shift(keybits), +8) of its key) into histogram buffer 0 of c->b.hist, bin seg * 256 + digit.
-void select_smallest(dmolp_ctx *c, const int32_t *seg, const uint64_t *key, const int *n_dev, int nseg, int keybits,
-                     uint8_t *sel, const int *stopped, const SplitArgs *split = nullptr, bool first_hist_ready = false);
+void select_window(dmolp_ctx *c, int nseg, int keybits, const SplitArgs &split, const int *stopped,
+                   bool first_hist_ready);
 inline int select_first_shift(int keybits) { return ((keybits + kRadixBits - 1) / kRadixBits - 1) * kRadixBits; }
 void select_prepare();  // kernel attributes; call once before any capture
-// The LP window by degree bins (k_select_deg): the same window as select_smallest with `split`, for at most
+// The LP window by degree bins (k_select_deg): the same window as select_window, for at most
 // kDegSelMaxK labels, with the boundary test's superbin counts in b.dsup (BndArgs::dsup).  Returns false
 // (nothing launched) for more labels.
 bool select_window_deg(dmolp_ctx *c, int nseg, const SplitArgs &split, const int *stopped);
@@ -78,11 +77,11 @@ void lp_window_from_list(dmolp_ctx *c, int k, int t, const double *RE_dev, int n
 void lp_apply_list(dmolp_ctx *c, int k, int eff, int n);
 
 // ---- phase 1 (seed_kernels.cu) ----
-void p1_mark_ball(dmolp_ctx *c, int seed);
-void p1_hub_argmax(dmolp_ctx *c, int64_t nhubs);
-void p1_init_labels(dmolp_ctx *c);
-void p1_set_seeds(dmolp_ctx *c, const int32_t *seeds_dev, int nseeds);
-void p1_fallback(dmolp_ctx *c, int best_part, int cur);
-void p1_round(dmolp_ctx *c, int k, int theta, int cur);
+// Seeds by the reference rule from b.hubs[0, nhubs) and the first seed: b.need[0, found), found = p1cnt[6].
+// b.covered, b.best and p1cnt are cleared by the caller.
+void p1_find_seeds(dmolp_ctx *c, int k, int first, int64_t nhubs);
+// Every growth round from the seeds b.need[0, k): labels, part sizes, the number of rounds in p1cnt[5].
+void p1_grow(dmolp_ctx *c, int k, int theta);
+void p1_prepare();  // kernel attributes
 
 }  // namespace dmolp

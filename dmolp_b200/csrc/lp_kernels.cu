@@ -1848,7 +1848,7 @@ void lp_iteration(dmolp_ctx *c, const LpLaunch &L, int t, bool first, bool last)
         ProfScope ps(c, 4, t);
         const SplitArgs sp = split_args(c, b, t, L.eff);
         if (!(deg_sel && select_window_deg(c, L.k, sp, stopped)))
-            select_smallest(c, b.bown, b.bkey, &b.cnt->npos, L.k, c->dbits + c->ibits, b.bsel, stopped, &sp, hist_ready);
+            select_window(c, L.k, c->dbits + c->ibits, sp, stopped, hist_ready);
     }
     {
         ProfScope ps(c, 1, t);
@@ -1887,7 +1887,7 @@ void lp_window_from_list(dmolp_ctx *c, int k, int t, const double *RE_dev, int n
     c->launches += 4;
     const SplitArgs sp = split_args(c, b, t, DMOLP_MAX_K);
     if (!(deg_sel && select_window_deg(c, k, sp, nullptr)))
-        select_smallest(c, b.bown, b.bkey, &b.cnt->npos, k, c->dbits + c->ibits, b.bsel, nullptr, &sp, a.hist != nullptr);
+        select_window(c, k, c->dbits + c->ibits, sp, nullptr, a.hist != nullptr);
 }
 
 // dmolp_lp_apply: window in b.cand (n entries), penalties in b.tpen; movers reported in bv/bnew.

@@ -1,278 +1,441 @@
-// Phase 1 on the resident CSR: seed coverage and the theta-limited multi-source BFS growth.
+// Phase 1 on the resident CSR, in two cooperative launches: the seeds, and the theta-limited multi-source BFS
+// growth with all its rounds.
 //
-//   ball      the radius-2 ball of a new seed (compute_bfs with MAX_LEVELS = 3, src/phase1/seed.cpp:20-101)
-//             is OR-ed into a coverage byte map: level 1 = the seed's row, level 2 = the rows of level 1
-//   hub scan  first unused, uncovered hub of maximum raw degree in hub order (seed.cpp:154-170): one
-//             64-bit atomicMax over (degree, ~hub_index)
-//   round     (partition.cpp:371-603) per part, the theta frontier vertices with the smallest
-//             (raw degree, id) -- segmented radix select -- expand; an unlabelled neighbour is claimed by
-//             atomicMin over part ids, which is the reference's "lowest part wins" (its parts are visited in
-//             ascending order with a shared visited set, partition.cpp:455-476); claimed vertices join
-//             their part's frontier, unselected frontier vertices carry over.
+//   seeds   per seed, its radius-2 ball (compute_bfs with MAX_LEVELS = 3, src/phase1/seed.cpp:20-101) is OR-ed
+//           into a coverage byte map: level 1 = the seed's row, level 2 = the rows of level 1; then the first
+//           uncovered hub of maximum raw degree in hub order (seed.cpp:154-170) is the next seed: one 64-bit
+//           atomicMax over (degree, ~hub_index).  A seed's ball covers it, so no hub is taken twice.
+//   growth  rounds (partition.cpp:371-603): per part, the theta frontier vertices with the smallest (raw degree,
+//           id) expand; an unlabelled neighbour is claimed by atomicMin over part ids, which is the reference's
+//           "lowest part wins" (its parts are visited in ascending order with a shared visited set,
+//           partition.cpp:455-476); claimed vertices join their part's frontier, unselected frontier vertices
+//           carry over.
+//
+// What bounds it: latency.  A round handles at most theta vertices per part, a few dependent gathers each, and
+// there are 20 to 80 rounds.  With a host check and seven launches per round a round cost 65 us on a 5 K-vertex
+// mesh and 160 us on a skewed graph of a million vertices; here it is two grid barriers (claims | labels), a third
+// when rows of more than kP1Piece arcs are split, and the select's only in rounds where a part has more than
+// theta frontier vertices: 12 and 70 us a round.  Whole phase 1 (hub list on the host included): 1.9 -> 0.6 ms on the
+// mesh, 8.9 -> 6.2 ms on the skewed graph.
+#include <algorithm>
 #include <climits>
 
-#include "kernels.cuh"
+#include "select_radix.cuh"
 
 namespace dmolp {
 namespace {
 
-// phase-1 counters (b.p1cnt): 0 = front size (cur), 1 = front size (next), 2 = claimed count,
-// 3 = labelled total, 4 = records
-__global__ void k_p1_level1(Buffers b, int seed) {
-    const int64_t s = b.off[seed], e = b.off[seed + 1];
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        b.covered[seed] = 1;
-        atomicAdd(b.p1te, (unsigned long long)(e - s));
-    }
-    for (int64_t j = s + blockIdx.x * blockDim.x + threadIdx.x; j < e; j += (int64_t)gridDim.x * blockDim.x)
-        b.covered[b.col[j]] = 1;
+constexpr int kP1Row = 16;     // rows of at most this many arcs are walked by one lane (a bit per claimed arc)
+constexpr int kP1BlockV = 128;  // vertices per block of the launches: few blocks make a barrier cheap
+
+// b.p1cnt: frontier sizes and queued row pieces by round parity, labelled vertices, rounds, seeds found
+enum { kFront = 0, kPieces = 2, kLabelled = 4, kRounds = 5, kFound = 6 };
+
+// The first warp of every block comes first, so short lists spread over the SMs.
+__device__ __forceinline__ int grid_warp() { return (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x; }
+__device__ __forceinline__ int grid_warps() { return (int)(blockDim.x >> 5) * (int)gridDim.x; }
+
+// Row [s, e) of vertex v queued in pieces of kP1Piece arcs.
+__device__ __forceinline__ void queue_row(const Buffers &b, int *ctr, int v, int64_t deg) {
+    const int n = (int)((deg + kP1Piece - 1) / kP1Piece);
+    const int q = atomicAdd(ctr, n);
+    for (int i = 0; i < n; ++i) b.chunkq[q + i] = make_int2(v, i * kP1Piece);
 }
 
-// Warp per level-1 vertex (the seed's neighbours, excluding the seed itself on a self-loop).
-__global__ void k_p1_level2(Buffers b, int seed) {
+__device__ __forceinline__ void cover_arcs(const Buffers &b, int64_t s, int64_t e) {
+    warp_row(b.col, s, e, threadIdx.x & 31, [&](int x) { b.covered[x] = 1; }, [] { return false; });
+}
+
+// seeds[0, found) to b.need, found to p1cnt.  b.covered, b.best[2] and p1cnt are zero on entry.
+__global__ void __launch_bounds__(kSelThreads, 1) k_p1_find_seeds(Buffers b, int k, int first, int nhubs,
+                                                                  unsigned int polls) {
     const int lane = threadIdx.x & 31;
-    const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int64_t s = b.off[seed], e = b.off[seed + 1];
+    int seed = first, found = 1;
     unsigned long long te = 0;
-    for (int64_t i = s + gw; i < e; i += nw) {
-        const int u = b.col[i];
-        if (u == seed) continue;
-        const int64_t us = b.off[u], ue = b.off[u + 1];
-        if (lane == 0) te += (unsigned long long)(ue - us);
-        for (int64_t j = us + lane; j < ue; j += 32) b.covered[ld_stream(b.col + j)] = 1;
+    if (blockIdx.x == 0 && threadIdx.x == 0) b.need[0] = first;
+    for (int p = 1; p < k; ++p) {
+        int *const npiece = &b.p1cnt[kPieces + (p & 1)];
+        const int64_t s = b.off[seed], e = b.off[seed + 1];
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            b.covered[seed] = 1;
+            te += (unsigned long long)(e - s);
+        }
+        for (int64_t i0 = s + (int64_t)grid_warp() * 32; i0 < e; i0 += (int64_t)grid_warps() * 32) {
+            const int64_t i = i0 + lane;
+            int64_t us = 0, ue = 0;
+            if (i < e) {
+                const int u = b.col[i];
+                b.covered[u] = 1;
+                if (u != seed) {
+                    us = b.off[u];
+                    ue = b.off[u + 1];
+                    te += (unsigned long long)(ue - us);
+                    if (ue - us > kP1Piece) queue_row(b, npiece, u, ue - us);
+                }
+            }
+            const int64_t deg = ue - us;
+            if (deg <= kP1Row)
+                for (int64_t j = us; j < ue; j += 8) {
+                    int x[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) x[q] = j + q < ue ? __ldg(b.col + j + q) : -1;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (x[q] >= 0) b.covered[x[q]] = 1;
+                }
+            for (unsigned m = __ballot_sync(DMOLP_FULL_MASK, deg > kP1Row && deg <= kP1Piece); m; m &= m - 1) {
+                const int l = __ffs(m) - 1;
+                cover_arcs(b, __shfl_sync(DMOLP_FULL_MASK, us, l), __shfl_sync(DMOLP_FULL_MASK, ue, l));
+            }
+        }
+        if (!grid_sync(b.ctrl, polls, 20)) return;
+        const int np = __ldcg(npiece);
+        if (np) {  // the same in every block
+            for (int q = grid_warp(); q < np; q += grid_warps()) {
+                const int2 c = b.chunkq[q];
+                const int64_t ps = b.off[c.x] + c.y, pe = b.off[c.x + 1];
+                cover_arcs(b, ps, pe - ps > kP1Piece ? ps + kP1Piece : pe);
+            }
+            if (!grid_sync(b.ctrl, polls, 21)) return;
+        }
+        // the next seed; the other parity's maximum and piece count were last read before the barrier above
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            b.best[(p + 1) & 1] = 0;
+            b.p1cnt[kPieces + ((p + 1) & 1)] = 0;
+        }
+        unsigned long long best = 0;
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nhubs; i += gridDim.x * blockDim.x) {
+            const int h = b.hubs[i];
+            if (b.covered[h]) continue;
+            const unsigned long long key = ((unsigned long long)(unsigned)b.rawdeg[h] << 32) |
+                                           (unsigned long long)(0xffffffffu - (unsigned)i);
+            best = best > key ? best : key;
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long ob = __shfl_xor_sync(DMOLP_FULL_MASK, best, o);
+            best = best > ob ? best : ob;
+        }
+        if (lane == 0 && best) atomicMax(&b.best[p & 1], best);
+        if (!grid_sync(b.ctrl, polls, 22)) return;
+        best = __ldcg(&b.best[p & 1]);
+        if (best == 0) break;  // the same in every block
+        seed = b.hubs[0xffffffffu - (unsigned)(best & 0xffffffffull)];
+        if (blockIdx.x == 0 && threadIdx.x == 0) b.need[p] = seed;
+        ++found;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) b.p1cnt[kFound] = found;
     te = warp_sum_u64(te);
     if (lane == 0 && te) atomicAdd(b.p1te, te);
 }
 
-__global__ void k_p1_hub_argmax(Buffers b, int64_t nhubs) {
-    unsigned long long best = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nhubs; i += (int64_t)gridDim.x * blockDim.x) {
-        if (b.hub_used[i]) continue;
-        const int h = b.hubs[i];
-        if (b.covered[h]) continue;
-        const unsigned long long key = ((unsigned long long)(unsigned)b.rawdeg[h] << 32) |
-                                       (unsigned long long)(0xffffffffu - (unsigned)i);
-        best = best > key ? best : key;
+// A warp's appends to the next frontier, collected in shared memory: the counter is one address, and with an append
+// per step and warp the 25 K row pieces of one round of a skewed graph of a million vertices took 90 us, not 61.
+constexpr int kStageP1 = 512;
+struct Append {
+    int32_t *stage, *next;
+    int *nnext;
+    int n;  // staged, the same in every lane
+    __device__ __forceinline__ void flush() {
+        const int lane = threadIdx.x & 31;
+        int base = 0;
+        if (lane == 0 && n) base = atomicAdd(nnext, n);
+        base = __shfl_sync(DMOLP_FULL_MASK, base, 0);
+        __syncwarp();
+        for (int i = lane; i < n; i += 32) next[base + i] = stage[i];
+        __syncwarp();
+        n = 0;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        unsigned long long ob = __shfl_xor_sync(DMOLP_FULL_MASK, best, o);
-        best = best > ob ? best : ob;
+    // Room for cnt entries of this lane; all lanes call it, and fewer than kStageP1 are asked for together.
+    __device__ __forceinline__ int32_t *take(int cnt) {
+        const int lane = threadIdx.x & 31;
+        int incl = cnt;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(DMOLP_FULL_MASK, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const int tot = __shfl_sync(DMOLP_FULL_MASK, incl, 31);
+        if (n + tot > kStageP1) flush();
+        int32_t *const r = stage + n + incl - cnt;
+        n += tot;
+        return r;
     }
-    if ((threadIdx.x & 31) == 0 && best) atomicMax(b.best, best);
+};
+
+// Claims of the arcs [s, e) of frontier vertices by one warp: unlabelled neighbours take atomicMin(part), and the one
+// thread that turns a claim from INT_MAX appends the vertex to the next frontier, as ~vertex.  All lanes call it;
+// the G lanes of a group hold the same row (s == e: none), part p, and walk it G * U arcs a step, so that a warp has
+// 32 / G rows in flight.
+template <int G, int U>
+__device__ __forceinline__ void claim_rows(const Buffers &b, int p, int64_t s, int64_t e, Append &out) {
+    for (int64_t j0 = s + (threadIdx.x & (G - 1)); __any_sync(DMOLP_FULL_MASK, j0 < e); j0 += G * U) {
+        int u[U];
+        bool f[U];
+        int cnt = 0;
+#pragma unroll
+        for (int q = 0; q < U; ++q) u[q] = j0 + q * G < e ? __ldg(b.col + j0 + q * G) : -1;
+#pragma unroll
+        for (int q = 0; q < U; ++q) f[q] = u[q] >= 0 && b.label[u[q]] < 0;
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (f[q]) {
+                f[q] = atomicMin(&b.claim[u[q]], p) == INT_MAX;
+                cnt += f[q];
+            }
+        if (!__any_sync(DMOLP_FULL_MASK, cnt > 0)) continue;
+        int32_t *slot = out.take(cnt);
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (f[q]) *slot++ = ~u[q];
+    }
 }
 
-__global__ void k_p1_init(Buffers b, int nv) {
+// All rounds from the seeds b.need[0, k) (-1: the part has none).  npart2[2]: frontier vertices per part, by round
+// parity.  smem_off: words of dynamic shared memory in front of this kernel's own 2k counters (the select's,
+// then the warps' staged appends).
+__global__ void __launch_bounds__(kSelThreads, 1) k_p1_grow(Buffers b, const SelArgs a, int nv, int k, int theta, int ibits,
+                                                            int smem_off) {
+    extern __shared__ unsigned int smem[];
+    int *const s_np = reinterpret_cast<int *>(smem) + smem_off;  // frontier vertices per part, next round
+    int *const s_ps = s_np + k;                                  // vertices labelled per part
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    int32_t *const npart2[2] = {b.npart, b.sel_below};
+    LpControl *const ctl = a.ctl;
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
         b.label[v] = -1;
         b.claim[v] = INT_MAX;
     }
-}
-
-// seeds_dev[p] (p < nseeds, -1 = no seed): label the seed and start its frontier.
-__global__ void k_p1_seeds(Buffers b, const int32_t *seeds, int nseeds) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        int n = 0, lab = 0;
-        for (int p = 0; p < nseeds; ++p) {
-            const int s = seeds[p];
+    if (blockIdx.x == 0) {
+        for (int p = threadIdx.x; p < k; p += blockDim.x) {
+            const int has = b.need[p] >= 0;
+            b.psize[p] = has;
+            npart2[0][p] = has;
+            npart2[1][p] = 0;
+        }
+        if (threadIdx.x < 8) b.p1cnt[threadIdx.x] = 0;
+    }
+    if (!grid_sync(ctl, a.polls, 23)) return;
+    if (blockIdx.x == 0)
+        for (int p = threadIdx.x; p < k; p += blockDim.x) {
+            const int s = b.need[p];
             if (s < 0) continue;
             b.label[s] = p;
-            b.win[0][n++] = s;
-            ++lab;
-            b.psize[p] += 1;
+            b.win[0][atomicAdd(&b.p1cnt[kFront], 1)] = s;
+            atomicAdd(&b.p1cnt[kLabelled], 1);
         }
-        b.p1cnt[0] = n;
-        b.p1cnt[3] = lab;
-    }
-}
-
-// All frontiers empty (partition.cpp:376-394): every unlabelled vertex joins `best` and its frontier.
-__global__ void k_p1_fallback(Buffers b, int nv, int best, int cur) {
-    int32_t *front = b.win[cur];
-    for (int v0 = blockIdx.x * blockDim.x; v0 < nv; v0 += gridDim.x * blockDim.x) {
-        const int v = v0 + threadIdx.x;
-        const bool un = v < nv && b.label[v] < 0;
-        if (un) b.label[v] = best;
-        const int slot = warp_append(&b.p1cnt[0], un);
-        if (un) front[slot] = v;
-        const int c = __popc(__ballot_sync(DMOLP_FULL_MASK, un));
-        if ((threadIdx.x & 31) == 0 && c) {
-            atomicAdd(&b.p1cnt[3], c);
-            atomicAdd((unsigned long long *)&b.psize[best], (unsigned long long)c);
-        }
-    }
-}
-
-// Selection records of the current frontier: segment = part, key = (raw degree, id).  The records per part
-// are counted in shared memory first (k parts), then added with one global atomic per part and block.
-__global__ void k_p1_records(Buffers b, int cur, int ibits, int k) {
-    extern __shared__ int s_np[];  // [k]
-    for (int p = threadIdx.x; p < k; p += blockDim.x) s_np[p] = 0;
-    __syncthreads();
-    const int n = b.p1cnt[0];
-    const int32_t *front = b.win[cur];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int v = front[i];
-        const int p = b.label[v];
-        b.bown[i] = p;
-        b.bkey[i] = ((uint64_t)(unsigned)b.rawdeg[v] << ibits) | (uint64_t)v;
-        b.bsel[i] = 0;
-        atomicAdd(&s_np[p], 1);
-    }
-    __syncthreads();
-    for (int p = threadIdx.x; p < k; p += blockDim.x)
-        if (s_np[p]) atomicAdd(&b.npart[p], s_np[p]);
-    if (blockIdx.x == 0 && threadIdx.x == 0) b.p1cnt[4] = n;
-}
-
-__global__ void k_p1_need(Buffers b, int k, int theta) {
-    for (int p = threadIdx.x; p < k; p += blockDim.x) {
-        const int n = b.npart[p];
-        b.need[p] = n < theta ? n : theta;
-        b.npart[p] = 0;  // consumed; ready for the next round
-    }
-}
-
-// Claims of the arcs [s, e) of a selected frontier vertex of part p, one warp: unlabelled neighbours take
-// atomicMin(part); the one thread that turns a claim from INT_MAX appends the vertex to the claimed list.
-__device__ __forceinline__ void claim_arcs(const Buffers &b, int p, int64_t s, int64_t e) {
-    const int lane = threadIdx.x & 31;
-    for (int64_t j0 = s; j0 < e; j0 += 32) {
-        const int64_t j = j0 + lane;
-        bool first = false;
-        int v = 0;
-        if (j < e) {
-            v = ld_stream(b.col + j);
-            if (b.label[v] < 0) first = atomicMin(&b.claim[v], p) == INT_MAX;
-        }
-        const int slot = warp_append(&b.p1cnt[2], first);
-        if (first) b.cand[slot] = v;
-    }
-}
-
-// Warp per selected frontier vertex: its first kChunk arcs; the rest of a longer row (the seeds are hubs) is
-// queued in kChunk pieces for k_p1_claim_chunks, so that no warp walks a whole hub row alone.  Claims are
-// atomicMin, so the order in which pieces run does not matter.
-__global__ void k_p1_claim(Buffers b, int cur) {
-    const int lane = threadIdx.x & 31;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-    const int n = b.p1cnt[0];
-    const int32_t *front = b.win[cur];
+    if (!grid_sync(ctl, a.polls, 24)) return;
     unsigned long long te = 0;
-    for (int i = gw; i < n; i += nw) {
-        if (!b.bsel[i]) continue;
-        const int u = front[i];
-        const int p = b.bown[i];
-        const int64_t s = b.off[u], e = b.off[u + 1];
-        if (lane == 0) {
-            te += (unsigned long long)(e - s);
-            for (int64_t c = s + kChunk; c < e; c += kChunk) {
-                const int q = atomicAdd(&b.p1cnt[5], 1);
-                b.chunkq[q] = make_int2(i, (int)(c - s));
+    int rounds = 0;
+    for (int par = 0; __ldcg(&b.p1cnt[kLabelled]) < nv; par ^= 1, ++rounds) {
+        int32_t *const front = b.win[par], *const next = b.win[par ^ 1];
+        int *const nnext = &b.p1cnt[kFront + (par ^ 1)], *const npiece = &b.p1cnt[kPieces + par];
+        int n = __ldcg(&b.p1cnt[kFront + par]);
+        for (int p = threadIdx.x; p < 2 * k; p += blockDim.x) s_np[p] = 0;
+        if (n == 0) {
+            // every frontier empty (partition.cpp:376-394): the unlabelled vertices join the smallest part
+            int best = 0;
+            long long bs = __ldcg(b.psize);
+            for (int p = 1; p < k; ++p) {
+                const long long x = __ldcg(b.psize + p);
+                if (x < bs) {
+                    bs = x;
+                    best = p;
+                }
+            }
+            if (!grid_sync(ctl, a.polls, 25)) return;  // every block has read the sizes
+            for (int v0 = grid_warp() * 32; v0 < nv; v0 += grid_warps() * 32) {
+                const int v = v0 + lane;
+                const bool un = v < nv && b.label[v] < 0;
+                if (un) b.label[v] = best;
+                const unsigned m = __ballot_sync(DMOLP_FULL_MASK, un);
+                int base = 0;
+                if (lane == 0 && m) {
+                    base = atomicAdd(&b.p1cnt[kFront + par], __popc(m));
+                    atomicAdd(&s_ps[0], __popc(m));  // (any slot: only the sum is used here)
+                }
+                base = __shfl_sync(DMOLP_FULL_MASK, base, 0);
+                if (un) front[base + __popc(m & ((1u << lane) - 1))] = v;
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                const int c = s_ps[0];
+                s_ps[0] = 0;
+                if (c) {
+                    atomicAdd(&b.p1cnt[kLabelled], c);
+                    atomicAdd(&npart2[par][best], c);
+                    atomicAdd((unsigned long long *)&b.psize[best], (unsigned long long)c);
+                }
+            }
+            if (!grid_sync(ctl, a.polls, 26)) return;
+            n = __ldcg(&b.p1cnt[kFront + par]);
+        }
+        bool over = false;
+        for (int p = threadIdx.x; p < k; p += blockDim.x) over |= __ldcg(npart2[par] + p) > theta;
+        over = __syncthreads_or(over);  // (and the cleared counters, and the last round's staged appends are out)
+        const int cap = (n + (int)gridDim.x - 1) / (int)gridDim.x;
+        const int lo = (int)blockIdx.x * cap, hi = min(n, lo + cap);  // this block's frontier slots
+        if (over) {
+            for (int i = lo + (int)threadIdx.x; i < hi; i += blockDim.x) {
+                const int v = front[i];
+                b.bown[i] = b.label[v];
+                b.bkey[i] = ((uint64_t)(unsigned)b.rawdeg[v] << ibits) | (uint64_t)v;
+                b.bsel[i] = 0;
+            }
+            __syncthreads();
+            const int how = select_body<false>(a, n, npart2[par]);
+            if (how == 0) return;
+            if (how == 2 && !grid_sync(ctl, a.polls, 27)) return;  // block 0 marked other blocks' records
+        }
+        // ---- claims of the selected vertices' arcs; the others carry over.  Few rows: eight lanes each; else a
+        //      lane per row of at most kP1Row arcs, eight lanes per longer one ----
+        Append out = {reinterpret_cast<int32_t *>(smem) + wib * kStageP1, next, nnext, 0};  // (the select is done)
+        const bool few = cap <= (int)(blockDim.x >> 3);  // the same in every block
+        const int step = few ? (int)(blockDim.x >> 3) : (int)blockDim.x;
+        for (int i0 = lo + (few ? wib * 4 : wib * 32); i0 < hi; i0 += step) {
+            const int i = i0 + (few ? lane >> 3 : lane);
+            const bool lead = !few || (lane & 7) == 0;
+            int v = 0, p = 0, mine = 0;  // a bit per arc whose neighbour this lane claimed first
+            int64_t s = 0, e = 0;
+            bool carry = false;
+            if (i < hi) {
+                v = front[i];
+                p = b.label[v];
+                if (!over || b.bsel[i]) {
+                    s = b.off[v];
+                    e = b.off[v + 1];
+                    if (lead) te += (unsigned long long)(e - s);
+                    if (e - s > kP1Piece) {
+                        if (lead) queue_row(b, npiece, v, e - s);
+                        e = s;
+                    }
+                } else if (lead) {
+                    carry = true;
+                    atomicAdd(&s_np[p], 1);
+                }
+            }
+            const int deg = (int)(e - s);
+            if (!few && deg <= kP1Row)
+                for (int j = 0; j < deg; j += 8) {
+                    int u[8];
+                    bool f[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) u[q] = j + q < deg ? __ldg(b.col + s + j + q) : -1;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) f[q] = u[q] >= 0 && b.label[u[q]] < 0;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (f[q] && atomicMin(&b.claim[u[q]], p) == INT_MAX) mine |= 1 << (j + q);
+                }
+            const int cnt = carry ? 1 : __popc(mine);
+            if (__any_sync(DMOLP_FULL_MASK, cnt > 0)) {
+                int32_t *slot = out.take(cnt);
+                if (carry) *slot = v;
+                for (unsigned m = (unsigned)mine; m; m &= m - 1) *slot++ = ~__ldg(b.col + s + __ffs(m) - 1);
+            }
+            if (few) {
+                claim_rows<8, 4>(b, p, s, e, out);
+            } else {
+                for (unsigned m = __ballot_sync(DMOLP_FULL_MASK, deg > kP1Row); m;) {
+                    int l = 32;  // the group's row: the (lane / 8)-th of the next four
+                    for (int g = 0; g < 4; ++g) {
+                        if (g == (lane >> 3) && m) l = __ffs(m) - 1;
+                        m &= m - 1;
+                    }
+                    const int src = l & 31;
+                    const int pl = __shfl_sync(DMOLP_FULL_MASK, p, src);
+                    const int64_t sl = __shfl_sync(DMOLP_FULL_MASK, s, src), el = __shfl_sync(DMOLP_FULL_MASK, e, src);
+                    claim_rows<8, 8>(b, pl, sl, l < 32 ? el : sl, out);
+                }
             }
         }
-        claim_arcs(b, p, s, e - s > kChunk ? s + kChunk : e);
+        out.flush();
+        if (!grid_sync(ctl, a.polls, 28)) return;
+        const int np = __ldcg(npiece);
+        if (np) {  // the same in every block
+            for (int q = grid_warp(); q < np; q += grid_warps()) {
+                const int2 c = b.chunkq[q];
+                const int64_t ps = b.off[c.x] + c.y, pe = b.off[c.x + 1];
+                claim_rows<32, 4>(b, b.label[c.x], ps, pe - ps > kP1Piece ? ps + kP1Piece : pe, out);
+            }
+            out.flush();
+            if (!grid_sync(ctl, a.polls, 29)) return;
+        }
+        // ---- claimed vertices take their part ----
+        const int nn = __ldcg(nnext);
+        for (int i = grid_warp() * 32 + lane; i < nn; i += grid_warps() * 32) {
+            const int v = ~next[i];
+            if (v < 0) continue;  // carried over
+            next[i] = v;
+            const int p = __ldcg(b.claim + v);
+            b.label[v] = p;
+            atomicAdd(&s_np[p], 1);
+            atomicAdd(&s_ps[p], 1);
+        }
+        __syncthreads();
+        int labelled = 0;
+        for (int p = threadIdx.x; p < k; p += blockDim.x) {
+            if (s_np[p]) atomicAdd(&npart2[par ^ 1][p], s_np[p]);
+            if (s_ps[p]) atomicAdd((unsigned long long *)&b.psize[p], (unsigned long long)s_ps[p]);
+            labelled += s_ps[p];
+        }
+        for (int o = 16; o > 0; o >>= 1) labelled += __shfl_xor_sync(DMOLP_FULL_MASK, labelled, o);
+        if (lane == 0 && labelled) atomicAdd(&b.p1cnt[kLabelled], labelled);
+        if (blockIdx.x == 0) {  // this round's frontier and the other parity's pieces were read before the last barrier
+            for (int p = threadIdx.x; p < k; p += blockDim.x) npart2[par][p] = 0;
+            if (threadIdx.x == 0) {
+                b.p1cnt[kFront + par] = 0;
+                b.p1cnt[kPieces + (par ^ 1)] = 0;
+            }
+        }
+        if (!grid_sync(ctl, a.polls, 30)) return;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) b.p1cnt[kRounds] = rounds;
     te = warp_sum_u64(te);
     if (lane == 0 && te) atomicAdd(b.p1te, te);
 }
 
-// Warp per queued piece of a long frontier row.
-__global__ void k_p1_claim_chunks(Buffers b, int cur) {
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-    const int n = b.p1cnt[5];
-    const int32_t *front = b.win[cur];
-    for (int q = gw; q < n; q += nw) {
-        const int2 c = b.chunkq[q];
-        const int u = front[c.x];
-        const int64_t rs = b.off[u], re = b.off[u + 1];
-        const int64_t s = rs + c.y;
-        claim_arcs(b, b.bown[c.x], s, re - s > kChunk ? s + kChunk : re);
-    }
+size_t grow_smem(int k, int *off) {
+    const size_t stage = (size_t)(kSelThreads / 32) * kStageP1 * sizeof(int32_t);
+    const size_t sel = std::max((select_smem_bytes(k) + 15) & ~(size_t)15, stage);
+    if (off) *off = (int)(sel / sizeof(int));
+    return sel + 2 * (size_t)k * sizeof(int);
 }
 
-// Claimed vertices take their part and join the next frontier; unselected frontier vertices carry over.
-__global__ void k_p1_commit(Buffers b, int cur) {
-    const int nclaim = b.p1cnt[2], nfront = b.p1cnt[0];
-    int32_t *next = b.win[cur ^ 1];
-    const int32_t *front = b.win[cur];
-    for (int i0 = blockIdx.x * blockDim.x; i0 < nclaim; i0 += gridDim.x * blockDim.x) {
-        const int i = i0 + threadIdx.x;
-        int v = 0, p = 0;
-        const bool ok = i < nclaim;
-        if (ok) {
-            v = b.cand[i];
-            p = b.claim[v];
-            b.label[v] = p;
-            b.claim[v] = INT_MAX;
-            atomicAdd((unsigned long long *)&b.psize[p], 1ull);
-        }
-        const int slot = warp_append(&b.p1cnt[1], ok);
-        if (ok) next[slot] = v;
-        const int c = __popc(__ballot_sync(DMOLP_FULL_MASK, ok));
-        if ((threadIdx.x & 31) == 0 && c) atomicAdd(&b.p1cnt[3], c);
-    }
-    for (int i0 = blockIdx.x * blockDim.x; i0 < nfront; i0 += gridDim.x * blockDim.x) {
-        const int i = i0 + threadIdx.x;
-        const bool carry = i < nfront && !b.bsel[i];
-        const int slot = warp_append(&b.p1cnt[1], carry);
-        if (carry) next[slot] = front[i];
-    }
+// All blocks are resident: at most one per SM, a cooperative launch.
+template <typename K, typename... A>
+void launch_resident(dmolp_ctx *c, K kernel, size_t smem, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)std::min<int64_t>(c->num_sms, std::max<int64_t>(8, (c->nv + kP1BlockV - 1) / kP1BlockV)));
+    cfg.blockDim = dim3(kSelThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    if (e != cudaSuccess && c->launch_error == cudaSuccess) c->launch_error = e;  // reported by the entry point
+    c->launches += 1;
 }
-
-// Next round: the next frontier becomes current.
-__global__ void k_p1_advance(Buffers b) {
-    b.p1cnt[0] = b.p1cnt[1];
-    b.p1cnt[1] = 0;
-    b.p1cnt[2] = 0;
-    b.p1cnt[5] = 0;
-}
-
-int grid_for(dmolp_ctx *c) { return c->num_sms * 4; }
 
 }  // namespace
 
-void p1_mark_ball(dmolp_ctx *c, int seed) {
-    k_p1_level1<<<c->num_sms, 256, 0, c->stream>>>(c->b, seed);
-    k_p1_level2<<<grid_for(c), kBlock, 0, c->stream>>>(c->b, seed);
-    c->launches += 2;
+void p1_find_seeds(dmolp_ctx *c, int k, int first, int64_t nhubs) {
+    launch_resident(c, k_p1_find_seeds, 0, c->b, k, first, (int)nhubs, c->wait_polls);
 }
 
-void p1_hub_argmax(dmolp_ctx *c, int64_t nhubs) {
-    cudaMemsetAsync(c->b.best, 0, sizeof(unsigned long long), c->stream);
-    k_p1_hub_argmax<<<grid_for(c), kBlock, 0, c->stream>>>(c->b, nhubs);
-    c->launches += 1;
+void p1_grow(dmolp_ctx *c, int k, int theta) {
+    int off = 0;
+    const size_t smem = grow_smem(k, &off);
+    SelArgs a = select_args(c, k, c->rbits + c->ibits);
+    a.theta = theta;
+    launch_resident(c, k_p1_grow, smem, c->b, a, (int)c->nv, k, theta, c->ibits, off);
 }
 
-void p1_init_labels(dmolp_ctx *c) {
-    k_p1_init<<<grid_for(c), kBlock, 0, c->stream>>>(c->b, (int)c->nv);
-    c->launches += 1;
-}
-
-void p1_set_seeds(dmolp_ctx *c, const int32_t *seeds_dev, int nseeds) {
-    k_p1_seeds<<<1, 32, 0, c->stream>>>(c->b, seeds_dev, nseeds);
-    c->launches += 1;
-}
-
-void p1_fallback(dmolp_ctx *c, int best_part, int cur) {
-    // the current frontier is empty (checked by the caller), so appending starts at 0 in win[cur]
-    k_p1_fallback<<<grid_for(c), kBlock, 0, c->stream>>>(c->b, (int)c->nv, best_part, cur);
-    c->launches += 1;
-}
-
-// One expansion round on frontier buffer `cur` (the frontier lives in win[cur], its size in p1cnt[0]).
-void p1_round(dmolp_ctx *c, int k, int theta, int cur) {
-    const int grid = grid_for(c);
-    k_p1_records<<<grid, kBlock, (size_t)k * sizeof(int), c->stream>>>(c->b, cur, c->ibits, k);
-    k_p1_need<<<1, 256, 0, c->stream>>>(c->b, k, theta);
-    c->launches += 2;
-    select_smallest(c, c->b.bown, c->b.bkey, &c->b.p1cnt[4], k, c->rbits + c->ibits, c->b.bsel, nullptr);
-    k_p1_claim<<<grid, kBlock, 0, c->stream>>>(c->b, cur);
-    k_p1_claim_chunks<<<grid, kBlock, 0, c->stream>>>(c->b, cur);
-    k_p1_commit<<<grid, kBlock, 0, c->stream>>>(c->b, cur);
-    k_p1_advance<<<1, 1, 0, c->stream>>>(c->b);
-    c->launches += 4;
+void p1_prepare() {
+    size_t m = 0;
+    for (int k : {kSmemSegMax, (int)DMOLP_MAX_K}) m = std::max(m, grow_smem(k, nullptr));
+    cudaFuncSetAttribute(k_p1_grow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m);
 }
 
 }  // namespace dmolp
