@@ -31,7 +31,7 @@ GENCODE = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", *GENCODE, "-Xcompiler", "-fPIC,-fno-fast-math,-ffp-contract=off",
               "--expt-relaxed-constexpr", "-Xptxas", "-v"]
 
-CUDA_SOURCES = ["dmolp_cabi.cu", "lp_kernels.cu", "seed_kernels.cu", "select_kernels.cu", "adjtext.cpp",
+CUDA_SOURCES = ["dmolp_cabi.cu", "lp_kernels.cu", "lp_loop.cu", "seed_kernels.cu", "select_kernels.cu", "adjtext.cpp",
                 "noalloc.cu", "ingest.cu", "hubsort.cpp", "batch_kernels.cu", "batch_cabi.cu", "batch_p1.cu", "features.cu", "decode.cu", "mpnn_kernels.cu", "mpnn_cabi.cu"]
 CUDA_HEADERS = ["common.cuh", "device_state.cuh", "kernels.cuh", "lp_device.cuh", "select_radix.cuh", "batch.cuh", "team.cuh", "mpnn.cuh", "umma.cuh", "ingest.cuh"]
 DROPIN_SOURCES = ["dropin.cpp"]

@@ -25,6 +25,14 @@ constexpr int kP1Piece = 512;    // phase 1: longer rows are split into pieces o
 constexpr int kHotMax = 16384;   // LP gathers: labels of up to this many highest-degree vertices per block
 constexpr int kHubChunk = 2048;  // row chunk of the decisions of deg > kLargeDeg vertices
 
+// The LP loop in one launch (lp_loop.cu): graphs of at most this many arcs have its buffers
+constexpr int64_t kLoopMaxArcs = 8 << 20;
+constexpr int kLoopShort = 32;   // its rows of more arcs ...
+constexpr int kLoopPiece = 256;  // ... are split into pieces of this many
+constexpr int kLoopMinIters = 4;
+constexpr size_t kLoopCntBytes = 256;
+inline size_t loop_pieces(int64_t narcs) { return (size_t)narcs / kLoopShort + 2; }
+
 // Polls of a grid-barrier generation word before the barrier gives up (about a second on B200).
 constexpr unsigned int kDefaultWaitPolls = 1u << 22;
 
@@ -58,7 +66,7 @@ struct LpControl {
     int mode;           // DMOLP_LP_MODE_*
     int pull;           // next iteration finds candidates by pulling (rows scanned for a window member)
     int sel_open[2];    // radix select: segments still needing records after a pass (by pass parity)
-    unsigned int bar_count, bar_gen;  // grid barrier of the cooperative selection kernel
+    unsigned int bar_count;  // grid barrier of the cooperative kernels
     int wait_timeout;   // a grid barrier gave up waiting (1 + the barrier's index in the kernel)
     int sel_tail;       // radix select: records appended to the list that block 0 finishes alone
 };
@@ -118,6 +126,12 @@ struct Buffers {
     // kept current by k_update
     uint16_t *vcnt = nullptr;      // [nv * 32]
     int32_t *active[2] = {nullptr, nullptr};  // [nv] radix-select active lists
+    // the LP loop in one launch: (vertex, degree) of the vertices with arcs by degree (ascending, descending), ids
+    // ascending among equals; record counts per label (or digit) and block; queued row pieces; counters
+    int2 *lpasc = nullptr, *lpdesc = nullptr;  // [record slots] each
+    int *lpblk = nullptr;                      // [max(MAX_K, 256) * num_sms]
+    int2 *lppiece = nullptr;                   // [2 * loop_pieces(narcs)]
+    void *lpcnt = nullptr;                     // [kLoopCntBytes]
     // per-part arrays (DMOLP_MAX_K); vc / intra hold signed values in two's complement
     unsigned int *hist = nullptr;        // [kSelHistBuffers * MAX_K * 256] radix-select histograms
     // degree-bin window selection (k <= kDegSelMaxK): superbin counts of the boundary records per label
@@ -176,6 +190,7 @@ struct dmolp_ctx {
     bool counts_kept = false;             // the current LP run decides from vcnt / hh (no label gathers)
     unsigned int wait_polls = dmolp::kDefaultWaitPolls;  // polls of a grid barrier before it gives up
     int nhot = 0;                         // hot vertices
+    bool loop_ordered = false;            // lpasc / lpdesc are built for the resident graph
     int lp_runs = 0;                      // dmolp_lp_run calls on the resident graph
     std::vector<int32_t> h_rawdeg;        // host copy for the hub sort
     bool h_rawdeg_valid = false;          // h_rawdeg mirrors the resident raw degrees
@@ -207,6 +222,7 @@ struct dmolp_ctx {
     long long prof_launches[5] = {0, 0, 0, 0, 0};
     double prof_bytes[5] = {0, 0, 0, 0, 0};
     cudaError_t launch_error = cudaSuccess;  // first failed launch that returns no status to its caller
+    char *h_res = nullptr;                 // pinned copy of the result buffers (dmolp_cabi.cu, fetch)
     void *arena = nullptr;                 // every resident buffer of the graph (layout in graph_alloc)
     size_t arena_cap = 0;
     dmolp::ingest::Pool scratch;           // device scratch of the text parse, reused across loads

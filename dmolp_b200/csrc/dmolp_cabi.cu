@@ -102,20 +102,16 @@ int clear_select_bins(dmolp_ctx *c) {
 // A grid barrier of a cooperative selection that gave up waiting (its blocks are co-resident, so only a
 // wait limit far below the default makes this happen): report it, and clear the barrier state and the
 // selections' counts for the next launch.
-int check_waits(dmolp_ctx *c) {
+int report_waits(dmolp_ctx *c, int to) {
     if (c->launch_error != cudaSuccess) {
         const cudaError_t e = c->launch_error;
         c->launch_error = cudaSuccess;
         cudaGetLastError();
         return fail(DMOLP_ERR_CUDA, std::string("window selection launch: ") + cudaGetErrorString(e));
     }
-    int to = 0;
-    DMOLP_CUDA(cudaMemcpyAsync(&to, &c->b.ctrl->wait_timeout, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    int st = sync(c);
-    if (st) return st;
     if (!to) return DMOLP_OK;
-    // bar_count, bar_gen, wait_timeout are adjacent
-    DMOLP_CUDA(cudaMemsetAsync(&c->b.ctrl->bar_count, 0, 3 * sizeof(int), c->stream));
+    // bar_count and wait_timeout are adjacent
+    DMOLP_CUDA(cudaMemsetAsync(&c->b.ctrl->bar_count, 0, 2 * sizeof(int), c->stream));
     DMOLP_CUDA(cudaMemsetAsync(c->b.hist, 0, (size_t)kSelHistBuffers * DMOLP_MAX_K * kRadix * sizeof(unsigned int),
                                c->stream));
     int st2 = clear_select_bins(c);
@@ -124,6 +120,27 @@ int check_waits(dmolp_ctx *c) {
     return fail(DMOLP_ERR_CUDA, "grid barrier " + std::to_string(to - 1) +
                                     " of a window selection gave up waiting (wait limit " +
                                     std::to_string(c->wait_polls) + " polls)");
+}
+
+int check_waits(dmolp_ctx *c) {
+    int to = 0;
+    DMOLP_CUDA(cudaMemcpyAsync(&to, &c->b.ctrl->wait_timeout, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    const int st = sync(c);
+    return st ? st : report_waits(c, to);
+}
+
+// The result buffers (b.need up to `end`) to the context's pinned copy, and a wait for the stream: one copy where
+// one per buffer, staged through pageable memory, cost 8 to 10 us each.  host_of(c, p) is then p's copy.
+constexpr size_t kResBytes = 32768 + kMaxIter * sizeof(LpRecordDev);
+int fetch(dmolp_ctx *c, const void *end) {
+    const size_t n = (const char *)end - (const char *)c->b.need;
+    if (n > kResBytes) return fail(DMOLP_ERR_STATE, "result buffers larger than their host copy");
+    DMOLP_CUDA(cudaMemcpyAsync(c->h_res, c->b.need, n, cudaMemcpyDeviceToHost, c->stream));
+    return sync(c);
+}
+template <typename T>
+const T *host_of(const dmolp_ctx *c, const T *p) {
+    return reinterpret_cast<const T *>(c->h_res + (reinterpret_cast<const char *>(p) - reinterpret_cast<const char *>(c->b.need)));
 }
 
 // The reference's balance = max over parts of count / expected (src/phase2/phase2.cpp:426-432).
@@ -151,27 +168,21 @@ void balances(const std::vector<long long> &vc, const std::vector<long long> &ec
 
 // Fused cut/balance pass over the resident labels; fills host copies.  Returns the status.
 int run_stats(dmolp_ctx *c, int k, unsigned long long *cut_arcs, std::vector<long long> &vc,
-              std::vector<long long> &intra, int *bad) {
+              std::vector<long long> &intra, int *bad, cudaEvent_t done = nullptr) {
     lp_reset_stats(c, k, nullptr);
     lp_stats(c, k, nullptr, nullptr);
-    std::vector<unsigned long long> hv(k), hi(k);
-    LpCounters cn;
-    LpControl ctl;
-    DMOLP_CUDA(cudaMemcpyAsync(hv.data(), c->b.vc, k * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-    DMOLP_CUDA(cudaMemcpyAsync(hi.data(), c->b.intra, k * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                               c->stream));
-    DMOLP_CUDA(cudaMemcpyAsync(&cn, c->b.cnt, sizeof(cn), cudaMemcpyDeviceToHost, c->stream));
-    DMOLP_CUDA(cudaMemcpyAsync(&ctl, c->b.ctrl, sizeof(ctl), cudaMemcpyDeviceToHost, c->stream));
-    int st = sync(c);
+    if (done) DMOLP_CUDA(cudaEventRecord(done, c->stream));
+    const int st = fetch(c, c->b.rec);
     if (st) return st;
+    const unsigned long long *hv = host_of(c, c->b.vc), *hi = host_of(c, c->b.intra);
     vc.assign(k, 0);
     intra.assign(k, 0);
     for (int p = 0; p < k; ++p) {
         vc[p] = (long long)hv[p];
         intra[p] = (long long)hi[p];
     }
-    *cut_arcs = cn.cut_arcs;
-    *bad = ctl.error;
+    *cut_arcs = host_of(c, c->b.cnt)->cut_arcs;
+    *bad = host_of(c, c->b.ctrl)->error;
     return DMOLP_OK;
 }
 
@@ -266,11 +277,8 @@ size_t layout(dmolp_ctx *c, char *base, int64_t nv, int64_t narcs, const size_t 
     ALLOC(b.dtcnt, 2 * kDegSelMaxK);
     ALLOC(b.dlkey, n);
     ALLOC(b.dtkey, n);
-    ALLOC(b.need, DMOLP_MAX_K);
     ALLOC(b.sel_below, DMOLP_MAX_K);
     ALLOC(b.npart, DMOLP_MAX_K);
-    ALLOC(b.vc, DMOLP_MAX_K);
-    ALLOC(b.intra, DMOLP_MAX_K);
     ALLOC(b.psize, DMOLP_MAX_K);
     ALLOC(b.tpen, DMOLP_MAX_K);
     ALLOC(b.RE, DMOLP_MAX_K);
@@ -278,14 +286,18 @@ size_t layout(dmolp_ctx *c, char *base, int64_t nv, int64_t narcs, const size_t 
     ALLOC(b.cnthist, (size_t)kMaxIter * 2 * DMOLP_MAX_K);
     ALLOC(b.logtab, kMaxIter + 1);
     ALLOC(b.ratiotab, kMaxIter + 1);
-    ALLOC(b.cnt, 1);
-    ALLOC(b.ctrl, 1);
-    ALLOC(b.rec, kMaxIter);
     ALLOC(b.covered, n);
     ALLOC(b.hubs, n);
     ALLOC(b.best, 2);
+    // what calls return, side by side: one copy to the host (fetch)
+    ALLOC(b.need, DMOLP_MAX_K);
+    ALLOC(b.vc, DMOLP_MAX_K);
+    ALLOC(b.intra, DMOLP_MAX_K);
+    ALLOC(b.cnt, 1);
+    ALLOC(b.ctrl, 1);
     ALLOC(b.p1cnt, 8);
     ALLOC(b.p1te, 1);
+    ALLOC(b.rec, kMaxIter);
     ALLOC(b.flag, 1);
     ALLOC(b.symcnt, 2);
     ALLOC(b.ball, nball[0] + nball[1] + nball[2]);
@@ -310,6 +322,16 @@ size_t layout(dmolp_ctx *c, char *base, int64_t nv, int64_t narcs, const size_t 
     ALLOC(b.hotlab, kHotMax);
     ALLOC(b.degh, 65536);
     ALLOC(b.vcnt, n * 32);
+    if (narcs <= kLoopMaxArcs) {
+        const size_t npos = nball[0] + nball[1] + nball[2];
+        ALLOC(b.lpasc, npos);
+        ALLOC(b.lpdesc, npos);
+        ALLOC(b.lpblk, (size_t)c->num_sms * DMOLP_MAX_K);
+        ALLOC(b.lppiece, 2 * loop_pieces(narcs));
+        char *cnt = nullptr;
+        ALLOC(cnt, kLoopCntBytes);
+        b.lpcnt = cnt;
+    }
 #undef ALLOC
     return off;
 }
@@ -372,6 +394,7 @@ int graph_finish(dmolp_ctx *c, bool rows_sorted) {
     c->hot_ready = false;
     c->nhot = 0;
     c->lp_runs = 0;
+    c->loop_ordered = false;
     lp_hub_index(c);
     select_prepare();
     // whether every arc has its reverse is tested when the LP loop first needs it (ensure_symmetry)
@@ -565,6 +588,7 @@ int dmolp_create(int device, dmolp_ctx **out) {
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
+    if (e == cudaSuccess) e = cudaHostAlloc((void **)&c->h_res, kResBytes, cudaHostAllocDefault);
     if (e != cudaSuccess) {
         delete c;
         return fail(DMOLP_ERR_CUDA, std::string("stream/event: ") + cudaGetErrorString(e));
@@ -584,6 +608,7 @@ int dmolp_destroy(dmolp_ctx *c) {
         if (c->pin[i]) cudaFreeHost(c->pin[i]);
         if (c->pin_ev[i]) cudaEventDestroy(c->pin_ev[i]);
     }
+    if (c->h_res) cudaFreeHost(c->h_res);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -928,13 +953,11 @@ static int find_seeds_impl(dmolp_ctx *c, int k, int first, const std::vector<int
     DMOLP_CUDA(cudaMemsetAsync(b.best, 0, 2 * sizeof(unsigned long long), c->stream));
     DMOLP_CUDA(cudaMemsetAsync(b.p1cnt, 0, 8 * sizeof(int), c->stream));
     p1_find_seeds(c, k, first, (int64_t)hubs.size());
-    std::vector<int> out(k);
-    int cnt[8];
-    DMOLP_CUDA(cudaMemcpyAsync(out.data(), b.need, (size_t)k * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    DMOLP_CUDA(cudaMemcpyAsync(cnt, b.p1cnt, sizeof(cnt), cudaMemcpyDeviceToHost, c->stream));
-    const int st = check_waits(c);
+    int st = fetch(c, b.rec);
+    if (!st) st = report_waits(c, host_of(c, b.ctrl)->wait_timeout);
     if (st) return st;
-    seeds.assign(out.begin(), out.begin() + cnt[6]);
+    const int32_t *out = host_of(c, b.need);
+    seeds.assign(out, out + host_of(c, b.p1cnt)[6]);
     return DMOLP_OK;
 }
 
@@ -976,16 +999,12 @@ static void complete_seeds(dmolp_ctx *c, int k, const std::vector<int> &hubs, st
     }
 }
 
-// Growth rounds (partition.cpp:335-604); seedk[p] = -1 for a part without a seed.
-static int expand_impl(dmolp_ctx *c, int k, int theta, const std::vector<int32_t> &seedk, int *rounds_out) {
-    Buffers &b = c->b;
-    const int64_t nv = c->nv;
-    *rounds_out = 0;
-    if (nv <= 0) return DMOLP_OK;
-    DMOLP_CUDA(cudaMemcpyAsync(b.need, seedk.data(), k * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
+// Growth rounds (partition.cpp:335-604); seedk[p] = -1 for a part without a seed.  Launched only: the rounds are
+// p1cnt[5], the caller checks the kernel's waits.
+static int expand_impl(dmolp_ctx *c, int k, int theta, const std::vector<int32_t> &seedk) {
+    DMOLP_CUDA(cudaMemcpyAsync(c->b.need, seedk.data(), k * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
     p1_grow(c, k, theta);
-    DMOLP_CUDA(cudaMemcpyAsync(rounds_out, b.p1cnt + 5, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    return check_waits(c);
+    return DMOLP_OK;
 }
 
 static int check_seed_args(dmolp_ctx *c, int k) {
@@ -1026,9 +1045,12 @@ int dmolp_expand_partitions(dmolp_ctx *c, int k, int theta, const int32_t *seeds
         seedk[p] = seeds[p];
     }
     DMOLP_CUDA(cudaSetDevice(c->device));
-    int r = 0;
-    st = expand_impl(c, k, theta, seedk, &r);
-    if (rounds) *rounds = r;
+    if (rounds) *rounds = 0;
+    if (c->nv == 0) return DMOLP_OK;
+    st = expand_impl(c, k, theta, seedk);
+    if (!st) st = fetch(c, c->b.rec);
+    if (!st) st = report_waits(c, host_of(c, c->b.ctrl)->wait_timeout);
+    if (!st && rounds) *rounds = host_of(c, c->b.p1cnt)[5];
     return st;
 }
 
@@ -1073,22 +1095,20 @@ int dmolp_phase1(dmolp_ctx *c, int k, int theta, int32_t *seeds_out, int64_t *ve
     std::vector<int32_t> seedk(k, -1);
     for (int p = 0; p < k && p < (int)seeds.size(); ++p) seedk[p] = seeds[p];
     if (seeds_out) std::copy(seedk.begin(), seedk.end(), seeds_out);
-    int rounds = 0;
-    st = expand_impl(c, k, theta, seedk, &rounds);
-    if (st) return st;
-    inf.rounds = rounds;
+    if (nv > 0) {
+        st = expand_impl(c, k, theta, seedk);
+        if (st) return st;
+    }
 
     // ---- initial metrics (phase1.cpp:83-153) ----
     unsigned long long arcs = 0;
     std::vector<long long> vc, intra;
     int bad = 0;
-    st = run_stats(c, k, &arcs, vc, intra, &bad);
+    st = run_stats(c, k, &arcs, vc, intra, &bad, c->ev1);
+    if (!st) st = report_waits(c, host_of(c, b.ctrl)->wait_timeout);
     if (st) return st;
-    DMOLP_CUDA(cudaEventRecord(c->ev1, c->stream));
-    unsigned long long te = 0;
-    DMOLP_CUDA(cudaMemcpyAsync(&te, b.p1te, sizeof(te), cudaMemcpyDeviceToHost, c->stream));
-    st = sync(c);
-    if (st) return st;
+    const unsigned long long te = *host_of(c, b.p1te);
+    inf.rounds = nv > 0 ? host_of(c, b.p1cnt)[5] : 0;
     float ms = 0;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
     inf.gpu_ms = ms;
@@ -1118,6 +1138,16 @@ int dmolp_phase1(dmolp_ctx *c, int k, int theta, int32_t *seeds_out, int64_t *ve
     return DMOLP_OK;
 }
 
+// Whether the run's iterations go in one launch (lp_loop.cu).  Below kLoopMaxArcs arcs the launches' fixed work is
+// what counts: a mesh of 0.76 M arcs, 20 iterations 1.17 -> 0.49 ms; preferential attachment of 6.4 M arcs, 48 labels
+// 2.83 -> 1.91 ms; a skewed graph of 7.5 M arcs, 64 parts 1.36 -> 1.10 ms.  Above it the launch per step wins, with
+// its pulled candidates and hub windows instead of a stamp per arc (a skewed graph of 14 M arcs 1.29 ms, here 1.76).
+// A run of fewer than kLoopMinIters iterations does not earn the slot orders (40 us).  Asymmetric graphs recount from
+// the arcs each iteration, and timed launches (profiling) are those of the launch per step.
+static bool use_loop(const dmolp_ctx *c, int iters) {
+    return c->symmetric && !c->profiling && c->narcs > 0 && c->narcs <= kLoopMaxArcs && iters >= kLoopMinIters;
+}
+
 int dmolp_lp_run(dmolp_ctx *c, int k, const dmolp_lp_config *cfg, dmolp_lp_result *res, dmolp_lp_record *records,
                  int max_records) {
     if (!c || !c->has_graph) return fail(DMOLP_ERR_STATE, "no graph uploaded");
@@ -1138,62 +1168,70 @@ int dmolp_lp_run(dmolp_ctx *c, int k, const dmolp_lp_config *cfg, dmolp_lp_resul
     const int max_iter = cfg->mode == DMOLP_LP_MODE_REF ? kMaxIter : cfg->iterations;
 
     DMOLP_CUDA(cudaEventRecord(c->ev0, c->stream));
-    DMOLP_CUDA(cudaMemsetAsync(b.stamp, 0, (size_t)(c->nv + 1) * sizeof(int32_t), c->stream));
-    DMOLP_CUDA(cudaMemsetAsync(b.sstamp, 0, (size_t)(c->nv + 1) * sizeof(int32_t), c->stream));
-    st = clear_select_bins(c);
-    if (st) return st;
-    DMOLP_CUDA(cudaMemsetAsync(b.ndiff, 0, (size_t)(c->nv + 1) * sizeof(int32_t), c->stream));
-    if (c->nb[2] > 0) {
-        DMOLP_CUDA(cudaMemsetAsync(b.hubwin, 0, (size_t)(c->nv + 1) * sizeof(int32_t), c->stream));
-        DMOLP_CUDA(cudaMemsetAsync(b.hub_in, 0, (size_t)c->nb[2] * sizeof(int32_t), c->stream));
-    }
     // symmetric graphs with at most 32 scored labels decide from kept label counts (no label gathers)
     c->counts_kept = c->symmetric && L.eff <= 32;
-    // The hot set (the labels of the highest-degree vertices in shared memory, a full pass over the arcs to
-    // build) pays off when the decisions gather labels, or over several runs on the graph; the first run of
-    // a kept-count graph goes without it.
-    if (!c->counts_kept || c->lp_runs > 0) {
-        st = lp_hot_prepare(c);
+    const bool loop = use_loop(c, max_iter);
+    if (loop) {
+        if (!c->loop_ordered) loop_order(c);
+        c->loop_ordered = true;
+        lp_reset_stats(c, k, nullptr);
+        lp_stats(c, k, nullptr, nullptr, false, c->counts_kept ? L.eff : 0, L.eff);
+        loop_run(c, L, max_iter);
+        st = check_launch(c);
         if (st) return st;
-    }
-    ++c->lp_runs;
-    lp_hot_refresh(c);
-    lp_reset_stats(c, k, nullptr);
-    // the run-start pass also counts every hub's row into hh on symmetric graphs (kept from the movers after)
-    lp_stats(c, k, nullptr, nullptr, true, c->counts_kept ? L.eff : 0, c->symmetric ? L.eff : 0);
-    lp_init_end(c, cfg->mode);
-    st = check_launch(c);
-    if (st) return st;
-    int stopped = 0;
-    // Iterations in blocks: FIXED mode one block of all iterations, REF mode blocks of 8 with a check of
-    // the stop flag in between.  Each block is captured into a CUDA graph once and replayed afterwards.
-    const int block = cfg->mode == DMOLP_LP_MODE_REF ? 8 : std::max(1, max_iter);
-    for (int t0 = 1; t0 <= max_iter; t0 += block) {
-        const int cnt = std::min(block, max_iter - t0 + 1);
-        if (c->use_graphs) {
-            st = run_block_graph(c, L, t0, cnt);
-            if (st) return st;
-        } else {
-            for (int t = t0; t < t0 + cnt; ++t) lp_iteration(c, L, t, t == t0, t == t0 + cnt - 1);
+    } else {
+        DMOLP_CUDA(cudaMemsetAsync(b.stamp, 0, (size_t)(c->nv + 1) * sizeof(int32_t), c->stream));
+        DMOLP_CUDA(cudaMemsetAsync(b.sstamp, 0, (size_t)(c->nv + 1) * sizeof(int32_t), c->stream));
+        st = clear_select_bins(c);
+        if (st) return st;
+        DMOLP_CUDA(cudaMemsetAsync(b.ndiff, 0, (size_t)(c->nv + 1) * sizeof(int32_t), c->stream));
+        if (c->nb[2] > 0) {
+            DMOLP_CUDA(cudaMemsetAsync(b.hubwin, 0, (size_t)(c->nv + 1) * sizeof(int32_t), c->stream));
+            DMOLP_CUDA(cudaMemsetAsync(b.hub_in, 0, (size_t)c->nb[2] * sizeof(int32_t), c->stream));
         }
-        if (cfg->mode == DMOLP_LP_MODE_REF && t0 + cnt <= max_iter) {
-            DMOLP_CUDA(cudaMemcpyAsync(&stopped, &b.ctrl->stopped, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-            st = sync(c);
+        // The hot set (the labels of the highest-degree vertices in shared memory, a full pass over the arcs to
+        // build) pays off when the decisions gather labels, or over several runs on the graph; the first run of
+        // a kept-count graph goes without it.
+        if (!c->counts_kept || c->lp_runs > 0) {
+            st = lp_hot_prepare(c);
             if (st) return st;
-            if (stopped) break;
+        }
+        ++c->lp_runs;
+        lp_hot_refresh(c);
+        lp_reset_stats(c, k, nullptr);
+        // the run-start pass also counts every hub's row into hh on symmetric graphs (kept from the movers after)
+        lp_stats(c, k, nullptr, nullptr, true, c->counts_kept ? L.eff : 0, c->symmetric ? L.eff : 0);
+        lp_init_end(c, cfg->mode);
+        st = check_launch(c);
+        if (st) return st;
+        int stopped = 0;
+        // Iterations in blocks: FIXED mode one block of all iterations, REF mode blocks of 8 with a check of
+        // the stop flag in between.  Each block is captured into a CUDA graph once and replayed afterwards.
+        const int block = cfg->mode == DMOLP_LP_MODE_REF ? 8 : std::max(1, max_iter);
+        for (int t0 = 1; t0 <= max_iter; t0 += block) {
+            const int cnt = std::min(block, max_iter - t0 + 1);
+            if (c->use_graphs) {
+                st = run_block_graph(c, L, t0, cnt);
+                if (st) return st;
+            } else {
+                for (int t = t0; t < t0 + cnt; ++t) lp_iteration(c, L, t, t == t0, t == t0 + cnt - 1);
+            }
+            if (cfg->mode == DMOLP_LP_MODE_REF && t0 + cnt <= max_iter) {
+                DMOLP_CUDA(cudaMemcpyAsync(&stopped, &b.ctrl->stopped, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+                st = sync(c);
+                if (st) return st;
+                if (stopped) break;
+            }
         }
     }
     DMOLP_CUDA(cudaEventRecord(c->ev1, c->stream));
-    LpControl ctl;
-    DMOLP_CUDA(cudaMemcpyAsync(&ctl, b.ctrl, sizeof(ctl), cudaMemcpyDeviceToHost, c->stream));
-    std::vector<unsigned long long> hv(k), hi(k);
-    DMOLP_CUDA(cudaMemcpyAsync(hv.data(), b.vc, k * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-    DMOLP_CUDA(cudaMemcpyAsync(hi.data(), b.intra, k * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream));
-    std::vector<LpRecordDev> recs(kMaxIter);
-    DMOLP_CUDA(cudaMemcpyAsync(recs.data(), b.rec, kMaxIter * sizeof(LpRecordDev), cudaMemcpyDeviceToHost, c->stream));
-    st = sync(c);
+    st = fetch(c, b.rec + kMaxIter);
     if (st) return st;
-    if (ctl.wait_timeout || c->launch_error != cudaSuccess) return check_waits(c);
+    const LpControl &ctl = *host_of(c, b.ctrl);
+    const unsigned long long *hv = host_of(c, b.vc), *hi = host_of(c, b.intra);
+    const LpRecordDev *recs = host_of(c, b.rec);
+    st = report_waits(c, ctl.wait_timeout);
+    if (st) return st;
     if (ctl.error) return fail(DMOLP_ERR_BAD_LABELS, "label outside [0,k) or odd cut-arc count");
     float ms = 0;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);

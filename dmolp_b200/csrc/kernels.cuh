@@ -76,6 +76,11 @@ void lp_iteration(dmolp_ctx *c, const LpLaunch &L, int t, bool first, bool last)
 void lp_window_from_list(dmolp_ctx *c, int k, int t, const double *RE_dev, int nprev);
 void lp_apply_list(dmolp_ctx *c, int k, int eff, int n);
 
+// ---- LP loop in one launch (lp_loop.cu) ----
+void loop_order(dmolp_ctx *c);  // slot orders (once per graph)
+void loop_run(dmolp_ctx *c, const LpLaunch &L, int iters);  // every iteration, after the run-start statistics pass
+void loop_prepare();  // kernel attributes
+
 // ---- phase 1 (seed_kernels.cu) ----
 // Seeds by the reference rule from b.hubs[0, nhubs) and the first seed: b.need[0, found), found = p1cnt[6].
 // b.covered, b.best and p1cnt are cleared by the caller.

@@ -1035,9 +1035,13 @@ __global__ void __launch_bounds__(256, 4) k_stats(Buffers b, StatsArgs a, const 
         } else {
             const int wpb = blockDim.x >> 5;
             const int gw = (bx - a.gv - a.g0) * wpb + wib, nw = a.g1 * wpb;
-            for (int i0 = gw * 32; i0 < a.nb1; i0 += nw * 32) {
+            // rows per warp and step: all warps take part where there are fewer than 32 rows for each (a warp walks
+            // its long rows one after another; with 32 each, the early vertices of a preferential-attachment graph
+            // of 150 K, which are the long rows, kept a few warps at it for 300 us)
+            const int R = min(32, (a.nb1 + nw - 1) / nw);
+            for (int i0 = gw * R; i0 < a.nb1; i0 += nw * R) {
                 const int i = i0 + lane;
-                const bool valid = i < a.nb1;
+                const bool valid = lane < R && i < a.nb1;
                 int v = 0, lv = 0;
                 int64_t s = 0, e = 0;
                 if (valid) {

@@ -641,6 +641,7 @@ void select_prepare() {
     cudaFuncSetAttribute(k_select_deg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ds_smem_bytes(kDegSelMaxK));
     cudaFuncSetAttribute(k_select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)select_smem_bytes(kSmemSegMax));
     p1_prepare();
+    loop_prepare();
 }
 
 }  // namespace dmolp
