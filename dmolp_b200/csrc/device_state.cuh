@@ -222,6 +222,9 @@ struct dmolp_ctx {
     long long prof_launches[5] = {0, 0, 0, 0, 0};
     double prof_bytes[5] = {0, 0, 0, 0, 0};
     cudaError_t launch_error = cudaSuccess;  // first failed launch that returns no status to its caller
+    // pinned staging of dmolp_graph_upload (allocated by the first upload that uses it)
+    char *up[3] = {nullptr, nullptr, nullptr};
+    cudaEvent_t up_ev[3] = {nullptr, nullptr, nullptr};
     char *h_res = nullptr;                 // pinned copy of the result buffers (dmolp_cabi.cu, fetch)
     void *arena = nullptr;                 // every resident buffer of the graph (layout in graph_alloc)
     size_t arena_cap = 0;
@@ -231,5 +234,7 @@ struct dmolp_ctx {
     cudaEvent_t pin_ev[4] = {nullptr, nullptr, nullptr, nullptr};
 };
 
+constexpr int kUpSlots = 3;
+constexpr size_t kUpSlot = 2u << 20;  // bytes per slot of an upload's staging
 constexpr int kPinSlots = 4;
 constexpr int64_t kPinSlot = 32ll << 20;  // bytes per staging slot

@@ -61,7 +61,7 @@ int dalloc(dmolp_ctx *c, T **p, size_t n) {
 
 void drop_graphs(dmolp_ctx *c) {
     for (auto &kv : c->graphs) {
-        cudaGraphExecDestroy(kv.second.exec);
+        if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
         for (cudaEvent_t e : kv.second.prof.ev) cudaEventDestroy(e);
     }
     c->graphs.clear();
@@ -192,11 +192,19 @@ std::vector<int> find_hubs(const std::vector<int32_t> &raw) {
     return dmolp::hubs_from_degrees(raw.data(), (int64_t)raw.size());
 }
 
-// Capture (once) and launch the iterations [t0, t0+cnt) of an LP run as one CUDA graph.
+// The iterations [t0, t0+cnt) of an LP run: launched one by one the first time on the resident graph, captured into a
+// CUDA graph the second time and replayed from then on.  The launches keep ahead of a first run (they take 25 us an
+// iteration, the kernels of a graph too large for the one-launch loop more); capturing and instantiating eight
+// iterations took 0.3 ms, which a single run after an upload paid for each of its blocks.
 int run_block_graph(dmolp_ctx *c, const LpLaunch &L, int t0, int cnt) {
     const auto key = std::make_tuple(L.k, L.eff, L.mode, t0, cnt, c->profiling ? 1 : 0);
     auto it = c->graphs.find(key);
     if (it == c->graphs.end()) {
+        c->graphs.emplace(key, dmolp_ctx::GraphEntry());
+        for (int t = t0; t < t0 + cnt; ++t) lp_iteration(c, L, t, t == t0, t == t0 + cnt - 1);
+        return check_launch(c);
+    }
+    if (!it->second.exec) {
         cudaGraph_t g = nullptr;
         dmolp_ctx::GraphEntry ge;
         const long long before = c->launches;
@@ -213,7 +221,7 @@ int run_block_graph(dmolp_ctx *c, const LpLaunch &L, int t0, int cnt) {
         e = cudaGraphInstantiate(&ge.exec, g, 0);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return fail(DMOLP_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-        it = c->graphs.emplace(key, ge).first;
+        it->second = ge;
     }
     DMOLP_CUDA(cudaGraphLaunch(it->second.exec, c->stream));
     c->launches += it->second.kernels;
@@ -487,6 +495,58 @@ int pinned_ring(dmolp_ctx *c) {
     return DMOLP_OK;
 }
 
+// Host array to device on the context's stream.  A large pageable array goes through three pinned slots, filled by all
+// host threads while the previous slot is on the link: the driver's own staging of pageable memory is one thread's
+// memcpy, 12 GB/s.  Smaller arrays, and pinned ones, are left to it.  The source is not read after the return; the
+// slots may still be.
+int upload_array(dmolp_ctx *c, void *dst, const void *src, size_t n) {
+    cudaPointerAttributes at;
+    bool direct = n < 2 * kUpSlot || omp_in_parallel();
+    if (!direct) {
+        if (cudaPointerGetAttributes(&at, src) != cudaSuccess) cudaGetLastError();
+        else direct = at.type != cudaMemoryTypeUnregistered;
+    }
+    for (int s = 0; s < kUpSlots && !direct; ++s) {
+        if (!c->up[s] && cudaHostAlloc((void **)&c->up[s], kUpSlot, cudaHostAllocDefault) != cudaSuccess) direct = true;
+        if (!direct && !c->up_ev[s] && cudaEventCreateWithFlags(&c->up_ev[s], cudaEventDisableTiming) != cudaSuccess)
+            direct = true;
+    }
+    if (direct) {
+        cudaGetLastError();
+        DMOLP_CUDA(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, c->stream));
+        return DMOLP_OK;
+    }
+    // threads copy their share of every slot and meet before it is sent; one of them sends
+    cudaError_t err = cudaSuccess;
+    const int T = std::max(1, std::min(omp_get_max_threads(), 16));
+#pragma omp parallel num_threads(T)
+    {
+        const int me = omp_get_thread_num(), nt = omp_get_num_threads();
+        size_t i = 0;
+        for (size_t pos = 0; pos < n; pos += kUpSlot, ++i) {
+            const int s = (int)(i % kUpSlots);
+            const size_t m = std::min(kUpSlot, n - pos);
+#pragma omp master
+            {
+                const cudaError_t e = cudaEventSynchronize(c->up_ev[s]);  // (an event never recorded is complete)
+                if (err == cudaSuccess) err = e;
+            }
+#pragma omp barrier
+            const size_t per = (m / nt + 63) & ~(size_t)63, a = std::min(m, per * me), z = me + 1 == nt ? m : std::min(m, a + per);
+            std::memcpy(c->up[s] + a, (const char *)src + pos + a, z - a);
+#pragma omp barrier
+#pragma omp master
+            {
+                cudaError_t e = cudaMemcpyAsync((char *)dst + pos, c->up[s], m, cudaMemcpyHostToDevice, c->stream);
+                if (e == cudaSuccess) e = cudaEventRecord(c->up_ev[s], c->stream);
+                if (err == cudaSuccess) err = e;
+            }
+        }
+    }
+    if (err != cudaSuccess) return fail(DMOLP_ERR_CUDA, std::string("graph upload: ") + cudaGetErrorString(err));
+    return DMOLP_OK;
+}
+
 // Parse the text on the device into the resident CSR.  A text the parse rejects leaves the previous graph
 // in place; a CUDA failure after that leaves no graph.
 int ingest_text(dmolp_ctx *c, uint8_t *d_txt, int64_t len, int64_t body0, int64_t body1, dmolp_ingest_info *info) {
@@ -608,6 +668,10 @@ int dmolp_destroy(dmolp_ctx *c) {
         if (c->pin[i]) cudaFreeHost(c->pin[i]);
         if (c->pin_ev[i]) cudaEventDestroy(c->pin_ev[i]);
     }
+    for (int i = 0; i < kUpSlots; ++i) {
+        if (c->up[i]) cudaFreeHost(c->up[i]);
+        if (c->up_ev[i]) cudaEventDestroy(c->up_ev[i]);
+    }
     if (c->h_res) cudaFreeHost(c->h_res);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
@@ -631,10 +695,13 @@ int dmolp_graph_upload(dmolp_ctx *c, int64_t nv, int64_t narcs, const int64_t *o
     int32_t *s_col = narcs ? (int32_t *)c->scratch.get(ingest::kTok, (size_t)narcs * sizeof(int32_t), err) : nullptr;
     int32_t *s_raw = raw && nv ? (int32_t *)c->scratch.get(ingest::kBadrow, (size_t)nv * sizeof(int32_t), err) : nullptr;
     if (!s_off || (narcs && !s_col) || (raw && nv && !s_raw)) return fail(DMOLP_ERR_NOMEM, err);
-    DMOLP_CUDA(cudaMemcpyAsync(s_off, off, (size_t)(nv + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, c->stream));
-    if (s_raw) DMOLP_CUDA(cudaMemcpyAsync(s_raw, raw, (size_t)nv * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
-    if (narcs)
-        DMOLP_CUDA(cudaMemcpyAsync(s_col, col, (size_t)narcs * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
+    int st = upload_array(c, s_off, off, (size_t)(nv + 1) * sizeof(int64_t));
+    if (!st && s_raw) st = upload_array(c, s_raw, raw, (size_t)nv * sizeof(int32_t));
+    if (!st && narcs) st = upload_array(c, s_col, col, (size_t)narcs * sizeof(int32_t));
+    if (st) {
+        cudaStreamSynchronize(c->stream);
+        return st;
+    }
     ingest::CsrInfo ci;
     if (ingest::check_csr(c->stream, s_off, s_col, s_raw, nv, narcs, c->scratch, ci, err)) {
         cudaGetLastError();
@@ -645,7 +712,7 @@ int dmolp_graph_upload(dmolp_ctx *c, int64_t nv, int64_t narcs, const int64_t *o
     if (ci.bad & 2) return fail(DMOLP_ERR_ARG, "a neighbour id is outside [0, nv)");
     if (ci.bad & 4) return fail(DMOLP_ERR_ARG, "negative raw degree");
     const int64_t maxraw = raw ? ci.maxraw : ci.maxdeg;
-    int st = graph_alloc(c, nv, narcs, ci.maxdeg, maxraw, ci.nb);
+    st = graph_alloc(c, nv, narcs, ci.maxdeg, maxraw, ci.nb);
     if (st) return st;
     Buffers &b = c->b;
     DMOLP_CUDA(cudaMemcpyAsync(b.off, s_off, (size_t)(nv + 1) * sizeof(int64_t), cudaMemcpyDeviceToDevice, c->stream));

@@ -197,8 +197,9 @@ class Partitioner:
         return Phase1Metrics(
             initial_edge_cut=info.initial_edge_cut, initial_vertex_balance=info.initial_vertex_balance,
             initial_edge_balance=info.initial_edge_balance, total_vertices=self.num_vertices,
-            total_edges=(int(g.raw_deg().astype(np.int64).sum() // 2) if g is not None
-                         else (self.raw_total or 0) // 2),
+            total_edges=((self.raw_total or 0) if g is None
+                         else int(g.offsets[-1] - g.offsets[0]) if g.raw_degree is None  # the rows' lengths
+                         else int(g.raw_degree.astype(np.int64).sum())) // 2,
             partition_vertex_counts=vc.tolist(), partition_edge_counts=ec.tolist(), seeds=seeds.tolist(),
             num_seeds_found=info.num_seeds_found, rounds=info.rounds, num_hubs=info.num_hubs,
             traversed_edges=info.traversed_edges, gpu_ms=info.gpu_ms,
