@@ -34,11 +34,16 @@ namespace {
 
 using batch::ClusterTeam;
 using batch::CtaTeam;
+using batch::GridTeam;
 using batch::Inst;
 
 constexpr int kAncThreads = 512;
 constexpr int kAncRow = 32;     // rows of at most this many arcs are searched by two lanes
 constexpr int kHugeRow = 4096;  // longer rows are searched by the whole team
+// A graph whose share of the batch is more than this many CTAs gets that share as a team of a cooperative launch: from
+// twice a cluster's 16 on, more CTAs beat the cheaper barrier (features of a skewed graph alone, 1 M vertices: 6.5 -> 4.6 ms).
+constexpr int kGridShare = 32;
+constexpr int kGridTeams = 4;  // at most 148 / 32
 constexpr int kWalkU = 16;      // walk: arcs in flight per vertex
 using batch::kLongRow;          // walk: longer rows are summed by a block of their own
 
@@ -52,12 +57,37 @@ __device__ __forceinline__ SearchRow load_row(const SearchRow *p) {
     return r;
 }
 
-struct AncSmem {
-    unsigned long long wbest[kAncThreads / 32], cbest;
+// What the team shares: in the first CTA's shared memory, or (GridTeam) in global memory.
+struct AncShared {
     int cnt[3];   // frontier counts, rotating: level L reads cnt[L % 3], fills the next, clears the one after
     int nhuge[2];
+    unsigned int word;                  // GridTeam: its barrier,
+    unsigned long long best[kAnchors];  // and the maxima of the anchors' keys; zero before the launch
+};
+
+struct AncSmem {
+    unsigned long long wbest[kAncThreads / 32], cbest;
+    AncShared sh;
     int inst;
 };
+
+// The team's maximum of a key, for anchor j.
+template <typename Tm>
+__device__ __forceinline__ bool anchor_max(unsigned long long &key, int, const Tm &tm, AncSmem &sm, AncShared &) {
+    key = batch::team_max<kAncThreads>(key, tm, sm.wbest, &sm.cbest);
+    return true;
+}
+__device__ __forceinline__ bool anchor_max(unsigned long long &key, int j, const GridTeam<kAncThreads> &tm, AncSmem &,
+                                           AncShared &sh) {
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long y = __shfl_xor_sync(DMOLP_FULL_MASK, key, o);
+        key = y > key ? y : key;
+    }
+    if ((threadIdx.x & 31) == 0 && key) atomicMax(&sh.best[j], key);
+    if (!tm.sync()) return false;
+    key = __ldcg(&sh.best[j]);
+    return true;
+}
 
 // Arcs [s, e) searched by a warp: neighbours farther than d get d and join list.
 __device__ __forceinline__ void search_arcs(const FeatWork &w, int64_t s, int64_t e, int d, int *ctr, SearchRow *list) {
@@ -98,8 +128,8 @@ __device__ __forceinline__ void search_arcs(const FeatWork &w, int64_t s, int64_
 // distance L + 1.  Two lanes per row of at most kAncRow arcs, eight arcs each in flight, so that a mesh's row
 // is one chain of row -> ids -> neighbours' rows -> atomic -> append.  The team's barrier at its end.
 template <typename Tm>
-__device__ __forceinline__ void search_level(const FeatWork &w, SearchRow *const front[2], SearchRow *huge, int nf,
-                                             int L, const Tm &tm, AncSmem &sm) {
+__device__ __forceinline__ bool search_level(const FeatWork &w, SearchRow *const front[2], SearchRow *huge, int nf,
+                                             int L, const Tm &tm, AncShared &sm) {
     const int lane = threadIdx.x & 31;
     const SearchRow *const fin = front[L & 1];
     SearchRow *const fout = front[(L + 1) & 1];
@@ -157,7 +187,7 @@ __device__ __forceinline__ void search_level(const FeatWork &w, SearchRow *const
             }
         }
     }
-    tm.sync();
+    if (!tm.sync()) return false;
     const int nh = *nhuge;
     if (nh > 0) {  // uniform over the team
         for (int i = 0; i < nh; ++i) {
@@ -166,12 +196,13 @@ __device__ __forceinline__ void search_level(const FeatWork &w, SearchRow *const
             for (int64_t c = s + (int64_t)tm.warp() * 512; c < e; c += (int64_t)tm.threads() * 16)
                 search_arcs(w, c, c + 512 < e ? c + 512 : e, d, nout, fout);
         }
-        tm.sync();
+        if (!tm.sync()) return false;
     }
+    return true;
 }
 
 template <typename Tm>
-__device__ void run_anchors(const FeatWork &w, int ii, const Tm &tm, AncSmem &sm) {
+__device__ void run_anchors(const FeatWork &w, int ii, const Tm &tm, AncSmem &sm, AncShared &sh) {
     const Inst I = w.inst[ii];
     const int vb = (int)I.vbase, nv = I.nv;
     SearchRow *const front[2] = {w.front0 + vb, w.front1 + vb};
@@ -189,7 +220,7 @@ __device__ void run_anchors(const FeatWork &w, int ii, const Tm &tm, AncSmem &sm
         r.dist = INT_MAX;  // not reached
         w.row[vb + i] = r;
     }
-    tm.sync();
+    if (!tm.sync()) return;
     for (int j = 0; j < kAnchors; ++j) {
         // the next anchor: maximum degree, then maximum distance to the anchors so far; lowest id on ties
         unsigned long long key = 0;
@@ -199,7 +230,7 @@ __device__ void run_anchors(const FeatWork &w, int ii, const Tm &tm, AncSmem &sm
             const unsigned long long c = ((unsigned long long)(unsigned)x << 32) | (0xFFFFFFFFu - (unsigned)i);
             key = c > key ? c : key;
         }
-        key = batch::team_max<kAncThreads>(key, tm, sm.wbest, &sm.cbest);
+        if (!anchor_max(key, j, tm, sm, sh)) return;
         const int a = vb + (int)(0xFFFFFFFFu - (unsigned)(key & 0xFFFFFFFFull));
         if (lead) {
             w.anchor[j * w.ninst + ii] = a;
@@ -207,18 +238,18 @@ __device__ void run_anchors(const FeatWork &w, int ii, const Tm &tm, AncSmem &sm
             r.dist = 0;
             w.row[a] = r;
             front[0][0] = r;
-            sm.cnt[1] = sm.cnt[2] = 0;
-            sm.nhuge[0] = sm.nhuge[1] = 0;
+            sh.cnt[1] = sh.cnt[2] = 0;
+            sh.nhuge[0] = sh.nhuge[1] = 0;
         }
-        tm.sync();
+        if (!tm.sync()) return;
         int nf = 1, L = 0;
         while (nf > 0) {
-            search_level(w, front, huge, nf, L, tm, sm);
-            nf = *tm.first(&sm.cnt[(L + 1) % 3]);
+            if (!search_level(w, front, huge, nf, L, tm, sh)) return;
+            nf = *tm.first(&sh.cnt[(L + 1) % 3]);
             ++L;
         }
         if (j == 0 && lead) w.ecc[ii] = L - 1;  // the first anchor's eccentricity
-        tm.sync();  // no count is cleared for the next search while it is read
+        if (!tm.sync()) return;  // no count is cleared for the next search while it is read
     }
 }
 
@@ -231,15 +262,32 @@ __global__ void __launch_bounds__(kAncThreads) k_anchors(FeatWork w, const int32
         const int q = sm.inst;
         __syncthreads();
         if (q >= n) break;
-        run_anchors(w, order[q], tm, sm);
+        run_anchors(w, order[q], tm, sm, sm.sh);
     }
 }
 
 __global__ void __launch_bounds__(kAncThreads) k_anchors_team(FeatWork w, const int32_t *order) {
     __shared__ AncSmem sm;
     const ClusterTeam<kAncThreads> tm;
-    run_anchors(w, order[blockIdx.x / tm.size()], tm, sm);
+    run_anchors(w, order[blockIdx.x / tm.size()], tm, sm, sm.sh);
     tm.sync();  // no CTA leaves while its counters are read
+}
+
+// Teams of CTAs [start[i], start[i + 1]) of one cooperative launch, team i on graph order[i].
+struct GridTeams {
+    int n, start[kGridTeams + 1];
+    AncShared *sh;
+    int *err;
+    unsigned int polls;
+};
+
+__global__ void __launch_bounds__(kAncThreads) k_anchors_grid(FeatWork w, const int32_t *order, GridTeams t) {
+    __shared__ AncSmem sm;
+    int i = 0;
+    while (i + 1 < t.n && (int)blockIdx.x >= t.start[i + 1]) ++i;
+    const GridTeam<kAncThreads> tm = {&t.sh[i].word, t.err, t.polls, t.start[i + 1] - t.start[i],
+                                      (int)blockIdx.x - t.start[i]};
+    run_anchors(w, order[i], tm, sm, t.sh[i]);
 }
 
 // ------------------------------------------------------------------------------------ per-vertex passes
@@ -467,20 +515,69 @@ int features(const FeatWork &w, const batch::View &b, cudaStream_t s) {
     cudaMemsetAsync(w.stats, 0, sizeof(double) * 16 * w.ninst, s);
     k_vinst<<<g, 256, 0, s>>>(w);
     {
-        const std::vector<int32_t> &order = *b.h_order;
-        const int slots = b.num_sms;
-        const batch::TeamPlan plan = batch::team_sizes(*b.h_inst, order, slots, kAncThreads, anchors_max_team());
+        std::vector<int32_t> order = *b.h_order;
+        int slots = b.num_sms;
         const int32_t *o = b.order;
-        b.fork->open(plan, s);
+        // graphs worth more than a cluster, largest first
+        double total = 0;
+        for (int32_t i : order) total += (double)((*b.h_inst)[i].narcs + (*b.h_inst)[i].nv);
+        GridTeams gt = {};
+        for (int32_t i : order) {
+            const Inst &I = (*b.h_inst)[i];
+            const int c = (int)((double)(I.narcs + I.nv) * b.num_sms / total);
+            if (gt.n == kGridTeams || c <= kGridShare || I.nv <= c * kAncThreads) break;
+            gt.start[gt.n + 1] = gt.start[gt.n] + std::min(c, slots);
+            slots -= std::min(c, slots);
+            ++gt.n;
+        }
+        if (gt.n > 0) {
+            static_assert(sizeof(AncShared) * kGridTeams <= kFeatSharedBytes, "the teams' counters fit their buffer");
+            gt.sh = reinterpret_cast<AncShared *>(w.shared);
+            gt.err = w.err;
+            gt.polls = w.polls;
+            cudaMemsetAsync(w.shared, 0, kFeatSharedBytes, s);
+            cudaEventRecord(b.fork->begin, s);  // the other graphs run next to them
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)gt.start[gt.n]);
+            cfg.blockDim = dim3(kAncThreads);
+            cfg.stream = s;
+            cudaLaunchAttribute at;
+            at.id = cudaLaunchAttributeCooperative;
+            at.val.cooperative = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            const cudaError_t le = cudaLaunchKernelEx(&cfg, k_anchors_grid, w, o, gt);
+            if (le != cudaSuccess) return (int)le;
+            order.erase(order.begin(), order.begin() + gt.n);
+            o += gt.n;
+            slots = std::max(slots, 1);
+        }
+        // (next to such teams every class runs on its own side stream, which the clusters of 16 have not)
+        const int most = anchors_max_team();
+        const batch::TeamPlan plan =
+            batch::team_sizes(*b.h_inst, order, slots, kAncThreads, gt.n > 0 ? std::min(most, batch::kMaxTeam / 2) : most);
+        const int j1 = batch::kTeamClasses - 1, n1 = plan.n[j1];
+        if (gt.n > 0) {
+            for (int j = 1; j <= j1; ++j)
+                if (plan.n[j] > 0) cudaStreamWaitEvent(b.fork->side[j - 1], b.fork->begin, 0);
+        } else {
+            b.fork->open(plan, s);
+        }
+        auto on = [&](int j) { return gt.n > 0 ? b.fork->side[j - 1] : b.fork->stream(plan, j, s); };
         for (int j = 0, c = batch::kMaxTeam; c > 1; ++j, c >>= 1) {
-            if (plan.n[j] > 0)
-                batch::launch_cluster(k_anchors_team, plan.n[j], c, kAncThreads, b.fork->stream(plan, j, s), w, o);
+            if (plan.n[j] > 0) batch::launch_cluster(k_anchors_team, plan.n[j], c, kAncThreads, on(j), w, o);
             o += plan.n[j];
         }
-        const int j1 = batch::kTeamClasses - 1, n1 = plan.n[j1];
-        if (n1 > 0)
-            k_anchors<<<std::min(slots, n1), kAncThreads, 0, b.fork->stream(plan, j1, s)>>>(w, o, n1, w.next);
-        b.fork->close(plan, s);
+        if (n1 > 0) k_anchors<<<std::min(b.num_sms, n1), kAncThreads, 0, on(j1)>>>(w, o, n1, w.next);
+        if (gt.n > 0) {
+            for (int j = 1; j <= j1; ++j)
+                if (plan.n[j] > 0) {
+                    cudaEventRecord(b.fork->end[j - 1], b.fork->side[j - 1]);
+                    cudaStreamWaitEvent(s, b.fork->end[j - 1], 0);
+                }
+        } else {
+            b.fork->close(plan, s);
+        }
     }
     std::vector<int32_t> ecc(w.ninst);
     cudaMemcpyAsync(ecc.data(), w.ecc, sizeof(int32_t) * w.ninst, cudaMemcpyDeviceToHost, s);

@@ -69,6 +69,8 @@ struct __align__(16) SearchRow {
     int len, dist;
 };
 
+constexpr size_t kFeatSharedBytes = 1024;
+
 struct FeatWork {
     const int64_t *off;
     const int32_t *col;
@@ -83,6 +85,9 @@ struct FeatWork {
     Chunk *chunks;                            // [nv / kChunkV + ninst + the batch's long rows]
     float *P0, *Q0, *P1, *Q1;                 // [nv * 8]
     double *stats;                            // [ninst * 16]
+    void *shared;                             // [kFeatSharedBytes] counters of the searches' largest teams
+    int *err;                                 // set by a wait that gave up after `polls` polls
+    uint32_t polls;
     float *Xf;                                // [nv * 16] features before rounding
     __nv_bfloat16 *X;                         // [nv * ldx] bf16 input of layer 1
     int ldx;

@@ -51,8 +51,9 @@ struct dmolp_mpnn {
     float *params = nullptr, *grads = nullptr, *m = nullptr, *v = nullptr;
     __nv_bfloat16 *W[3] = {}, *Wt[3] = {};
     int *err = nullptr;
-    uint32_t wait_polls = 1u << 24;  // GEMM completion-barrier polls before it gives up (dmolp_mpnn_set_wait_limit)
+    uint32_t wait_polls = 1u << 24;  // polls of a GEMM completion or team barrier before it gives up
     double *loss = nullptr;
+    char *shared = nullptr;  // [kFeatSharedBytes]
     int step = 0;
     std::vector<void *> fixed;
     // per-batch workspace
@@ -159,7 +160,7 @@ int sync_check(dmolp_mpnn *m, cudaStream_t s, const char *what) {
     MCUDA(cudaMemcpy(&e, m->err, sizeof(int), cudaMemcpyDeviceToHost));
     if (e) {
         cudaMemset(m->err, 0, sizeof(int));
-        return fail(DMOLP_ERR_CUDA, std::string(what) + ": a tensor-core wait timed out");
+        return fail(DMOLP_ERR_CUDA, std::string(what) + ": a bounded wait (tensor-core completion or team barrier) timed out");
     }
     return DMOLP_OK;
 }
@@ -273,6 +274,7 @@ int dmolp_mpnn_create(int device, dmolp_mpnn **out) {
     }
     if (!r) r = alloc_into(o, &m->err, 1);
     if (!r) r = alloc_into(o, &m->loss, 1);
+    if (!r) r = alloc_into(o, &m->shared, kFeatSharedBytes);
     if (r) {
         dmolp_mpnn_destroy(m);
         return r;
@@ -357,6 +359,9 @@ int dmolp_mpnn_features(dmolp_mpnn *m, dmolp_batch *b, float *features) {
     w.P1 = m->P1;
     w.Q1 = m->Q1;
     w.stats = m->stats;
+    w.shared = m->shared;
+    w.err = m->err;
+    w.polls = m->wait_polls;
     w.Xf = m->Xf;
     w.X = m->C1;
     w.ldx = 2 * kIn;

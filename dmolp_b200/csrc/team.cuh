@@ -18,7 +18,10 @@ struct CtaTeam {
     __device__ __forceinline__ int thread() const { return threadIdx.x; }
     __device__ __forceinline__ constexpr int threads() const { return NT; }
     __device__ __forceinline__ int warp() const { return threadIdx.x >> 5; }
-    __device__ __forceinline__ void sync() const { __syncthreads(); }
+    __device__ __forceinline__ bool sync() const {
+        __syncthreads();
+        return true;
+    }
     template <typename T>
     __device__ __forceinline__ T *at(T *p, int) const {
         return p;
@@ -44,7 +47,10 @@ struct ClusterTeam {
     __device__ __forceinline__ int warp() const { return (int)(threadIdx.x >> 5) * n + rank; }
     __device__ __forceinline__ int threads() const { return NT * n; }
     __device__ __forceinline__ int thread() const { return warp() * 32 + (int)(threadIdx.x & 31); }
-    __device__ __forceinline__ void sync() const { cooperative_groups::this_cluster().sync(); }
+    __device__ __forceinline__ bool sync() const {
+        cooperative_groups::this_cluster().sync();
+        return true;
+    }
     template <typename T>
     __device__ __forceinline__ T *at(T *p, int r) const {
         return cooperative_groups::this_cluster().map_shared_rank(p, r);
@@ -52,6 +58,49 @@ struct ClusterTeam {
     template <typename T>
     __device__ __forceinline__ T *first(T *p) const {
         return at(p, 0);
+    }
+};
+
+// Some of the CTAs of a cooperative launch (all resident), for graphs that are worth more CTAs than a cluster has.
+// They share no shared memory: the team's counters are one object in global memory, which first(p) leaves as it is,
+// and code for this team keeps nothing else per CTA in it.  sync() is a barrier on one word: the first CTA adds
+// 2^31 - (n - 1), every other CTA 1, so the arrivals flip the top bit and leave the rest; the fences of thread 0,
+// between barriers of the block, order the whole block's accesses.  It returns false when the wait gave up after
+// `polls` polls, or another CTA's did (*err is then set): the caller leaves the kernel at once.
+template <int NT>
+struct GridTeam {
+    unsigned int *word;
+    int *err;
+    unsigned int polls;
+    int n, rank;
+    __device__ __forceinline__ int size() const { return n; }
+    __device__ __forceinline__ bool is_first() const { return rank == 0; }
+    __device__ __forceinline__ int rank_of() const { return rank; }
+    __device__ __forceinline__ int warp() const { return (int)(threadIdx.x >> 5) * n + rank; }
+    __device__ __forceinline__ int threads() const { return NT * n; }
+    __device__ __forceinline__ int thread() const { return warp() * 32 + (int)(threadIdx.x & 31); }
+    __device__ __forceinline__ bool sync() const {
+        bool pass = true;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            const unsigned int old = atomicAdd(word, rank == 0 ? 0x80000000u - ((unsigned int)n - 1u) : 1u);
+            volatile unsigned int *w = word;
+            volatile int *gave_up = err;
+            for (unsigned int i = 0; ((*w ^ old) & 0x80000000u) == 0u; ++i) {
+                if (i >= polls || ((i & 63u) == 63u && *gave_up)) {
+                    atomicExch(err, 1);
+                    pass = false;
+                    break;
+                }
+            }
+            __threadfence();
+        }
+        return __syncthreads_and(pass);
+    }
+    template <typename T>
+    __device__ __forceinline__ T *first(T *p) const {
+        return p;
     }
 };
 
