@@ -46,8 +46,9 @@ struct GemmArgs {
     uint32_t polls;  // polls of the MMA completion barrier before the GEMM gives up (then: err, TMEM freed)
 };
 
-// One launch of the tensor-core GEMM: N = output tile width, KT = K tile.
-void gemm(const GemmArgs &g, int n, int kt, int num_sms, cudaStream_t s);
+// One launch of the tensor-core GEMM, N = n: row kinds with (n, K) = (64, 32), (64, 128), (16, 128), (128, 16) or
+// (128, 64), the weight gradient with n = 64 or 16.
+void gemm(const GemmArgs &g, int n, int num_sms, cudaStream_t s);
 
 void agg_fwd(const batch::View &b, __nv_bfloat16 *buf, int C);
 void agg_bwd(const batch::View &b, const float *dC, const __nv_bfloat16 *Hbuf, int ldh, __nv_bfloat16 *G, float *db);

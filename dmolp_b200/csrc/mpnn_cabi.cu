@@ -198,7 +198,7 @@ void run_forward(dmolp_mpnn *m, const batch::View &b) {
             g.out_f32 = m->Z3;
             g.ldo32 = kOut;
         }
-        gemm(g, kN[l], l == 0 ? 32 : 64, b.num_sms, s);
+        gemm(g, kN[l], b.num_sms, s);
         if (l < 2) agg_fwd(b, out[l], kHidden);
     }
     m->have_z = true;
@@ -224,7 +224,7 @@ void run_backward(dmolp_mpnn *m, const batch::View &b) {
         w.ldb = ldg;
         w.nb = kN[l];
         w.out_w = m->grads + kOffW[l];
-        gemm(w, kN[l], 64, b.num_sms, s);
+        gemm(w, kN[l], b.num_sms, s);
         if (l == 0) break;
         GemmArgs d = base_args(m, nv);
         d.kind = kBwdData;
@@ -237,7 +237,7 @@ void run_backward(dmolp_mpnn *m, const batch::View &b) {
         d.out_f32 = m->dC;
         d.ldo32 = 2 * kHidden;
         d.off = b.off;
-        gemm(d, 2 * kHidden, kN[l] == 16 ? 16 : 64, b.num_sms, s);
+        gemm(d, 2 * kHidden, b.num_sms, s);
         agg_bwd(b, m->dC, C[l], kK[l], m->G, m->grads + kOffB[l - 1]);
         Gin = m->G;
         ldg = kHidden;

@@ -8,11 +8,11 @@
 //
 // The concatenation [H | mean H] is one BF16 buffer per layer: the GEMM epilogue of layer l writes H_{l+1}
 // into the left half of layer l+1's buffer and the aggregation kernel fills its right half.  The GEMMs
-// stage 128-row tiles of A and the B tile into shared memory in the no-swizzle K-major core-matrix layout
+// copy 128-row tiles of A and the whole of B into shared memory in the no-swizzle K-major core-matrix layout
 // (umma.cuh), one thread issues tcgen05.mma into a tensor-memory accumulator, completion is signalled on an
 // mbarrier (bounded wait: a stuck MMA sets an error flag instead of hanging), and the epilogue reads the
-// accumulator with tcgen05.ld.  The weight gradient is the same GEMM with vertices as the reduction axis,
-// staged transposed, each CTA adding its partial sums to dW with atomics.
+// accumulator with tcgen05.ld.  The weight gradient has the vertices as its reduction axis: both operands are
+// MN-major, and each CTA adds its partial sums to dW with atomics.
 #include <algorithm>
 #include <cfloat>
 #include <vector>
@@ -37,138 +37,249 @@ __device__ __forceinline__ float inv_degree(int64_t deg) {
 }
 
 // ------------------------------------------------------------------------------------------------ GEMM
-template <int N, int KT>
-__global__ void __launch_bounds__(128) k_gemm(GemmArgs g) {
-    extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ __align__(8) uint64_t mbar;
-    __shared__ uint32_t tslot;
-    constexpr uint32_t NCOL = N < 32 ? 32 : N;
-    constexpr int CH = KT / 8;  // 16-byte chunks per tile row
-    uint8_t *sA = smem, *sB = smem + 128 * KT * 2;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (warp == 0) umma::tmem_alloc(&tslot, NCOL);
-    if (tid == 0) {
-        umma::mbar_init(&mbar, 1);
+// What bounds these: bytes.  K is at most 128, so a row's 32 to 256 bytes are read once for at most 16 KFLOP.  The
+// row kernels therefore keep the whole weight tile in shared memory, and copy a CTA's next row tile (asynchronously,
+// 16 bytes per thread) while the tensor core and the epilogue work on the current one; the weight gradient copies
+// its next 64 vertices behind the current MMAs, in the MN-major layout, which takes rows as they are.  Eight
+// consecutive threads fill one core matrix: no bank conflicts, and whole sectors of four rows' neighbouring chunks.
+// Before, tiles of K = 64 were staged through registers (transposed element by element for the weight gradient) with
+// nothing else in flight.  A training step of 64 graphs (0.72 M vertices): its eight GEMMs 1.42 -> 0.63 ms.
+constexpr int kGemmThreads = 128;
+
+// Accumulator columns c0 .. c0 + 15 of a warp's 32 rows from row0 on to the outputs, lane r holding row r (inv: its
+// 1 / degree for the data gradient).  They go through the warp's shared stage, so that neighbouring lanes write
+// neighbouring words: a store of 16 bytes per row took a transaction per lane (128 columns out of K = 16: 167 us for
+// 0.72 M rows, now 101).
+constexpr int kStagePitch = 20;  // floats per row: 16-byte aligned, conflict-free by rows
+constexpr size_t kStageBytes = (size_t)kGemmThreads * kStagePitch * sizeof(float);
+
+__device__ __forceinline__ void store_rows(const GemmArgs &g, float *stage, int row0, int c0, float inv, float (&v)[16]) {
+    const int lane = threadIdx.x & 31;
+    if (g.off && c0 >= kHidden) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = __fmul_rn(v[i], inv);
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        if (g.bias) v[i] = __fadd_rn(v[i], g.bias[c0 + i]);
+        if (g.relu) v[i] = fmaxf(v[i], 0.0f);
+    }
+    float4 *mine = reinterpret_cast<float4 *>(stage + lane * kStagePitch);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) mine[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    __syncwarp();
+    if (g.out_bf16) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {  // two lanes per row
+            const int r = i * 16 + (lane >> 1), row = row0 + r;
+            const float4 *src = reinterpret_cast<const float4 *>(stage + r * kStagePitch) + (lane & 1) * 2;
+            const float4 x = src[0], y = src[1];
+            const float f[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+            __align__(16) __nv_bfloat16 h[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) h[j] = __float2bfloat16_rn(f[j]);
+            if (row < g.rows)
+                *reinterpret_cast<uint4 *>(g.out_bf16 + (size_t)row * g.ldo + c0 + (lane & 1) * 8) =
+                    *reinterpret_cast<const uint4 *>(h);
+        }
+    }
+    if (g.out_f32) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {  // four lanes per row
+            const int r = i * 8 + (lane >> 2), row = row0 + r;
+            const float4 x = *(reinterpret_cast<const float4 *>(stage + r * kStagePitch) + (lane & 3));
+            if (row < g.rows) *reinterpret_cast<float4 *>(g.out_f32 + (size_t)row * g.ldo32 + c0 + (lane & 3) * 4) = x;
+        }
+    }
+    __syncwarp();  // the stage may be written again
+}
+
+// Tensor memory and the completion barrier of a CTA; returns the accumulator's address.
+__device__ __forceinline__ uint32_t gemm_begin(uint64_t *mbar, uint32_t *tslot, uint32_t ncol) {
+    if (threadIdx.x < 32) umma::tmem_alloc(tslot, ncol);
+    if (threadIdx.x == 0) {
+        umma::mbar_init(mbar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
-    const uint32_t tmem = tslot;
+    return *tslot;
+}
+
+// Nothing is in flight when the CTA ends: copies, MMAs (a wait that gave up is waited for once more), tensor memory.
+__device__ __forceinline__ void gemm_end(const GemmArgs &g, bool ok, uint64_t *mbar, uint32_t phase, uint32_t tmem,
+                                         uint32_t ncol) {
+    umma::copy_wait<0>();
+    if (!ok) {
+        umma::mbar_wait(mbar, phase, kWaitLimit);  // let an MMA still in flight finish before the free
+        if (threadIdx.x == 0) atomicExch(g.err, 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) umma::tmem_free(tmem, ncol);
+}
+
+// Rows of A [rows x K] times B^T [N x K]: 128 rows per item.
+template <int N, int K>
+struct RowGemm {
+    static constexpr size_t kTileA = 128 * K * 2, kTileB = (size_t)N * K * 2, kSmem = 2 * kTileA + kTileB + kStageBytes;
+    static constexpr uint32_t kCols = N < 32 ? 32 : N;
+    // resident CTAs per SM: shared memory, tensor memory (512 columns), and no more than eight
+    static constexpr int kFit = (int)(220 * 1024 / (kSmem + 1024)), kTm = 512 / (int)kCols;
+    static constexpr int kPerSm = kFit < kTm ? (kFit < 8 ? kFit : 8) : (kTm < 8 ? kTm : 8);
+};
+
+template <int N, int K>
+__global__ void __launch_bounds__(kGemmThreads) k_gemm_rows(GemmArgs g) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ uint32_t tslot;
+    constexpr int CH = K / 8;  // 16-byte chunks per row
+    constexpr uint32_t TA = RowGemm<N, K>::kTileA, NCOL = RowGemm<N, K>::kCols;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t tmem = gemm_begin(&mbar, &tslot, NCOL);
     constexpr uint32_t idesc = umma::idesc_bf16_f32(128, N);
+    const uint32_t sA = umma::smem_addr(smem), sB = sA + 2 * TA;
+    float *const stage =
+        reinterpret_cast<float *>(smem + 2 * TA + RowGemm<N, K>::kTileB) + warp * 32 * kStagePitch;
+    const int nitems = (g.rows + 127) / 128;
+    // chunk q of a tile is row 8 (q / 8 / CH) + q % 8, chunk (q / 8) % CH, and lies at byte 16 q
+    for (int q = tid; q < N * CH; q += kGemmThreads) {
+        const int n = q / (8 * CH) * 8 + (q & 7), c = (q >> 3) % CH;
+        umma::copy16(sB + 16 * q, g.B + (size_t)(n < g.nb ? n : 0) * g.ldb + c * 8, n < g.nb);
+    }
+    auto load = [&](int item, uint32_t dst) {
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            const int q = i * kGemmThreads + tid;
+            const int row = item * 128 + q / (8 * CH) * 8 + (q & 7), c = (q >> 3) % CH;
+            umma::copy16(dst + 16 * q, g.A + (size_t)min(row, g.rows - 1) * g.lda + c * 8, row < g.rows);
+        }
+    };
+    if ((int)blockIdx.x < nitems) load(blockIdx.x, sA);
+    umma::copy_commit();
+    uint32_t phase = 0, buf = 0;
+    bool ok = true;
+    for (int item = blockIdx.x; item < nitems; item += gridDim.x, buf ^= 1) {
+        // the next tile, into the buffer whose MMAs ended before the last epilogue
+        if (item + (int)gridDim.x < nitems) load(item + gridDim.x, sA + (buf ^ 1) * TA);
+        umma::copy_commit();
+        umma::copy_wait<1>();
+        umma::fence_async_smem();
+        umma::fence_before_sync();
+        __syncthreads();
+        if (tid == 0) {
+            umma::fence_after_sync();
+            const uint32_t a0 = sA + buf * TA;
+#pragma unroll
+            for (int s = 0; s < K / 16; ++s)
+                umma::mma_bf16(tmem, umma::smem_desc(a0 + 256 * s, 128, K * 16),
+                               umma::smem_desc(sB + 256 * s, 128, K * 16), idesc, s > 0);
+            umma::mma_commit(&mbar);
+        }
+        ok = __syncthreads_and(umma::mbar_wait(&mbar, phase, g.polls));
+        if (!ok) break;
+        phase ^= 1;
+        umma::fence_after_sync();
+        // ---- epilogue: warp w owns accumulator rows (TMEM lanes) 32w .. 32w+31 ----
+        const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
+        const int row0 = item * 128 + warp * 32;
+        float inv = 0.f;
+        if (g.off && row0 + lane < g.rows) inv = inv_degree(g.off[row0 + lane + 1] - g.off[row0 + lane]);
+#pragma unroll
+        for (int c0 = 0; c0 < N; c0 += 16) {
+            float v[16];
+            umma::tmem_ld16(trow + c0, v);
+            store_rows(g, stage, row0, c0, inv, v);
+        }
+        umma::fence_before_sync();
+        __syncthreads();  // the accumulator is read before the next tile's first MMA overwrites it
+    }
+    gemm_end(g, ok, &mbar, phase, tmem, NCOL);
+}
+
+// dW [m_valid x N] += A^T [m x vertices] times G [vertices x N]: an item is `chunk` vertices, 64 per step.
+constexpr int kWgtK = 64, kWgtM = 128;
+template <int N>
+constexpr size_t wgt_smem() {
+    return 2 * (size_t)(kWgtM + N) * kWgtK * 2;
+}
+
+template <int N>
+__global__ void __launch_bounds__(kGemmThreads) k_gemm_wgt(GemmArgs g) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ uint32_t tslot;
+    constexpr uint32_t TA = kWgtM * kWgtK * 2, TB = N * kWgtK * 2, NCOL = N < 32 ? 32 : N;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t tmem = gemm_begin(&mbar, &tslot, NCOL);
+    constexpr uint32_t idesc = umma::idesc_bf16_f32(kWgtM, N) | umma::kMajorMN;
+    const uint32_t sA = umma::smem_addr(smem), sB = sA + 2 * TA;
+    const int nitems = (g.rows + g.chunk - 1) / g.chunk, MB = g.m_valid / 8;
+    for (uint32_t i = tid; i < 2 * TA / 16; i += kGemmThreads)  // columns from m_valid on stay zero
+        reinterpret_cast<uint4 *>(smem)[i] = zero4();
+    __syncthreads();
     uint32_t phase = 0;
-    int ok = 1;
-    const bool wgt = g.kind == kBwdWeight;
-    const int nitems = wgt ? (g.rows + g.chunk - 1) / g.chunk : (g.rows + 127) / 128;
-    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
-        const int r0 = wgt ? item * g.chunk : item * 128;
-        const int ktot = wgt ? min(g.chunk, g.rows - r0) : g.K;
-        for (int kc = 0; kc < ktot; kc += KT) {
-            // ---- stage the A (128 x KT) and B (N x KT) tiles ----
-            if (!wgt) {
-                for (int q = tid; q < 128 * CH; q += 128) {
-                    const int r = q / CH, c = q % CH, row = r0 + r, kk = kc + c * 8;
-                    uint4 x = zero4();
-                    if (row < g.rows && kk < g.K) x = *reinterpret_cast<const uint4 *>(g.A + (size_t)row * g.lda + kk);
-                    *reinterpret_cast<uint4 *>(sA + umma::tile_offset(r, c * 8, KT)) = x;
-                }
-                for (int q = tid; q < N * CH; q += 128) {
-                    const int n = q / CH, c = q % CH, kk = kc + c * 8;
-                    uint4 x = zero4();
-                    if (n < g.nb && kk < g.K) x = *reinterpret_cast<const uint4 *>(g.B + (size_t)n * g.ldb + kk);
-                    *reinterpret_cast<uint4 *>(sB + umma::tile_offset(n, c * 8, KT)) = x;
-                }
-            } else {
-                // A(m, k) = C[vertex r0+kc+k][feature m], B(n, k) = G[vertex r0+kc+k][n]: transposed staging
-                for (int q = tid; q < KT * 16; q += 128) {
-                    const int k = q / 16, m = (q % 16) * 8, v = kc + k;
-                    uint4 x = zero4();
-                    if (v < ktot && m < g.m_valid)
-                        x = *reinterpret_cast<const uint4 *>(g.A + (size_t)(r0 + v) * g.lda + m);
-                    const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&x);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        *reinterpret_cast<__nv_bfloat16 *>(sA + umma::tile_offset(m + j, k, KT)) = e[j];
-                }
-                for (int q = tid; q < KT * (N / 8); q += 128) {
-                    const int k = q / (N / 8), n = (q % (N / 8)) * 8, v = kc + k;
-                    uint4 x = zero4();
-                    if (v < ktot) x = *reinterpret_cast<const uint4 *>(g.B + (size_t)(r0 + v) * g.ldb + n);
-                    const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&x);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        *reinterpret_cast<__nv_bfloat16 *>(sB + umma::tile_offset(n + j, k, KT)) = e[j];
-                }
+    bool ok = true;
+    for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+        const int r0 = item * g.chunk, n = min(g.chunk, g.rows - r0), steps = (n + kWgtK - 1) / kWgtK;
+        // vertex 8 kg + k of a step, 16-byte chunk c of its row: byte ((kg * chunks + c) * 8 + k) * 16
+        auto load = [&](int step, uint32_t buf) {
+            const int v0 = step * kWgtK;
+            for (int q = tid; q < kWgtK * MB; q += kGemmThreads) {
+                const int k = q & 7, c = (q >> 3) % MB, kg = (q >> 3) / MB, v = v0 + kg * 8 + k;
+                umma::copy16(sA + buf * TA + ((kg * (kWgtM / 8) + c) * 8 + k) * 16,
+                             g.A + (size_t)(r0 + min(v, n - 1)) * g.lda + c * 8, v < n);
             }
+            for (int q = tid; q < kWgtK * (N / 8); q += kGemmThreads) {
+                const int k = q & 7, c = (q >> 3) % (N / 8), v = v0 + (q >> 3) / (N / 8) * 8 + k;
+                umma::copy16(sB + buf * TB + q * 16, g.B + (size_t)(r0 + min(v, n - 1)) * g.ldb + c * 8, v < n);
+            }
+        };
+        load(0, 0);
+        umma::copy_commit();
+        for (int i = 0; i < steps; ++i) {
+            if (i > 0) {  // the other buffer's MMAs
+                ok = __syncthreads_and(umma::mbar_wait(&mbar, phase, g.polls));
+                if (!ok) break;
+                phase ^= 1;
+            }
+            if (i + 1 < steps) load(i + 1, (i + 1) & 1);
+            umma::copy_commit();
+            umma::copy_wait<1>();
             umma::fence_async_smem();
             umma::fence_before_sync();
             __syncthreads();
             if (tid == 0) {
                 umma::fence_after_sync();
-                const uint32_t a0 = umma::smem_addr(sA), b0 = umma::smem_addr(sB);
+                const uint32_t a0 = sA + (i & 1) * TA, b0 = sB + (i & 1) * TB;
 #pragma unroll
-                for (int s = 0; s < KT / 16; ++s)
-                    umma::mma_bf16(tmem, umma::smem_desc(a0 + 256 * s, 128, KT * 16),
-                                   umma::smem_desc(b0 + 256 * s, 128, KT * 16), idesc, kc > 0 || s > 0);
+                for (int s = 0; s < kWgtK / 16; ++s)
+                    umma::mma_bf16(tmem, umma::smem_desc(a0 + s * 2 * kWgtM * 16, kWgtM * 16, 128),
+                                   umma::smem_desc(b0 + s * 2 * N * 16, N * 16, 128), idesc, i > 0 || s > 0);
                 umma::mma_commit(&mbar);
             }
-            const bool done = umma::mbar_wait(&mbar, phase, g.polls);
-            ok = __syncthreads_and(done);
-            if (!ok) break;
-            phase ^= 1;
-            umma::fence_after_sync();
         }
         if (!ok) break;
-        // ---- epilogue: warp w owns accumulator rows (TMEM lanes) 32w .. 32w+31 ----
+        ok = __syncthreads_and(umma::mbar_wait(&mbar, phase, g.polls));
+        if (!ok) break;
+        phase ^= 1;
+        umma::fence_after_sync();
         const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
         const int r = warp * 32 + lane;
 #pragma unroll
         for (int c0 = 0; c0 < N; c0 += 16) {
             float v[16];
             umma::tmem_ld16(trow + c0, v);
-            if (wgt) {
-                if (r < g.m_valid)
+            if (r < g.m_valid)
 #pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (c0 + i < g.nb && v[i] != 0.0f) atomicAdd(&g.out_w[(size_t)r * g.nb + c0 + i], v[i]);
-            } else {
-                const int row = r0 + r;
-                if (row < g.rows) {
-                    if (g.off && c0 >= kHidden) {
-                        const float inv = inv_degree(g.off[row + 1] - g.off[row]);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i] = __fmul_rn(v[i], inv);
-                    }
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        if (g.bias) v[i] = __fadd_rn(v[i], g.bias[c0 + i]);
-                        if (g.relu) v[i] = fmaxf(v[i], 0.0f);
-                    }
-                    if (g.out_bf16) {
-                        __align__(16) __nv_bfloat16 h[16];
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) h[i] = __float2bfloat16_rn(v[i]);
-                        uint4 *dst = reinterpret_cast<uint4 *>(g.out_bf16 + (size_t)row * g.ldo + c0);
-                        dst[0] = reinterpret_cast<const uint4 *>(h)[0];
-                        dst[1] = reinterpret_cast<const uint4 *>(h)[1];
-                    }
-                    if (g.out_f32) {
-                        float4 *dst = reinterpret_cast<float4 *>(g.out_f32 + (size_t)row * g.ldo32 + c0);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                    }
-                }
-            }
+                for (int i = 0; i < 16; ++i)
+                    if (c0 + i < g.nb && v[i] != 0.0f) atomicAdd(&g.out_w[(size_t)r * g.nb + c0 + i], v[i]);
         }
         umma::fence_before_sync();
-        __syncthreads();  // the accumulator is read before the next tile's first MMA overwrites it
+        __syncthreads();  // the accumulator is read before the next item's first MMA overwrites it
     }
-    if (!ok) {
-        umma::mbar_wait(&mbar, phase, kWaitLimit);  // let an MMA still in flight finish before the free
-        if (tid == 0) atomicExch(g.err, 1);
-    }
-    __syncthreads();
-    if (warp == 0) umma::tmem_free(tmem, NCOL);
+    gemm_end(g, ok, &mbar, phase, tmem, NCOL);
 }
 
 // ------------------------------------------------------------------------------------ aggregation
@@ -505,12 +616,19 @@ __global__ void k_coords(const float *__restrict__ Xf, const float *__restrict__
     }
 }
 
-template <int N, int KT>
-void launch_gemm(const GemmArgs &g, int num_sms, cudaStream_t s) {
-    const size_t smem = (size_t)(128 + N) * KT * 2;
-    const int items = g.kind == kBwdWeight ? (g.rows + g.chunk - 1) / g.chunk : (g.rows + 127) / 128;
-    const int grid = std::max(1, std::min(items, num_sms * 4));
-    k_gemm<N, KT><<<grid, 128, smem, s>>>(g);
+template <int N, int K>
+void launch_rows(const GemmArgs &g, int num_sms, cudaStream_t s) {
+    using R = RowGemm<N, K>;
+    cudaFuncSetAttribute(k_gemm_rows<N, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R::kSmem);
+    const int grid = std::max(1, std::min((g.rows + 127) / 128, num_sms * R::kPerSm));
+    k_gemm_rows<N, K><<<grid, kGemmThreads, R::kSmem, s>>>(g);
+}
+
+template <int N>
+void launch_wgt(const GemmArgs &g, int num_sms, cudaStream_t s) {
+    cudaFuncSetAttribute(k_gemm_wgt<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wgt_smem<N>());
+    const int grid = std::max(1, std::min((g.rows + g.chunk - 1) / g.chunk, num_sms * 4));
+    k_gemm_wgt<N><<<grid, kGemmThreads, wgt_smem<N>(), s>>>(g);
 }
 
 inline int grid_for(int64_t n, int num_sms) {
@@ -520,12 +638,20 @@ inline int grid_for(int64_t n, int num_sms) {
 
 }  // namespace
 
-void gemm(const GemmArgs &g, int n, int kt, int num_sms, cudaStream_t s) {
-    if (n == 64 && kt == 32) launch_gemm<64, 32>(g, num_sms, s);
-    else if (n == 64 && kt == 64) launch_gemm<64, 64>(g, num_sms, s);
-    else if (n == 16 && kt == 64) launch_gemm<16, 64>(g, num_sms, s);
-    else if (n == 128 && kt == 16) launch_gemm<128, 16>(g, num_sms, s);
-    else if (n == 128 && kt == 64) launch_gemm<128, 64>(g, num_sms, s);
+void gemm(const GemmArgs &g, int n, int num_sms, cudaStream_t s) {
+    if (g.rows <= 0) return;
+    if (g.kind == kBwdWeight) {
+        if (n == 64) launch_wgt<64>(g, num_sms, s);
+        else launch_wgt<16>(g, num_sms, s);
+    } else if (n == 64) {
+        if (g.K == 32) launch_rows<64, 32>(g, num_sms, s);
+        else launch_rows<64, 128>(g, num_sms, s);
+    } else if (n == 16) {
+        launch_rows<16, 128>(g, num_sms, s);
+    } else {
+        if (g.K == 16) launch_rows<128, 16>(g, num_sms, s);
+        else launch_rows<128, 64>(g, num_sms, s);
+    }
 }
 
 void agg_fwd(const batch::View &b, __nv_bfloat16 *buf, int C) {

@@ -36,6 +36,12 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes
     return d;
 }
 
+// The MN-major no-swizzle layout, for operands whose rows in memory run along M (or N): core matrices of 128 bytes
+// hold 8 steps of K x 8 consecutive M values (16 bytes per K).  The descriptor's offsets keep their meaning: leading =
+// from one core matrix to the next along K, stride = to the next along M; the instruction descriptor sets the major
+// bits (bit 15 A, bit 16 B).
+constexpr uint32_t kMajorMN = (1u << 15) | (1u << 16);
+
 // Instruction descriptor of tcgen05.mma kind::f16: FP32 accumulator (bits 4-5 = 1), A and B BF16 (bits 7-9,
 // 10-12 = 1), both K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
@@ -68,6 +74,17 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
 __device__ __forceinline__ void mma_commit(uint64_t *mbar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
         smem_addr(mbar)));
+}
+
+// ---- asynchronous 16-byte copies, global to shared (full = false: zeros) ----
+__device__ __forceinline__ void copy16(uint32_t dst, const void *src, bool full) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(full ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// Until at most N of this thread's groups are in flight.
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // ---- mbarrier ----
