@@ -42,6 +42,7 @@ struct LpCounters {
     int nbnd;         // boundary candidates (selection records)
     int nwin[2];      // window (selected set) sizes, double-buffered by iteration parity
     int nactive[2];   // radix-select active lists
+    int napply, apply_iter;  // movers of the iteration whose labels are due, and that iteration (k_update)
     int nchanged;     // selected vertices whose label changed (movers)
     int ndec[3];      // selected vertices per decision class
     int ndec_prev[3]; // the previous iteration's ndec (its window by class, for the marking)

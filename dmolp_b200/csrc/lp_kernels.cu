@@ -41,8 +41,8 @@ namespace {
 constexpr int kGridPerSm = 4;
 
 // ------------------------------------------------------------------------------------ begin
-// Start of iteration t (one block): counters, the iteration record, penalties.
-__device__ void lp_begin(const Buffers &b, int k, int t, long long narcs, double *s_re, double *s_tp) {
+// Start of iteration t (one block): counters, the iteration record.
+__device__ void lp_begin(const Buffers &b, int k, int t, long long narcs) {
     LpControl *ctl = b.ctrl;
     LpCounters *cn = b.cnt;
     for (int p = threadIdx.x; p < k; p += blockDim.x) b.npart[p] = 0;
@@ -70,16 +70,6 @@ __device__ void lp_begin(const Buffers &b, int k, int t, long long narcs, double
         r.te_cand = r.te_sel = r.te_stats = 0;
         r.arcs_bnd = r.arcs_dec = r.arcs_upd = r.arcs_mark = r.te_hubsel = 0;
         r.win_sum = 0;
-    }
-    // ---- statistics -> expected values and calculatePenalties (phase2.cpp:110-115, 158-209) ----
-    // (RE and the penalties in shared memory while the serial sums read them, then out to global)
-    if (threadIdx.x < 32) {
-        warp_penalties(k, [&](int p) { return sll(b.vc[p]); }, [&](int p) { return sll(b.intra[p]) / 2; },
-                       b.logtab[t], s_re, s_tp, b.penhist + (size_t)(t - 1) * DMOLP_MAX_K);
-        for (int p = threadIdx.x; p < k; p += 32) {
-            b.RE[p] = s_re[p];
-            b.tpen[p] = s_tp[p];
-        }
     }
 }
 
@@ -131,12 +121,34 @@ __global__ void k_mark_chunks(Buffers b, int t) {
     block_atomic_add(rd, &b.rec[t - 1].arcs_mark);
 }
 
+// hubwin[u] = hubs of the previous window whose rows hold u, kept across iterations: a hub that entered
+// the window (sstamp == t-1) adds one to every vertex of its row, a hub that left subtracts one.  Thread
+// per hub: flip hub_in and queue the row in kHubChunk pieces (block bx of nbx).
+__device__ __forceinline__ void hubwin_queue(const Buffers &b, int t, int nhub, int bx, int nbx) {
+    for (int i = bx * blockDim.x + threadIdx.x; i < nhub; i += nbx * blockDim.x) {
+        const int h = b.bucket[2][i];
+        const int now = b.sstamp[h] == t - 1;
+        if (now == b.hub_in[i]) continue;
+        b.hub_in[i] = now;
+        const int64_t deg = b.off[h + 1] - b.off[h];
+        const int nch = (int)((deg + kHubChunk - 1) / kHubChunk);
+        const int base = atomicAdd(&b.cnt->nhubw, nch);
+        for (int c = 0; c < nch; ++c) b.hubwq[base + c] = make_int2(i, c * kHubChunk);
+    }
+}
+
 // The loop's marking: the previous window by decision class (dec[c], ndec_prev[c]; the lists are rewritten
 // only by this iteration's selection, after the marking).  Blocks [0, g0): thread per vertex of class 0
 // (rows of at most kDecSmall arcs), then the hubs (class 2), which stamp only themselves -- their
-// neighbours are candidates through hubwin; blocks [g0, grid): warp per vertex of class 1.
-__global__ void __launch_bounds__(256, 5) k_mark_win(Buffers b, int t, int g0) {
-    if (b.ctrl->stopped || b.ctrl->pull) return;
+// neighbours are candidates through hubwin; blocks [g0, g1): warp per vertex of class 1; blocks from g1 on:
+// the hubs that entered or left the window (a launch of their own cost 5 us an iteration).
+__global__ void __launch_bounds__(256, 5) k_mark_win(Buffers b, int t, int g0, int g1, int nhub) {
+    if (b.ctrl->stopped) return;
+    if ((int)blockIdx.x >= g1) {
+        hubwin_queue(b, t, nhub, (int)blockIdx.x - g1, (int)gridDim.x - g1);
+        return;
+    }
+    if (b.ctrl->pull) return;
     const LpCounters *cn = b.cnt;
     const int lane = threadIdx.x & 31;
     unsigned long long rd = 0;
@@ -162,7 +174,7 @@ __global__ void __launch_bounds__(256, 5) k_mark_win(Buffers b, int t, int g0) {
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += stride) b.stamp[b.dec[2][i]] = t;
     } else {
         const int gw = (((int)blockIdx.x - g0) * (int)blockDim.x + (int)threadIdx.x) >> 5;
-        const int nw = (((int)gridDim.x - g0) * (int)blockDim.x) >> 5;
+        const int nw = ((g1 - g0) * (int)blockDim.x) >> 5;
         const int n1 = cn->ndec_prev[1];
         for (int i = gw; i < n1; i += nw) {
             const int v = b.dec[1][i];
@@ -176,23 +188,6 @@ __global__ void __launch_bounds__(256, 5) k_mark_win(Buffers b, int t, int g0) {
         }
     }
     block_atomic_add(rd, &b.rec[t - 1].arcs_mark);
-}
-
-// hubwin[u] = hubs of the previous window whose rows hold u, kept across iterations: a hub that entered
-// the window (sstamp == t-1) adds one to every vertex of its row, a hub that left subtracts one.  Thread
-// per hub: flip hub_in and queue the row in kHubChunk pieces.
-__global__ void k_hubwin_queue(Buffers b, int t, int nhub) {
-    if (b.ctrl->stopped) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nhub; i += gridDim.x * blockDim.x) {
-        const int h = b.bucket[2][i];
-        const int now = b.sstamp[h] == t - 1;
-        if (now == b.hub_in[i]) continue;
-        b.hub_in[i] = now;
-        const int64_t deg = b.off[h + 1] - b.off[h];
-        const int nch = (int)((deg + kHubChunk - 1) / kHubChunk);
-        const int base = atomicAdd(&b.cnt->nhubw, nch);
-        for (int c = 0; c < nch; ++c) b.hubwq[base + c] = make_int2(i, c * kHubChunk);
-    }
 }
 
 // Warp per queued chunk: +1 (hub entered) or -1 (hub left) on every vertex of the chunk.
@@ -803,6 +798,10 @@ __global__ void __launch_bounds__(256, 2) k_update(Buffers b, int k, int eff, in
     const int lane = threadIdx.x & 31;
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
     const int n = b.cnt->nchanged;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // for k_apply_turn, which resets the count
+        b.cnt->napply = n;
+        b.cnt->apply_iter = t;
+    }
     long long dcut = 0;
     unsigned long long rd = 0;
     // arc (v, u) of a mover v from label a to c, u's labels g = (old, pending or -1, hub index or -1)
@@ -919,11 +918,9 @@ __global__ void __launch_bounds__(256, 2) k_update(Buffers b, int k, int eff, in
     }
 }
 
-// Movers take their labels.
-__global__ void k_apply(Buffers b) {
-    if (b.ctrl->stopped) return;
-    const int n = b.cnt->nchanged;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+// Movers take their labels (block bx of nbx).
+__device__ __forceinline__ void apply_movers(const Buffers &b, int n, int bx, int nbx) {
+    for (int i = bx * blockDim.x + threadIdx.x; i < n; i += nbx * blockDim.x) {
         const int v = b.mov[i];
         const int nl = b.newlab[v];
         b.label[v] = nl;
@@ -931,6 +928,11 @@ __global__ void k_apply(Buffers b) {
         const int r = b.hrank[v];
         if (r >= 0) b.hotlab[r] = (unsigned)nl < 255u ? (uint8_t)nl : (uint8_t)255;
     }
+}
+
+__global__ void k_apply(Buffers b) {
+    if (b.ctrl->stopped) return;
+    apply_movers(b, b.cnt->nchanged, (int)blockIdx.x, (int)gridDim.x);
 }
 
 // ------------------------------------------------------------------------------------ stats
@@ -1296,28 +1298,57 @@ __device__ void lp_end(const Buffers &b, int k, int t, long long narcs, int mode
 }
 
 // Between iterations, one block: the end of iteration t_end (when > 0), then, unless that stopped the
-// loop, the start of iteration t_begin (when > 0).
-__global__ void k_lp_turn(Buffers b, int k, int t_end, int t_begin, long long narcs, int mode, int symmetric) {
+// loop, the start of iteration t_begin (when > 0).  Warp 1 computes the penalties of t_begin meanwhile
+// (calculatePenalties, phase2.cpp:110-115, 158-209; RE and the penalties in shared memory while the serial sums read
+// them, then out to global).
+__device__ __forceinline__ void lp_turn(const Buffers &b, int k, int t_end, int t_begin, long long narcs, int mode,
+                                        int symmetric) {
     __shared__ int s_stopped;
     __shared__ double s_re[DMOLP_MAX_K], s_tp[DMOLP_MAX_K];
     if (threadIdx.x == 0) s_stopped = b.ctrl->stopped;
     __syncthreads();
     if (s_stopped) return;
+    if (t_begin > 0 && (threadIdx.x >> 5) == 1)
+        warp_penalties(k, [&](int p) { return sll(b.vc[p]); }, [&](int p) { return sll(b.intra[p]) / 2; },
+                       b.logtab[t_begin], s_re, s_tp, b.penhist + (size_t)(t_begin - 1) * DMOLP_MAX_K);
     if (t_end > 0) {
         lp_end(b, k, t_end, narcs, mode, symmetric);
-        __syncthreads();
         if (threadIdx.x == 0) s_stopped = b.ctrl->stopped;
-        __syncthreads();
-        if (s_stopped) return;
     }
-    if (t_begin > 0) lp_begin(b, k, t_begin, narcs, s_re, s_tp);
+    __syncthreads();
+    if (s_stopped || t_begin <= 0) return;
+    lp_begin(b, k, t_begin, narcs);
+    for (int p = threadIdx.x; p < k; p += blockDim.x) {
+        b.RE[p] = s_re[p];
+        b.tpen[p] = s_tp[p];
+    }
 }
 
-// Asymmetric graphs: decide whether the full statistics pass runs (the reference skips it on an empty
-// window and, with its stopping rules, on zero changes) and clear its accumulators.
-__global__ void k_lp_mid(Buffers b, int k, int t, int mode) {
+__global__ void __launch_bounds__(256) k_lp_turn(Buffers b, int k, int t_end, int t_begin, long long narcs, int mode,
+                                                 int symmetric) {
+    lp_turn(b, k, t_end, t_begin, narcs, mode, symmetric);
+}
+
+// Symmetric graphs: block 0 turns the iteration while the others give the movers their labels, in one launch (two
+// cost 5 us more an iteration).  The movers' number comes from k_update: the turn resets the count, and may stop the
+// loop, while the labels are written; apply_iter tells an iteration that ran from one after the stop.
+__global__ void __launch_bounds__(256) k_apply_turn(Buffers b, int k, int t_end, int t_begin, long long narcs, int mode) {
+    if (blockIdx.x == 0) {
+        lp_turn(b, k, t_end, t_begin, narcs, mode, 1);
+        return;
+    }
+    if (b.cnt->apply_iter == t_end) apply_movers(b, b.cnt->napply, (int)blockIdx.x - 1, (int)gridDim.x - 1);
+}
+
+// Asymmetric graphs: the movers take their labels, while block 0 decides whether the full statistics pass runs (the
+// reference skips it on an empty window and, with its stopping rules, on zero changes) and clears its accumulators.
+__global__ void __launch_bounds__(256) k_apply_mid(Buffers b, int k, int t, int mode) {
     LpControl *ctl = b.ctrl;
     if (ctl->stopped) return;
+    if (blockIdx.x > 0) {
+        apply_movers(b, b.cnt->nchanged, (int)blockIdx.x - 1, (int)gridDim.x - 1);
+        return;
+    }
     __shared__ int s_skip;
     if (threadIdx.x == 0) {
         const int win = b.cnt->nwin[t & 1], ch = b.cnt->nchanged;
@@ -1337,6 +1368,7 @@ __global__ void k_lp_mid(Buffers b, int k, int t, int mode) {
 __global__ void k_lp_init_end(Buffers b, int mode) {
     LpControl *ctl = b.ctrl;
     const unsigned long long arcs = b.cnt->cut_arcs;
+    b.cnt->apply_iter = 0;
     ctl->mode = mode;
     ctl->conv = 0;
     ctl->iters_run = 0;
@@ -1831,12 +1863,12 @@ void lp_iteration(dmolp_ctx *c, const LpLaunch &L, int t, bool first, bool last)
     if (t > 1) {
         // the previous window by decision class; hubs through hubwin
         ProfScope ps(c, 2, t);
-        k_mark_win<<<grid, kBlock, 0, c->stream>>>(b, t, grid / 2);
+        const int gq = c->nb[2] > 0 ? clampi((c->nb[2] + 255) / 256, 1, grid) : 0;
+        k_mark_win<<<grid + gq, kBlock, 0, c->stream>>>(b, t, grid / 2, grid, c->nb[2]);
         c->launches += 1;
         if (c->nb[2] > 0) {
-            k_hubwin_queue<<<clampi((c->nb[2] + 255) / 256, 1, grid), kBlock, 0, c->stream>>>(b, t, c->nb[2]);
             k_hubwin_apply<<<grid, kBlock, 0, c->stream>>>(b, t);
-            c->launches += 2;
+            c->launches += 1;
         }
     }
     const bool deg_sel = L.k <= kDegSelMaxK;  // the degree-bin selection (else the radix selection)
@@ -1864,17 +1896,15 @@ void lp_iteration(dmolp_ctx *c, const LpLaunch &L, int t, bool first, bool last)
             k_update<<<grid, kBlock, 2 * L.k * sizeof(unsigned long long), c->stream>>>(b, L.k, L.eff, t,
                                                                                          c->counts_kept ? 1 : 0);
         }
-        k_apply<<<grid, kBlock, 0, c->stream>>>(b);
+        k_apply_turn<<<grid + 1, kBlock, 0, c->stream>>>(b, L.k, t, last ? 0 : t + 1, (long long)c->narcs, L.mode);
         c->launches += 2;
     } else {
-        k_apply<<<grid, kBlock, 0, c->stream>>>(b);
-        k_lp_mid<<<1, 256, 0, c->stream>>>(b, L.k, t, L.mode);
+        k_apply_mid<<<grid + 1, kBlock, 0, c->stream>>>(b, L.k, t, L.mode);
         const StatsArgs a = stats_args(c, L.k, true);
         k_stats<<<stats_grid(c, a), kBlock, stats_smem(a), c->stream>>>(b, a, stopped, &b.ctrl->skip_stats);
+        k_lp_turn<<<1, 256, 0, c->stream>>>(b, L.k, t, last ? 0 : t + 1, (long long)c->narcs, L.mode, sym);
         c->launches += 3;
     }
-    k_lp_turn<<<1, 256, 0, c->stream>>>(b, L.k, t, last ? 0 : t + 1, (long long)c->narcs, L.mode, sym);
-    c->launches += 1;
 }
 
 // dmolp_window_select: previous window in win[(t-1)&1] (nprev entries), RE in b.RE, stamps cleared.
