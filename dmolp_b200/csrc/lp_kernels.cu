@@ -218,6 +218,7 @@ struct BndArgs {
     unsigned int *dsup;  // when set: degree-superbin counts of the boundary records per label (k <= 64)
     int nb0, nb1, nb2;
     int g0, g1;  // block split: [0,g0) thread class, [g0,g0+g1) warp class, rest block class
+    int push_blocks;  // push mode: blocks that take part
 };
 
 __device__ __forceinline__ uint64_t sel_key(const Buffers &b, int own, int deg, int v, int ibits, int maxdeg) {
@@ -243,6 +244,10 @@ constexpr int kBndPushU = 4;  // k_bnd push mode: record slots per thread and st
 
 __global__ void __launch_bounds__(256, 5) k_bnd(Buffers b, BndArgs a, int k) {
     if (b.ctrl->stopped) return;
+    const bool pull = !a.all && b.ctrl->pull;
+    // every block clears and adds k superbin tables: in push mode, whose slots cost the same, only as many as are
+    // resident take part
+    if (!pull && (int)blockIdx.x >= a.push_blocks) return;
     // [k] boundary records per label in this block, then [k * 256] first-digit or [k * kDsBins] superbin counts
     extern __shared__ int s_npart[];
     unsigned int *s_hist = reinterpret_cast<unsigned int *>(s_npart + k);
@@ -250,7 +255,6 @@ __global__ void __launch_bounds__(256, 5) k_bnd(Buffers b, BndArgs a, int k) {
     const int nhist = a.dsup ? k * kDsBins : (a.hist ? k * kRadix : 0);
     for (int i = threadIdx.x; i < nhist; i += blockDim.x) s_hist[i] = 0u;
     __syncthreads();
-    const bool pull = !a.all && b.ctrl->pull;
     const int tp = a.t - 1;
     const int lane = threadIdx.x & 31;
     unsigned long long te = 0, rd = 0, nc = 0, nbd = 0;
@@ -277,7 +281,7 @@ __global__ void __launch_bounds__(256, 5) k_bnd(Buffers b, BndArgs a, int k) {
         // ---- every record slot, thread per slot; kBndPushU slots per thread with their loads in flight
         //      together (the per-slot chain slot -> vertex state -> offsets is latency, not bandwidth) ----
         const int n = a.nb0 + a.nb1 + a.nb2;
-        const int nt = (int)gridDim.x * (int)blockDim.x;
+        const int nt = min((int)gridDim.x, a.push_blocks) * (int)blockDim.x;
         for (int p0 = blockIdx.x * blockDim.x + threadIdx.x; p0 < n; p0 += kBndPushU * nt) {
             int v[kBndPushU], st[kBndPushU], hw[kBndPushU], nd[kBndPushU], lv[kBndPushU], deg[kBndPushU];
             bool cand[kBndPushU];
@@ -1645,6 +1649,7 @@ BndArgs bnd_args(dmolp_ctx *c, int t, int all, int hubwin, int k, bool hist_for_
     const int cap = c->num_sms * 8;
     a.g0 = clampi((c->nb[0] + 255) / 256, 1, cap);
     a.g1 = clampi((c->nb[1] + 7) / 8, 1, cap);
+    a.push_blocks = c->num_sms * 5;
     return a;
 }
 

@@ -227,6 +227,10 @@ __global__ void __launch_bounds__(kDsThreads, 1) k_select_deg(DegSelArgs a) {
             np_[u] = r < whi ? a.seg[r] : -1;
             nkey[u] = r < whi ? a.key[r] : 0;
         }
+        bool some = false;
+#pragma unroll
+        for (int u = 0; u < kDsU; ++u) some |= p[u] >= 0;
+        if (!__any_sync(DMOLP_FULL_MASK, some)) continue;  // empty slots only
 #pragma unroll
         for (int u = 0; u < kDsU; ++u) {
             take[u] = part[u] = false;
