@@ -236,6 +236,8 @@ struct dmolp_ctx {
 };
 
 constexpr int kUpSlots = 3;
-constexpr size_t kUpSlot = 2u << 20;  // bytes per slot of an upload's staging
+// Bytes per slot of an upload's staging: small enough that a slot is still in the host's caches when it is sent, and
+// cheap to pin (123 MB: 3.5 ms and 8.5 the first time on a context; with slots of 2 MB 4.2 and 11 to 26).
+constexpr size_t kUpSlot = 512u << 10;
 constexpr int kPinSlots = 4;
 constexpr int64_t kPinSlot = 32ll << 20;  // bytes per staging slot
