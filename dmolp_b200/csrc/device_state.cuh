@@ -85,6 +85,17 @@ struct LpRecordDev {
     unsigned long long win_sum;    // sum of window_mix(v) over the selected window (order-independent checksum)
 };
 
+// Hub list on the device (seed_kernels.cu): degree statistics, the sort's range when it is handed to the host.
+struct HubState {
+    unsigned long long total;  // sum of the raw degrees
+    int dmax;                  // their maximum D
+    int vhigh, vlow;           // highest vertex of degree D; lowest one with an id below D (INT_MAX: none)
+    int first, depth, cut;     // range [first, nv), depth left, cut (-1, or the range was partitioned there)
+    int cutl[2];               // scratch
+};
+constexpr int64_t kHubDeviceMin = 1 << 17;  // vertices from which the sort starts on the device ...
+constexpr int kHubHostMax = 1 << 14;        // ... and the pairs that are left to the host
+
 struct Buffers {
     // graph
     int64_t *off = nullptr;    // [nv+1]
@@ -164,6 +175,7 @@ struct Buffers {
     int32_t *hubs = nullptr;             // [nv]
     int32_t *claim = nullptr;            // [nv] (aliases stamp)
     unsigned long long *best = nullptr;  // [2] packed hub argmax, by seed parity
+    HubState *hubst = nullptr;           // [1]
     int *p1cnt = nullptr;                // [8] phase-1 counters
     unsigned long long *p1te = nullptr;  // [1]
     int *flag = nullptr;                 // [1] scratch flag (symmetry check)

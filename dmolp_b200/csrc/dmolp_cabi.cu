@@ -303,6 +303,7 @@ size_t layout(dmolp_ctx *c, char *base, int64_t nv, int64_t narcs, const size_t 
     ALLOC(b.intra, DMOLP_MAX_K);
     ALLOC(b.cnt, 1);
     ALLOC(b.ctrl, 1);
+    ALLOC(b.hubst, 1);
     ALLOC(b.p1cnt, 8);
     ALLOC(b.p1te, 1);
     ALLOC(b.rec, kMaxIter);
@@ -1028,12 +1029,76 @@ static int find_seeds_impl(dmolp_ctx *c, int k, int first, const std::vector<int
     return DMOLP_OK;
 }
 
+// The host mirror of the raw degrees, fetched when first needed.
+static int host_degrees(dmolp_ctx *c) {
+    if (c->h_rawdeg_valid) return DMOLP_OK;
+    c->h_rawdeg.resize(c->nv);
+    if (c->nv)
+        DMOLP_CUDA(cudaMemcpyAsync(c->h_rawdeg.data(), c->b.rawdeg, (size_t)c->nv * sizeof(int32_t),
+                                   cudaMemcpyDeviceToHost, c->stream));
+    const int st = sync(c);
+    if (st) return st;
+    c->h_rawdeg_valid = true;
+    return DMOLP_OK;
+}
+
+// The hub list (find_hub_nodes, init.cpp:139-177) with the hubs' degrees, and the first seed (init.cpp:179-187).
+// Large graphs: the degree statistics come from the device, and so do the sort's first partitions when the hubs are
+// few (the sort then follows the right sides); what is left, at most kHubHostMax pairs or a range just split at the
+// hubs' start, is finished here.  Measured on a million vertices with 464 hubs: 2.4 -> 0.21 ms, and the raw
+// degrees stay on the device.  Where the hubs are many (meshes: more than half of the vertices) the whole order is
+// nearly needed, and the host's parallel sort does it.
+static int hub_list(dmolp_ctx *c, std::vector<int> &hubs, std::vector<int> &degree, int *first) {
+    Buffers &b = c->b;
+    const int64_t nv = c->nv;
+    hubs.clear();
+    degree.clear();
+    if (nv >= kHubDeviceMin && c->num_sms <= 256) {
+        p1_hub_stats(c);
+        int st = fetch(c, b.rec);
+        if (!st) st = report_waits(c, host_of(c, b.ctrl)->wait_timeout);
+        if (st) return st;
+        const HubState hs = *host_of(c, b.hubst);
+        const int64_t H = dmolp::hub_count(nv, (int64_t)hs.total, hs.dmax), t0 = nv - H;
+        *first = hs.vlow != INT_MAX ? hs.vlow : hs.vhigh;
+        if (H == 0) return DMOLP_OK;
+        if (H <= nv / 16) {
+            p1_hub_top(c, t0, dmolp::introsort_depth(nv));
+            st = fetch(c, b.rec);
+            if (!st) st = report_waits(c, host_of(c, b.ctrl)->wait_timeout);
+            if (st) return st;
+            const HubState ht = *host_of(c, b.hubst);
+            const int64_t m = nv - ht.first;
+            std::vector<std::pair<int32_t, int32_t>> a((size_t)m + 1);
+            a[0] = std::make_pair(-1, INT32_MIN);  // stands for what lies in front of the range
+            static_assert(sizeof(a[0]) == sizeof(uint64_t), "pairs are copied as they are on the device");
+            DMOLP_CUDA(cudaMemcpyAsync(a.data() + 1, b.dlkey + ht.first, (size_t)m * sizeof(uint64_t),
+                                       cudaMemcpyDeviceToHost, c->stream));
+            st = sync(c);
+            if (st) return st;
+            dmolp::finish_top(a.data() + 1, m, t0 - ht.first, ht.depth, ht.cut < 0 ? -1 : ht.cut - ht.first, ht.first == 0);
+            for (int64_t i = m; i > m - H; --i) {
+                hubs.push_back(a[(size_t)i].first);
+                degree.push_back(a[(size_t)i].second);
+            }
+            return DMOLP_OK;
+        }
+    }
+    const int st = host_degrees(c);
+    if (st) return st;
+    hubs = find_hubs(c->h_rawdeg);
+    for (int h : hubs) degree.push_back(c->h_rawdeg[h]);
+    *first = dmolp::first_seed_of(c->h_rawdeg.data(), nv).first;  // including its id-vs-degree tie test
+    return DMOLP_OK;
+}
+
 // Seed completion: where the reference rule found fewer than k seeds the reference reads past its seed
 // vector (partition.cpp:347).  Remaining seeds: unused hubs by raw degree (first in hub order on ties),
 // then other vertices by raw degree (lowest id on ties).
-static void complete_seeds(dmolp_ctx *c, int k, const std::vector<int> &hubs, std::vector<int> &seeds) {
+static int complete_seeds(dmolp_ctx *c, int k, const std::vector<int> &hubs, const std::vector<int> &hub_degree,
+                          std::vector<int> &seeds) {
     const int64_t nv = c->nv;
-    if ((int64_t)seeds.size() >= k || nv <= 0) return;
+    if ((int64_t)seeds.size() >= k || nv <= 0) return DMOLP_OK;
     std::vector<char> used(hubs.size(), 0), is_seed(nv, 0);
     for (int s : seeds) {
         is_seed[s] = 1;
@@ -1044,17 +1109,20 @@ static void complete_seeds(dmolp_ctx *c, int k, const std::vector<int> &hubs, st
         int bestv = -1, bd = -1;
         int64_t bi = -1;
         for (size_t i = 0; i < hubs.size(); ++i)
-            if (!used[i] && c->h_rawdeg[hubs[i]] > bd) {
-                bd = c->h_rawdeg[hubs[i]];
+            if (!used[i] && hub_degree[i] > bd) {
+                bd = hub_degree[i];
                 bestv = hubs[i];
                 bi = (int64_t)i;
             }
-        if (bestv == -1)
+        if (bestv == -1) {
+            const int st = host_degrees(c);
+            if (st) return st;
             for (int64_t v = 0; v < nv; ++v)
                 if (!is_seed[v] && c->h_rawdeg[v] > bd) {
                     bd = c->h_rawdeg[v];
                     bestv = (int)v;
                 }
+        }
         if (bestv == -1) break;
         seeds.push_back(bestv);
         is_seed[bestv] = 1;
@@ -1064,6 +1132,7 @@ static void complete_seeds(dmolp_ctx *c, int k, const std::vector<int> &hubs, st
             if (it != hubs.end()) used[it - hubs.begin()] = 1;
         }
     }
+    return DMOLP_OK;
 }
 
 // Growth rounds (partition.cpp:335-604); seedk[p] = -1 for a part without a seed.  Launched only: the rounds are
@@ -1130,33 +1199,26 @@ int dmolp_phase1(dmolp_ctx *c, int k, int theta, int32_t *seeds_out, int64_t *ve
     DMOLP_CUDA(cudaSetDevice(c->device));
     Buffers &b = c->b;
     const int64_t nv = c->nv;
-    if (!c->h_rawdeg_valid) {  // a device-parsed graph: fetch the raw degrees once
-        c->h_rawdeg.resize(nv);
-        if (nv)
-            DMOLP_CUDA(cudaMemcpyAsync(c->h_rawdeg.data(), b.rawdeg, (size_t)nv * sizeof(int32_t),
-                                       cudaMemcpyDeviceToHost, c->stream));
-        int s0 = sync(c);
-        if (s0) return s0;
-        c->h_rawdeg_valid = true;
-    }
     dmolp_phase1_info inf;
     std::memset(&inf, 0, sizeof(inf));
     DMOLP_CUDA(cudaEventRecord(c->ev0, c->stream));
 
-    // ---- hubs and first seed on the host (order-dependent; see the top of this file) ----
+    // ---- hubs and first seed (order-dependent; see the top of this file) ----
     const auto th0 = std::chrono::steady_clock::now();
-    std::vector<int> hubs = find_hubs(c->h_rawdeg);
-    // init.cpp:179-187, including its id-vs-degree tie test
-    const std::pair<int, int> first = dmolp::first_seed_of(c->h_rawdeg.data(), nv);
+    std::vector<int> hubs, hub_degree;
+    int first = -1;
+    st = hub_list(c, hubs, hub_degree, &first);
+    if (st) return st;
     inf.num_hubs = (int64_t)hubs.size();
     DMOLP_CUDA(cudaMemsetAsync(b.p1te, 0, sizeof(unsigned long long), c->stream));
     const auto th1 = std::chrono::steady_clock::now();
     inf.hubs_ms = std::chrono::duration<double, std::milli>(th1 - th0).count();
     std::vector<int> seeds;
-    st = find_seeds_impl(c, k, first.first, hubs, seeds);
+    st = find_seeds_impl(c, k, first, hubs, seeds);
     if (st) return st;
     inf.num_seeds_found = (int32_t)seeds.size();
-    complete_seeds(c, k, hubs, seeds);
+    st = complete_seeds(c, k, hubs, hub_degree, seeds);
+    if (st) return st;
     const auto th2 = std::chrono::steady_clock::now();
     inf.seeds_ms = std::chrono::duration<double, std::milli>(th2 - th1).count();
     std::vector<int32_t> seedk(k, -1);

@@ -321,18 +321,9 @@ void top_by_degree(Pair *a, int64_t n, int64_t t0) {
 // of non-negative integers below 2^53 is exact in a double, so the integer total and the largest degree give
 // the same bits, and the number of hubs H follows from them before any sorting: only the top H places of
 // std::sort's order are computed (top_by_degree), not the whole order.
-std::vector<int> hubs_of_pairs(Pair *sd, int64_t n) {
+int64_t hub_count(int64_t n, int64_t total_i, int32_t dmax) {
     const int N = (int)n;
-    std::vector<int> hubs;
-    if (N < 2) return hubs;
-    int64_t total_i = 0;
-    int32_t dmax = INT32_MIN;
-#pragma omp parallel for reduction(+ : total_i) reduction(max : dmax) schedule(static) \
-    if (N >= kParallelMin && !omp_in_parallel())
-    for (int i = 0; i < N; ++i) {
-        total_i += sd[i].second;
-        dmax = std::max(dmax, sd[i].second);
-    }
+    if (N < 2) return 0;
     const double total = (double)total_i;
     const double y1 = (double)total_i / total, y0 = (double)(total_i - dmax) / total;
     const double inv_n = 1.0 / N;
@@ -345,10 +336,45 @@ std::vector<int> hubs_of_pairs(Pair *sd, int64_t n) {
         if ((i + 1) * inv_n > x_int) ++H;
         else break;
     }
+    return H;
+}
+
+std::vector<int> hubs_of_pairs(Pair *sd, int64_t n) {
+    const int N = (int)n;
+    std::vector<int> hubs;
+    if (N < 2) return hubs;
+    int64_t total_i = 0;
+    int32_t dmax = INT32_MIN;
+#pragma omp parallel for reduction(+ : total_i) reduction(max : dmax) schedule(static) \
+    if (N >= kParallelMin && !omp_in_parallel())
+    for (int i = 0; i < N; ++i) {
+        total_i += sd[i].second;
+        dmax = std::max(dmax, sd[i].second);
+    }
+    const int H = (int)hub_count(n, total_i, dmax);
     if (H == 0) return hubs;
     top_by_degree(sd, n, n - H);
     for (int i = N - 1; i >= N - H; --i) hubs.push_back(sd[i].first);
     return hubs;
+}
+
+int introsort_depth(int64_t n) { return 2 * lg(n); }
+
+// The rest of top_by_degree after its first steps ran elsewhere: a[0, m) is the loop's current range, the end of the
+// whole array (whole: it is the whole array), t0 in it, depth what is left of the limit.  cut >= 0: the range has just
+// been partitioned at cut, above t0.  Unless whole, a[-1] must not be above anything in a.
+void finish_top(Pair *a, int64_t m, int64_t t0, int64_t depth, int64_t cut, bool whole) {
+    Pair *last = a + m, *leaf = a;
+    if (cut >= 0) {
+        introsort_loop(a + cut, last, depth, false);
+        last = a + cut;
+    }
+    top_loop(a, last, depth, a + t0, &leaf, false);
+    if (whole && leaf == a) {
+        final_insertion(a, m, threads_for(m));
+        return;
+    }
+    for (Pair *i = leaf; i != a + m; ++i) linear_insert(i);
 }
 
 // find_hub_nodes on pairs in the reference's map order.

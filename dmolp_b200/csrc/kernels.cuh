@@ -13,6 +13,11 @@ namespace dmolp {
 std::vector<int> hubs_from_pairs(std::vector<std::pair<int, int>> sd);
 // The same on the raw degrees of one rank (pairs in map order, vertex V-1 down to 0, built on all threads).
 std::vector<int> hubs_from_degrees(const int32_t *degree, int64_t nv);
+// The number of hubs of n vertices with the given sum and maximum of degrees; the sort's depth limit; and the rest of
+// the top of its order from where the device left it (hubsort.cpp).
+int64_t hub_count(int64_t n, int64_t total, int32_t dmax);
+int introsort_depth(int64_t n);
+void finish_top(std::pair<int32_t, int32_t> *a, int64_t m, int64_t t0, int64_t depth, int64_t cut, bool whole);
 // find_first_seed's (vertex, degree) over that order, its id-vs-degree tie test included.
 std::pair<int, int> first_seed_of(const int32_t *degree, int64_t nv);
 
@@ -82,6 +87,12 @@ void loop_run(dmolp_ctx *c, const LpLaunch &L, int iters);  // every iteration, 
 void loop_prepare();  // kernel attributes
 
 // ---- phase 1 (seed_kernels.cu) ----
+// Sum and maximum of the raw degrees, and what find_first_seed's closed form needs, to *b.hubst.
+void p1_hub_stats(dmolp_ctx *c);
+// The first steps of the hub sort on pairs (vertex, degree) in the reference's order, built in b.dlkey: Hoare
+// partitions as long as the right side holds position t0 and more than kHubHostMax pairs are left; the state to
+// *b.hubst.
+void p1_hub_top(dmolp_ctx *c, int64_t t0, int depth);
 // Seeds by the reference rule from b.hubs[0, nhubs) and the first seed: b.need[0, found), found = p1cnt[6].
 // b.covered, b.best and p1cnt are cleared by the caller.
 void p1_find_seeds(dmolp_ctx *c, int k, int first, int64_t nhubs);

@@ -393,6 +393,214 @@ __global__ void __launch_bounds__(kSelThreads, 1) k_p1_grow(Buffers b, const Sel
     if (lane == 0 && te) atomicAdd(b.p1te, te);
 }
 
+// ------------------------------------------------------------------------------------ hub list
+// Degree statistics: total, maximum D, then find_first_seed's closed form (hubsort.cpp, first_seed_of).
+__global__ void __launch_bounds__(kSelThreads, 1) k_hub_stats(Buffers b, LpControl *ctl, int nv, unsigned int polls) {
+    HubState *const h = b.hubst;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        h->total = 0;
+        h->dmax = INT_MIN;
+        h->vhigh = -1;
+        h->vlow = INT_MAX;
+    }
+    if (!grid_sync(ctl, polls, 50)) return;
+    unsigned long long sum = 0;
+    int mx = INT_MIN;
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
+        const int d = b.rawdeg[v];
+        sum += (unsigned long long)d;
+        mx = max(mx, d);
+    }
+    sum = warp_sum_u64(sum);
+    mx = __reduce_max_sync(DMOLP_FULL_MASK, mx);
+    if ((threadIdx.x & 31) == 0) {
+        if (sum) atomicAdd(&h->total, sum);
+        atomicMax(&h->dmax, mx);
+    }
+    if (!grid_sync(ctl, polls, 51)) return;
+    const int D = __ldcg(&h->dmax);
+    int hi = -1, lo = INT_MAX;
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x)
+        if (b.rawdeg[v] == D) {
+            hi = max(hi, v);
+            if (v < D) lo = min(lo, v);
+        }
+    if (hi >= 0) atomicMax(&h->vhigh, hi);
+    if (lo != INT_MAX) atomicMin(&h->vlow, lo);
+}
+
+// The swap of libstdc++'s median-of-three: the pivot to position r.
+__device__ __forceinline__ void median_swap(int2 *a, int r, int x, int y, int z) {
+    const int dx = a[x].y, dy = a[y].y, dz = a[z].y;
+    int m;
+    if (dx < dy) m = dy < dz ? y : (dx < dz ? z : x);
+    else m = dx < dz ? x : (dy < dz ? z : y);
+    const int2 t = a[r];
+    a[r] = a[m];
+    a[m] = t;
+}
+
+// std::sort's partitions of (vertex, degree) pairs by degree, followed into the right side while it holds position t0
+// (hubsort.cpp, top_by_degree, does the same on the host: 1.9 ms for a million pairs; the whole list now takes 0.21).
+// Hoare's scans pair the k-th position from the left whose degree is not below the pivot's with the k-th from the right
+// whose degree is not above it, and swap while the left one lies before the right one.  With l(p) such positions left
+// of p and r(p) at or right of it, the number of swaps is the maximum over p of min(l(p), r(p)); l grows and r falls,
+// so the maximum lies in the block's slice where they cross.  The cut is the next left position, or the last swapped
+// right one if that comes first.  Per partition: pivot | counts | pairs listed by rank | swaps, a barrier each.
+__global__ void __launch_bounds__(kSelThreads, 1) k_hub_top(Buffers b, LpControl *ctl, int nv, int t0, int depth,
+                                                            unsigned int polls) {
+    constexpr int kW = kSelThreads / 32, kMaxGrid = 256;
+    __shared__ int s_l[kW], s_r[kW], s_bl[kMaxGrid + 1], s_br[kMaxGrid + 1], s_star, s_m;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, G = gridDim.x, B = blockIdx.x;
+    const unsigned upto = lane == 31 ? ~0u : (2u << lane) - 1u;  // this lane and those below
+    int2 *const a = reinterpret_cast<int2 *>(b.dlkey);
+    int *const blk = reinterpret_cast<int *>(b.psize);  // [2 * G] counts of every block
+    int32_t *const posl = b.cand, *const posr = b.bv;
+    HubState *const h = b.hubst;
+    for (int i = B * blockDim.x + threadIdx.x; i < nv; i += G * blockDim.x)
+        a[i] = make_int2(nv - 1 - i, b.rawdeg[nv - 1 - i]);
+    if (B == 0 && threadIdx.x == 0) h->cutl[0] = h->cutl[1] = INT_MAX;
+    if (!grid_sync(ctl, polls, 52)) return;
+    int first = 0, split = -1;
+    for (int par = 0; nv - first > kHubHostMax && depth > 0; par ^= 1) {
+        --depth;
+        if (B == 0 && threadIdx.x == 0) {
+            median_swap(a, first, first + 1, first + (nv - first) / 2, nv - 1);
+            h->cutl[par ^ 1] = INT_MAX;  // last read before the last barrier
+        }
+        if (!grid_sync(ctl, polls, 53)) return;
+        const int pv = a[first].y, lo0 = first + 1, n = nv - lo0;
+        const int len = (n + G - 1) / G, wlen = ((len + kW - 1) / kW + 31) & ~31;
+        // warp w's share [x, y) of block sb's slice
+        auto share = [&](int sb, int &x, int &y) {
+            const int s = lo0 + min(n, sb * len), e = lo0 + min(n, (sb + 1) * len);
+            x = min(e, s + w * wlen);
+            y = min(e, x + wlen);
+        };
+        auto count = [&](int sb) {
+            int x, y, cl = 0, cr = 0;
+            share(sb, x, y);
+            for (int i = x + lane; i < y; i += 32) {
+                const int d = a[i].y;
+                cl += d >= pv;
+                cr += d <= pv;
+            }
+            cl = __reduce_add_sync(DMOLP_FULL_MASK, cl);
+            cr = __reduce_add_sync(DMOLP_FULL_MASK, cr);
+            if (lane == 0) {
+                s_l[w] = cl;
+                s_r[w] = cr;
+            }
+            __syncthreads();
+        };
+        // counts in front of warp w's share, from the slice's start
+        auto before = [&](int &cl, int &cr) {
+            cl = __reduce_add_sync(DMOLP_FULL_MASK, lane < w ? s_l[lane] : 0);
+            cr = __reduce_add_sync(DMOLP_FULL_MASK, lane < w ? s_r[lane] : 0);
+        };
+        count(B);
+        if (w == 0) {
+            const int cl = __reduce_add_sync(DMOLP_FULL_MASK, s_l[lane]), cr = __reduce_add_sync(DMOLP_FULL_MASK, s_r[lane]);
+            if (lane == 0) {
+                blk[B] = cl;
+                blk[G + B] = cr;
+            }
+        }
+        int myl, myr;
+        before(myl, myr);
+        if (!grid_sync(ctl, polls, 54)) return;
+        if (w == 0) {  // exclusive prefixes over the blocks
+            int bl = 0, br = 0;
+            for (int j0 = 0; j0 < G; j0 += 32) {
+                const int j = j0 + lane;
+                const int cl = j < G ? __ldcg(blk + j) : 0, cr = j < G ? __ldcg(blk + G + j) : 0;
+                int il = cl, ir = cr;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int yl = __shfl_up_sync(DMOLP_FULL_MASK, il, o), yr = __shfl_up_sync(DMOLP_FULL_MASK, ir, o);
+                    if (lane >= o) {
+                        il += yl;
+                        ir += yr;
+                    }
+                }
+                if (j < G) {
+                    s_bl[j + 1] = bl + il;
+                    s_br[j + 1] = br + ir;
+                }
+                bl += __shfl_sync(DMOLP_FULL_MASK, il, 31);
+                br += __shfl_sync(DMOLP_FULL_MASK, ir, 31);
+            }
+            if (lane == 0) {
+                s_bl[0] = s_br[0] = 0;
+                s_star = INT_MAX;
+            }
+        }
+        __syncthreads();
+        const int totr = s_br[G];
+        for (int j = threadIdx.x; j < G; j += blockDim.x)
+            if (s_bl[j + 1] >= totr - s_br[j + 1]) atomicMin(&s_star, j);
+        __syncthreads();
+        const int star = s_star;  // the slice in which the counts cross (the last slice: r is 0 at its end)
+        if (threadIdx.x == 0) s_m = min(s_bl[star], totr - s_br[star]);
+        count(star);
+        {
+            int x, y, cl, cr, best = 0;
+            before(cl, cr);
+            cl += s_bl[star];
+            cr += s_br[star];
+            share(star, x, y);
+            for (int i0 = x; i0 < y; i0 += 32) {
+                const int i = i0 + lane;
+                const int d = i < y ? a[i].y : 0;
+                const unsigned ml = __ballot_sync(DMOLP_FULL_MASK, i < y && d >= pv);
+                const unsigned mr = __ballot_sync(DMOLP_FULL_MASK, i < y && d <= pv);
+                if (i < y) best = max(best, min(cl + __popc(ml & upto), totr - cr - __popc(mr & upto)));
+                cl += __popc(ml);
+                cr += __popc(mr);
+            }
+            best = __reduce_max_sync(DMOLP_FULL_MASK, best);
+            if (lane == 0) atomicMax(&s_m, best);
+        }
+        __syncthreads();
+        const int m = s_m;  // swaps; the same in every block
+        {
+            int x, y, cl = s_bl[B] + myl, cr = s_br[B] + myr;
+            share(B, x, y);
+            for (int i0 = x; i0 < y; i0 += 32) {
+                const int i = i0 + lane;
+                const int d = i < y ? a[i].y : 0;
+                const bool left = i < y && d >= pv, right = i < y && d <= pv;
+                const unsigned ml = __ballot_sync(DMOLP_FULL_MASK, left), mr = __ballot_sync(DMOLP_FULL_MASK, right);
+                const int rl = cl + __popc(ml & upto) - 1;         // 0-based from the left
+                const int rr = totr - (cr + __popc(mr & upto));    // 0-based from the right
+                if (left && rl < m) posl[rl] = i;
+                if (left && rl == m) h->cutl[par] = i;
+                if (right && rr < m) posr[rr] = i;
+                cl += __popc(ml);
+                cr += __popc(mr);
+            }
+        }
+        if (!grid_sync(ctl, polls, 55)) return;
+        const int cut = min(__ldcg(&h->cutl[par]), m > 0 ? __ldcg(posr + m - 1) : INT_MAX);
+        for (int q = B * blockDim.x + threadIdx.x; q < m; q += G * blockDim.x) {
+            const int i = posl[q], j = posr[q];
+            const int2 t = a[i];
+            a[i] = a[j];
+            a[j] = t;
+        }
+        if (!grid_sync(ctl, polls, 56)) return;
+        if (cut > t0) {
+            split = cut;
+            break;
+        }
+        first = cut;
+    }
+    if (B == 0 && threadIdx.x == 0) {
+        h->first = first;
+        h->depth = depth;
+        h->cut = split;
+    }
+}
+
 size_t grow_smem(int k, int *off) {
     const size_t stage = (size_t)(kSelThreads / 32) * kStageP1 * sizeof(int32_t);
     const size_t sel = std::max((select_smem_bytes(k) + 15) & ~(size_t)15, stage);
@@ -419,6 +627,14 @@ void launch_resident(dmolp_ctx *c, K kernel, size_t smem, A... args) {
 }
 
 }  // namespace
+
+void p1_hub_stats(dmolp_ctx *c) {
+    launch_resident(c, k_hub_stats, 0, c->b, c->b.ctrl, (int)c->nv, c->wait_polls);
+}
+
+void p1_hub_top(dmolp_ctx *c, int64_t t0, int depth) {
+    launch_resident(c, k_hub_top, 0, c->b, c->b.ctrl, (int)c->nv, (int)t0, depth, c->wait_polls);
+}
 
 void p1_find_seeds(dmolp_ctx *c, int k, int first, int64_t nhubs) {
     launch_resident(c, k_p1_find_seeds, 0, c->b, k, first, (int)nhubs, c->wait_polls);
