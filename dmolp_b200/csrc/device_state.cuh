@@ -251,5 +251,7 @@ constexpr int kUpSlots = 3;
 // Bytes per slot of an upload's staging: small enough that a slot is still in the host's caches when it is sent, and
 // cheap to pin (123 MB: 3.5 ms and 8.5 the first time on a context; with slots of 2 MB 4.2 and 11 to 26).
 constexpr size_t kUpSlot = 512u << 10;
+// Arrays from this size on: pinning costs 3 to 8 ms the first time on a context, and 32 MB gain 2.
+constexpr size_t kUpMin = 32u << 20;
 constexpr int kPinSlots = 4;
 constexpr int64_t kPinSlot = 32ll << 20;  // bytes per staging slot

@@ -1,8 +1,8 @@
 // C-ABI entry points (include/dmolp_b200.h): context, resident graph, phase 1, phase 2, metrics.
 //
-// Host-side steps that decide ORDER-dependent results stay on the host, in the reference's exact form:
-// the hub sort (an unstable std::sort over vertices V-1..0, src/phase1/init.cpp:139-177) and the first-seed
-// scan (init.cpp:179-187).  Everything that touches the graph's arcs runs on the device.
+// Steps that decide ORDER-dependent results keep the reference's exact form: the hub sort (an unstable std::sort over
+// vertices V-1..0, src/phase1/init.cpp:139-177), on the host or begun on the device and finished here, and the
+// first-seed scan (init.cpp:179-187).  Everything that touches the graph's arcs runs on the device.
 #include <fcntl.h>
 #include <omp.h>
 #include <sys/stat.h>
@@ -502,7 +502,7 @@ int pinned_ring(dmolp_ctx *c) {
 // slots may still be.
 int upload_array(dmolp_ctx *c, void *dst, const void *src, size_t n) {
     cudaPointerAttributes at;
-    bool direct = n < 2 * kUpSlot || omp_in_parallel();
+    bool direct = n < kUpMin || omp_in_parallel();
     if (!direct) {
         if (cudaPointerGetAttributes(&at, src) != cudaSuccess) cudaGetLastError();
         else direct = at.type != cudaMemoryTypeUnregistered;

@@ -1,5 +1,5 @@
-// Phase 1 on the resident CSR, in two cooperative launches: the seeds, and the theta-limited multi-source BFS
-// growth with all its rounds.
+// Phase 1 on the resident CSR, in cooperative launches: the seeds, and the theta-limited multi-source BFS growth with
+// all its rounds.
 //
 //   seeds   per seed, its radius-2 ball (compute_bfs with MAX_LEVELS = 3, src/phase1/seed.cpp:20-101) is OR-ed
 //           into a coverage byte map: level 1 = the seed's row, level 2 = the rows of level 1; then the first
@@ -15,8 +15,10 @@
 // there are 20 to 80 rounds.  With a host check and seven launches per round a round cost 65 us on a 5 K-vertex
 // mesh and 160 us on a skewed graph of a million vertices; here it is two grid barriers (claims | labels), a third
 // when rows of more than kP1Piece arcs are split, and the select's only in rounds where a part has more than
-// theta frontier vertices: 12 and 70 us a round.  Whole phase 1 (hub list on the host included): 1.9 -> 0.6 ms on the
-// mesh, 8.9 -> 6.2 ms on the skewed graph.
+// theta frontier vertices: 12 and 70 us a round.  Seeds and growth: 1.8 -> 0.5 ms on the mesh, 5.6 -> 2.2 ms on the
+// skewed graph.
+//
+// Large graphs with few hubs get their hub list here, too (k_hub_stats, k_hub_top).
 #include <algorithm>
 #include <climits>
 
