@@ -1018,6 +1018,7 @@ static int find_seeds_impl(dmolp_ctx *c, int k, int first, const std::vector<int
     if (hubs.empty() || k <= 1) return DMOLP_OK;
     DMOLP_CUDA(cudaMemcpyAsync(b.hubs, hubs.data(), hubs.size() * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
     DMOLP_CUDA(cudaMemsetAsync(b.covered, 0, (size_t)nv, c->stream));
+    if (!c->rows_sorted) DMOLP_CUDA(cudaMemsetAsync(b.claim, 0, (size_t)nv * sizeof(int32_t), c->stream));
     DMOLP_CUDA(cudaMemsetAsync(b.best, 0, 2 * sizeof(unsigned long long), c->stream));
     DMOLP_CUDA(cudaMemsetAsync(b.p1cnt, 0, 8 * sizeof(int), c->stream));
     p1_find_seeds(c, k, first, (int64_t)hubs.size());

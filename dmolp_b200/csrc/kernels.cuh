@@ -94,7 +94,7 @@ void p1_hub_stats(dmolp_ctx *c);
 // *b.hubst.
 void p1_hub_top(dmolp_ctx *c, int64_t t0, int depth);
 // Seeds by the reference rule from b.hubs[0, nhubs) and the first seed: b.need[0, found), found = p1cnt[6].
-// b.covered, b.best and p1cnt are cleared by the caller.
+// b.covered, b.best, p1cnt and, unless the rows are strictly increasing, b.claim are cleared by the caller.
 void p1_find_seeds(dmolp_ctx *c, int k, int first, int64_t nhubs);
 // Every growth round from the seeds b.need[0, k): labels, part sizes, the number of rounds in p1cnt[5].
 void p1_grow(dmolp_ctx *c, int k, int theta);

@@ -37,7 +37,8 @@ enum { kFront = 0, kPieces = 2, kLabelled = 4, kRounds = 5, kFound = 6 };
 __device__ __forceinline__ int grid_warp() { return (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x; }
 __device__ __forceinline__ int grid_warps() { return (int)(blockDim.x >> 5) * (int)gridDim.x; }
 
-// Row [s, e) of vertex v queued in pieces of kP1Piece arcs.
+// Row [s, e) of vertex v queued in pieces of kP1Piece arcs.  The queue's narcs / 256 + 2 places are enough for every row
+// once (at least kP1Piece / 2 arcs a piece), so between two resets of the counter no row is queued twice.
 __device__ __forceinline__ void queue_row(const Buffers &b, int *ctr, int v, int64_t deg) {
     const int n = (int)((deg + kP1Piece - 1) / kP1Piece);
     const int q = atomicAdd(ctr, n);
@@ -48,8 +49,10 @@ __device__ __forceinline__ void cover_arcs(const Buffers &b, int64_t s, int64_t 
     warp_row(b.col, s, e, threadIdx.x & 31, [&](int x) { b.covered[x] = 1; }, [] { return false; });
 }
 
-// seeds[0, found) to b.need, found to p1cnt.  b.covered, b.best[2] and p1cnt are zero on entry.
-__global__ void __launch_bounds__(kSelThreads, 1) k_p1_find_seeds(Buffers b, int k, int first, int nhubs,
+// seeds[0, found) to b.need, found to p1cnt.  b.covered, b.best[2] and p1cnt are zero on entry.  repeats: rows may list
+// an id more than once (b.claim is then zero on entry); the first occurrence of a neighbour in the seed's row claims
+// its place in the queue, the others only count its arcs, as a walk of each occurrence would.
+__global__ void __launch_bounds__(kSelThreads, 1) k_p1_find_seeds(Buffers b, int k, int first, int nhubs, int repeats,
                                                                   unsigned int polls) {
     const int lane = threadIdx.x & 31;
     int seed = first, found = 1;
@@ -72,7 +75,8 @@ __global__ void __launch_bounds__(kSelThreads, 1) k_p1_find_seeds(Buffers b, int
                     us = b.off[u];
                     ue = b.off[u + 1];
                     te += (unsigned long long)(ue - us);
-                    if (ue - us > kP1Piece) queue_row(b, npiece, u, ue - us);
+                    if (ue - us > kP1Piece && (!repeats || atomicExch(&b.claim[u], p) != p))
+                        queue_row(b, npiece, u, ue - us);
                 }
             }
             const int64_t deg = ue - us;
@@ -639,7 +643,7 @@ void p1_hub_top(dmolp_ctx *c, int64_t t0, int depth) {
 }
 
 void p1_find_seeds(dmolp_ctx *c, int k, int first, int64_t nhubs) {
-    launch_resident(c, k_p1_find_seeds, 0, c->b, k, first, (int)nhubs, c->wait_polls);
+    launch_resident(c, k_p1_find_seeds, 0, c->b, k, first, (int)nhubs, c->rows_sorted ? 0 : 1, c->wait_polls);
 }
 
 void p1_grow(dmolp_ctx *c, int k, int theta) {
