@@ -1302,8 +1302,11 @@ int dmolp_lp_run(dmolp_ctx *c, int k, const dmolp_lp_config *cfg, dmolp_lp_resul
     c->counts_kept = c->symmetric && L.eff <= 32;
     const bool loop = use_loop(c, max_iter);
     if (loop) {
+        // The slot orders count as built once a call with them has ended without an error: a launch of theirs that
+        // failed is reported here, one that gave up ends the loop's at its start.
         if (!c->loop_ordered) loop_order(c);
-        c->loop_ordered = true;
+        if (c->launch_error != cudaSuccess) return report_waits(c, 0);
+        c->loop_ordered = false;
         lp_reset_stats(c, k, nullptr);
         lp_stats(c, k, nullptr, nullptr, false, c->counts_kept ? L.eff : 0, L.eff);
         loop_run(c, L, max_iter);
@@ -1362,6 +1365,7 @@ int dmolp_lp_run(dmolp_ctx *c, int k, const dmolp_lp_config *cfg, dmolp_lp_resul
     const LpRecordDev *recs = host_of(c, b.rec);
     st = report_waits(c, ctl.wait_timeout);
     if (st) return st;
+    if (loop) c->loop_ordered = true;
     if (ctl.error) return fail(DMOLP_ERR_BAD_LABELS, "label outside [0,k) or odd cut-arc count");
     float ms = 0;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);

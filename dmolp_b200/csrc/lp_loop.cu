@@ -302,6 +302,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1) k_lp_loop(Buffers b, LoopArgs
     const unsigned below = (1u << lane) - 1;
     int *const s_my = s_w + w * k;
     LpControl *const ctl = b.ctrl;
+    // The slot orders' launch of the same call gave up at one of its barriers: the orders hold no ids of this graph.
+    if (*(volatile int *)&ctl->wait_timeout) return;
 
     // ---- start (the statistics pass has run) ----
     long long prev_cut = 0;
