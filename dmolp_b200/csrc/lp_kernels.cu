@@ -1307,9 +1307,9 @@ __device__ void lp_end(const Buffers &b, int k, int t, long long narcs, int mode
 // them, then out to global).
 __device__ __forceinline__ void lp_turn(const Buffers &b, int k, int t_end, int t_begin, long long narcs, int mode,
                                         int symmetric) {
-    __shared__ int s_stopped;
+    __shared__ int s_stopped, s_ended;  // before the end of t_end, and after it
     __shared__ double s_re[DMOLP_MAX_K], s_tp[DMOLP_MAX_K];
-    if (threadIdx.x == 0) s_stopped = b.ctrl->stopped;
+    if (threadIdx.x == 0) s_stopped = s_ended = b.ctrl->stopped;
     __syncthreads();
     if (s_stopped) return;
     if (t_begin > 0 && (threadIdx.x >> 5) == 1)
@@ -1317,10 +1317,10 @@ __device__ __forceinline__ void lp_turn(const Buffers &b, int k, int t_end, int 
                        b.logtab[t_begin], s_re, s_tp, b.penhist + (size_t)(t_begin - 1) * DMOLP_MAX_K);
     if (t_end > 0) {
         lp_end(b, k, t_end, narcs, mode, symmetric);
-        if (threadIdx.x == 0) s_stopped = b.ctrl->stopped;
+        if (threadIdx.x == 0) s_ended = b.ctrl->stopped;
     }
     __syncthreads();
-    if (s_stopped || t_begin <= 0) return;
+    if (s_ended || t_begin <= 0) return;
     lp_begin(b, k, t_begin, narcs);
     for (int p = threadIdx.x; p < k; p += blockDim.x) {
         b.RE[p] = s_re[p];
