@@ -663,8 +663,11 @@ void agg_fwd(const batch::View &b, __nv_bfloat16 *buf, int C) {
 
 void agg_bwd(const batch::View &b, const float *dC, const __nv_bfloat16 *Hbuf, int ldh, __nv_bfloat16 *G, float *db) {
     const int nv = (int)b.nv;
-    const size_t smem = b.nlong > 0 ? 2 * kLongTile * 16 * sizeof(uint4) : 0;
-    cudaFuncSetAttribute(k_agg_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // The limit is the kernel's, not the launch's: the same value in every call, or a thread whose batch has no long
+    // rows could lower it between another's setting and its launch.
+    constexpr size_t kTiles = 2 * kLongTile * 16 * sizeof(uint4);
+    cudaFuncSetAttribute(k_agg_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTiles);
+    const size_t smem = b.nlong > 0 ? kTiles : 0;
     k_agg_bwd<<<b.nlong + grid_for((int64_t)nv * 32, b.num_sms), 256, smem, b.stream>>>(b.off, b.col, nv, b.longrow,
                                                                                        b.nlong, dC, Hbuf, ldh, G, db);
 }
