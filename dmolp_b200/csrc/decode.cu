@@ -6,10 +6,11 @@
 // axis.  The axis: mean and covariance of the part in double, cyclic Jacobi on the 8x8 covariance, the
 // eigenvector of the largest eigenvalue signed so that its largest-magnitude component is positive.
 //
-// A part's vertices stay contiguous in a permutation (ascending ids), so each warp owns a run of it and keeps
-// the part's sums in registers; only where a run ends or crosses into the next part do they go to a record in
-// shared memory, and one warp per part adds those records in order.  All sums have a fixed order, so the result
-// does not depend on scheduling.  The selection is an MSD radix select over keys (orderable float bits of the
+// A part's vertices stay contiguous in a permutation (ascending ids), cut into segments whose length depends on the
+// part's size alone (segment_length).  A warp sums a segment at a time in registers, to the segment's record in global
+// memory, and one warp per part adds the records in order.  So the sums' order, and with it the result, depends neither
+// on scheduling nor on the team, that is on what else is in the batch.  (Sums over whatever vertices a warp held did:
+// the team's size moved the last bits of mean and axis.)  The selection is an MSD radix select over keys (orderable float bits of the
 // projection, id) with 6-bit digits and no lists: a record is open while its leading digits are its part's
 // prefix.  A stable partition of the permutation by the part's threshold key then forms the children.
 //
@@ -36,18 +37,22 @@ constexpr int kWarps = kDecThreads / 32;
 constexpr int kParts = batch::kBatchMaxK;
 constexpr int kDims = 8;
 constexpr int kTri = kDims * (kDims + 1) / 2;
-constexpr int kRun = 128;             // granularity of the warps' runs, in vertices
+constexpr int kSeg = 512;      // vertices of a segment of a small part; multiples of it in parts of more than ...
+constexpr int kMaxSegs = 256;  // ... this many such (one per warp of the largest team)
 constexpr int kRecs = kWarps + kParts;  // a CTA's warps meet at most this many (warp, part) pairs
+static_assert(kSeg == kDecSeg && kTri == kDecRecord && kParts / 2 == kDecSplits, "the records' workspace");
+
+// Vertices per segment of a part of n.
+__device__ __forceinline__ int segment_length(int n) { return ((n - 1) / (kSeg * kMaxSegs) + 1) * kSeg; }
 
 struct DecSmem {
-    double rec[kRecs][kTri];  // sums of this CTA's warps per (warp, part): index warp + the part's ordinal
     double mean[kParts][kDims], axis[kParts][kDims];
     double A[kWarps][kDims][kDims], V[kWarps][kDims][kDims];  // eigen-decomposition, a matrix per warp
     uint64_t prefix[kParts], cut[kParts];  // selection: digits fixed so far; keys below cut are selected
     int hist[2][kParts * kDigits];         // zero between selections
     int lrec[kRecs];                       // selected vertices per (warp, part)
     int kp[kParts], beg[kParts], cnt[kParts], need[kParts], below[kParts], keep[kParts], fin[kParts];
-    int part[kParts], run0[kParts + 1];  // splitting parts by ordinal, and their first runs
+    int part[kParts], len[kParts], seg0[kParts + 1];  // splitting parts by ordinal, segment lengths, first segments
     int nsplit, bad, inst;
 };
 
@@ -97,45 +102,72 @@ __device__ void jacobi8(double (*A)[kDims], double (*V)[kDims]) {
     __syncwarp();
 }
 
-// A warp's share of a level: the runs [a, b) of the splitting parts, whose runs follow each other by ordinal.
+// A warp's share of a level: the segments [a, b) of the splitting parts, whose segments follow each other by ordinal.
 // f(ordinal, first position, last position) for each part it meets, positions in the permutation.
 template <typename F>
 __device__ __forceinline__ void for_parts(const DecSmem &sm, int a, int b, F f) {
     int o = 0;
-    while (o < sm.nsplit && sm.run0[o + 1] <= a) ++o;
+    while (o < sm.nsplit && sm.seg0[o + 1] <= a) ++o;
     for (; a < b; ++o) {
-        const int p = sm.part[o], r0 = sm.run0[o];
-        const int z = b < sm.run0[o + 1] ? b : sm.run0[o + 1];
-        const int i0 = sm.beg[p] + (a - r0) * kRun;
-        const int i1 = z == sm.run0[o + 1] ? sm.beg[p] + sm.cnt[p] : sm.beg[p] + (z - r0) * kRun;
-        f(o, i0, i1);
+        const int p = sm.part[o], s0 = sm.seg0[o], end = sm.beg[p] + sm.cnt[p];
+        const int z = b < sm.seg0[o + 1] ? b : sm.seg0[o + 1];
+        const int i0 = sm.beg[p] + (a - s0) * sm.len[o];
+        f(o, i0, z == sm.seg0[o + 1] ? end : sm.beg[p] + (z - s0) * sm.len[o]);
         a = z;
     }
 }
 
-// The sums of ordinal o over the team's records of width n <= kTri, in run order, to lanes: lane l returns
-// entries l and l + 32.
-template <typename Tm>
-__device__ __forceinline__ double2 add_records(const Tm &tm, DecSmem &sm, int o, int per, int n) {
+// The same segment by segment: f(ordinal, segment, first position, last position).
+template <typename F>
+__device__ __forceinline__ void for_segments(const DecSmem &sm, int a, int b, F f) {
+    int o = 0;
+    for (; a < b; ++a) {
+        while (sm.seg0[o + 1] <= a) ++o;
+        const int p = sm.part[o], end = sm.beg[p] + sm.cnt[p];
+        const int i0 = sm.beg[p] + (a - sm.seg0[o]) * sm.len[o];
+        f(o, a, i0, end - i0 < sm.len[o] ? end : i0 + sm.len[o]);
+    }
+}
+
+// Sums over the warp's lanes of N values each (a power of two): lane l returns the sum of x[l % N].  Halves of the
+// values are exchanged, so N - 1 shuffles do what 5 N would; the tree of additions is that of the butterfly.
+template <int N>
+__device__ __forceinline__ double lane_sums(double *x) {
     const int lane = threadIdx.x & 31;
-    const int w0 = sm.run0[o] / per, w1 = (sm.run0[o + 1] - 1) / per;
-    double2 s = make_double2(0.0, 0.0);
-    for (int w = w0; w <= w1; w += 8) {  // eight records in flight
+#pragma unroll
+    for (int w = N / 2; w > 0; w >>= 1) {
+        const bool up = lane & w;
+#pragma unroll
+        for (int i = 0; i < w; ++i) {
+            const double give = up ? x[i] : x[i + w], keep = up ? x[i + w] : x[i];
+            x[i] = keep + __shfl_xor_sync(DMOLP_FULL_MASK, give, w);
+        }
+    }
+#pragma unroll
+    for (int o = N; o < 32; o <<= 1) x[0] += __shfl_xor_sync(DMOLP_FULL_MASK, x[0], o);
+    return x[0];
+}
+
+// The sums of the records of the segments [s, e), of width n <= kTri, in order, to lanes: lane l returns entries l and
+// l + 32.  Written by other CTAs: read past L1.
+__device__ __forceinline__ double2 add_records(const double *rec, int s, int e, int n) {
+    const int lane = threadIdx.x & 31;
+    double2 t = make_double2(0.0, 0.0);
+    for (; s < e; s += 8) {  // eight records in flight
         double x[8], y[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const bool in = w + q <= w1;
-            const double *r = tm.at(&sm.rec[(in ? (w + q) % kWarps : 0) + (in ? o : 0)][0], in ? (w + q) / kWarps : 0);
-            x[q] = in && lane < n ? r[lane] : 0.0;
-            y[q] = in && lane + 32 < n ? r[lane + 32] : 0.0;
+            const double *r = rec + (size_t)(s + q) * kTri + lane;
+            x[q] = s + q < e && lane < n ? __ldcg(r) : 0.0;
+            y[q] = s + q < e && lane + 32 < n ? __ldcg(r + 32) : 0.0;
         }
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            s.x += x[q];
-            s.y += y[q];
+            t.x += x[q];
+            t.y += y[q];
         }
     }
-    return s;
+    return t;
 }
 
 template <typename Tm>
@@ -147,6 +179,7 @@ __device__ void run_decode(const DecodeWork &w, int ii, const Tm &tm, DecSmem &s
     const int wid = tm.rank_of() * kWarps + wib;  // a CTA's warps are consecutive here
     int32_t *perm[2] = {w.l0 + vb, w.l1 + vb};
     uint64_t *const key = w.key + vb;  // by position in the permutation
+    double *const rec = w.rec + decode_record(vb, ii) * kTri;
     const float *const Z = w.Z + (size_t)vb * 16;
     const int bits = 32 + I.ibits, npass = (bits + kDigitBits - 1) / kDigitBits, top = npass * kDigitBits;
     auto coords = [&](int v, float (&x)[kDims]) {
@@ -182,14 +215,14 @@ __device__ void run_decode(const DecodeWork &w, int ii, const Tm &tm, DecSmem &s
     }
     int cur = 0;
     for (int level = 0; level < 7; ++level, cur ^= 1) {
-        // ---- the splitting parts and their runs (by every CTA alike) ----
+        // ---- the splitting parts and their segments (by every CTA alike) ----
         __syncthreads();
         if (wib == 0) {
-            int nsplit = 0, runs = 0;
+            int nsplit = 0, segs = 0;
             for (int p0 = 0; p0 < kParts; p0 += 32) {
                 const int p = p0 + lane;
                 const bool split = sm.kp[p] >= 2 && sm.cnt[p] > 0;
-                const int r = split ? (sm.cnt[p] + kRun - 1) / kRun : 0;
+                const int len = split ? segment_length(sm.cnt[p]) : 1, r = split ? (sm.cnt[p] - 1) / len + 1 : 0;
                 int incl = r;
                 for (int o = 1; o < 32; o <<= 1) {
                     const int y = __shfl_up_sync(DMOLP_FULL_MASK, incl, o);
@@ -199,14 +232,15 @@ __device__ void run_decode(const DecodeWork &w, int ii, const Tm &tm, DecSmem &s
                 if (split) {
                     const int o = nsplit + __popc(m & ((1u << lane) - 1));
                     sm.part[o] = p;
-                    sm.run0[o] = runs + incl - r;
+                    sm.len[o] = len;
+                    sm.seg0[o] = segs + incl - r;
                 }
                 nsplit += __popc(m);
-                runs += __shfl_sync(DMOLP_FULL_MASK, incl, 31);
+                segs += __shfl_sync(DMOLP_FULL_MASK, incl, 31);
             }
             if (lane == 0) {
                 sm.nsplit = nsplit;
-                sm.run0[nsplit] = runs;
+                sm.seg0[nsplit] = segs;
             }
         }
         for (int p = threadIdx.x; p < kParts; p += kDecThreads) {
@@ -220,12 +254,12 @@ __device__ void run_decode(const DecodeWork &w, int ii, const Tm &tm, DecSmem &s
         any = __any_sync(DMOLP_FULL_MASK, any);
         __syncthreads();
         if (!any) break;
-        const int nsplit = sm.nsplit, runs = sm.run0[nsplit];
-        const int per = runs > 0 ? (runs + team_warps - 1) / team_warps : 1;
-        const int a = min(wid * per, runs), b = min(a + per, runs);
+        const int nsplit = sm.nsplit, segs = sm.seg0[nsplit];
+        const int per = segs > 0 ? (segs + team_warps - 1) / team_warps : 1;
+        const int a = min(wid * per, segs), b = min(a + per, segs);
         const int32_t *const pm = perm[cur];
         // ---- means ----
-        for_parts(sm, a, b, [&](int o, int i0, int i1) {
+        for_segments(sm, a, b, [&](int, int seg, int i0, int i1) {
             double acc[kDims];
 #pragma unroll
             for (int d = 0; d < kDims; ++d) acc[d] = 0.0;
@@ -235,21 +269,18 @@ __device__ void run_decode(const DecodeWork &w, int ii, const Tm &tm, DecSmem &s
 #pragma unroll
                 for (int d = 0; d < kDims; ++d) acc[d] += (double)x[d];
             }
-#pragma unroll
-            for (int d = 0; d < kDims; ++d) {
-                for (int s = 16; s > 0; s >>= 1) acc[d] += __shfl_xor_sync(DMOLP_FULL_MASK, acc[d], s);
-                if (lane == d) sm.rec[wib + o][d] = acc[d];
-            }
+            const double t = lane_sums<kDims>(acc);
+            if (lane < kDims) rec[(size_t)seg * kTri + lane] = t;
         });
         tm.sync();
         for (int o = tm.warp(); o < nsplit; o += team_warps) {
-            const double s = add_records(tm, sm, o, per, kDims).x / (double)sm.cnt[sm.part[o]];
+            const double s = add_records(rec, sm.seg0[o], sm.seg0[o + 1], kDims).x / (double)sm.cnt[sm.part[o]];
             if (lane < kDims)
                 for (int r = 0; r < tm.size(); ++r) *tm.at(&sm.mean[o][lane], r) = s;
         }
         tm.sync();
         // ---- covariances (upper triangles), principal axes ----
-        for_parts(sm, a, b, [&](int o, int i0, int i1) {
+        for_segments(sm, a, b, [&](int o, int seg, int i0, int i1) {
             double acc[kTri], mu[kDims];
 #pragma unroll
             for (int i = 0; i < kTri; ++i) acc[i] = 0.0;
@@ -267,15 +298,13 @@ __device__ void run_decode(const DecodeWork &w, int ii, const Tm &tm, DecSmem &s
 #pragma unroll
                     for (int e = c; e < kDims; ++e) acc[q++] += x[c] * x[e];
             }
-#pragma unroll
-            for (int q = 0; q < kTri; ++q) {
-                for (int s = 16; s > 0; s >>= 1) acc[q] += __shfl_xor_sync(DMOLP_FULL_MASK, acc[q], s);
-                if (lane == (q & 31)) sm.rec[wib + o][q] = acc[q];
-            }
+            const double t0 = lane_sums<32>(acc), t1 = lane_sums<kTri - 32>(acc + 32);
+            rec[(size_t)seg * kTri + lane] = t0;
+            if (lane < kTri - 32) rec[(size_t)seg * kTri + 32 + lane] = t1;
         });
         tm.sync();
         for (int o = tm.warp(); o < nsplit; o += team_warps) {
-            const double2 s = add_records(tm, sm, o, per, kTri);
+            const double2 s = add_records(rec, sm.seg0[o], sm.seg0[o + 1], kTri);
             double(*A)[kDims] = sm.A[wib], (*V)[kDims] = sm.V[wib];
             int q = 0;
             for (int c = 0; c < kDims; ++c)
@@ -359,9 +388,9 @@ __device__ void run_decode(const DecodeWork &w, int ii, const Tm &tm, DecSmem &s
         for_parts(sm, a, b, [&](int o, int i0, int i1) {
             const int p = sm.part[o], kl = sm.kp[p] / 2, kr = sm.kp[p] - kl;
             const uint64_t cut = sm.cut[p];
-            // selected vertices of the part in front of this run: its earlier warps' records
+            // selected vertices of the part in front of this share: its earlier warps' counts
             int left = 0;
-            for (int x = sm.run0[o] / per + lane; x < wid; x += 32)
+            for (int x = sm.seg0[o] / per + lane; x < wid; x += 32)
                 left += *tm.at(&sm.lrec[x % kWarps + o], x / kWarps);
             left = __reduce_add_sync(DMOLP_FULL_MASK, left);
             const int nl = (int)(((long long)sm.cnt[p] * kl) / sm.kp[p]);
@@ -378,7 +407,7 @@ __device__ void run_decode(const DecodeWork &w, int ii, const Tm &tm, DecSmem &s
                 left += __popc(m);
             }
         });
-        tm.sync();  // records and tables are read before they change; the new order is complete
+        tm.sync();  // counts and tables are read before they change; the new order is complete
         if (wib == 0) {  // a child p + kl never falls on a part that still splits: its labels are [p, p + kp)
             int kp[2], beg[2], cnt[2];
 #pragma unroll

@@ -69,6 +69,7 @@ struct dmolp_mpnn {
     int32_t *anchor = nullptr, *ecc = nullptr, *status = nullptr, *target = nullptr, *dl0 = nullptr, *dl1 = nullptr;
     int32_t *dorder = nullptr;  // [ninst] graphs of a decoder call, largest first
     uint64_t *key = nullptr;
+    double *rec = nullptr;
     int *next = nullptr;
     float *P0 = nullptr, *Q0 = nullptr, *P1 = nullptr, *Q1 = nullptr;
     double *stats = nullptr, *gscore = nullptr;
@@ -115,6 +116,7 @@ int ensure_ws(dmolp_mpnn *m, const batch::View &b, bool train) {
     MTRY(alloc_into(o, &m->Xf, n * 16));
     MTRY(alloc_into(o, &m->Pc, n * 16));
     MTRY(alloc_into(o, &m->key, n));
+    MTRY(alloc_into(o, &m->rec, decode_record(b.nv, b.ninst) * kDecRecord));
     MTRY(alloc_into(o, &m->G3, n * 16));
     MTRY(alloc_into(o, &m->vinst, n));
     MTRY(alloc_into(o, &m->dl0, n));
@@ -459,6 +461,7 @@ static int decode_impl(dmolp_mpnn *m, dmolp_batch *b, const float *embedding, co
         w.inst = v.inst;
         w.Z = m->Pc;
         w.key = m->key;
+        w.rec = m->rec;
         w.label = v.label;
         w.l0 = m->dl0;
         w.l1 = m->dl1;
