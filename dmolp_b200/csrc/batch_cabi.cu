@@ -109,7 +109,8 @@ int run_graph(dmolp_batch *b, const dmolp_batch_tuning &t, const dmolp_lp_config
     if (occ <= 0) return fail(DMOLP_ERR_ARG, "unsupported launch shape");
     const int bps = t.blocks_per_sm <= 0 ? occ : std::min(t.blocks_per_sm, occ);
     const int grid = std::max(1, std::min(b->ninst, b->num_sms * bps));
-    const auto key = std::make_tuple(t.block_threads, t.thread_row_max, grid, (int)cfg.mode, (int)cfg.iterations,
+    // (the residency, not the grid that it is clamped to: the teams' sizes follow from it, too)
+    const auto key = std::make_tuple(t.block_threads, t.thread_row_max, bps, (int)cfg.mode, (int)cfg.iterations,
                                      (int)cfg.cap);
     auto it = b->graphs.find(key);
     if (it == b->graphs.end()) {
