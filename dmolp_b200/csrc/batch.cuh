@@ -42,7 +42,7 @@ struct Args {
     int32_t *ndiff;  // neighbours with another label, exact at every iteration start
     int32_t *l_bnd, *l_win0, *l_win1;  // per-instance slices at vbase
     uint64_t *rec0, *rec1;             // selection records, per-instance slices at vbase
-    uint16_t *cnt;                     // kept label counts, per-instance slices at cbase
+    uint16_t *cnt;                     // kept label counts, per-instance slices at cbase (null: no graph has any)
     const Inst *inst;
     const int32_t *order;
     int ninst;

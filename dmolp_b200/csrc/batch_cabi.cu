@@ -29,6 +29,8 @@ struct dmolp_batch {
     int64_t nv = 0, narcs = 0;
     std::vector<void *> allocations;
     Args a{};
+    int64_t ncnt = 0;           // 16-bit label counts of the graphs that can keep them
+    bool counts_ready = false;  // allocated, or given up, by a phase 2 of the resident batch
     Inst *inst = nullptr;
     int32_t *order = nullptr, *saved = nullptr, *longrow = nullptr;
     int nlong = 0;
@@ -87,6 +89,8 @@ void free_all(dmolp_batch *b) {
     for (void *p : b->allocations) cudaFree(p);
     b->allocations.clear();
     b->a = Args();
+    b->ncnt = 0;
+    b->counts_ready = false;
     b->has_graph = false;
     b->tuned = false;
 }
@@ -102,6 +106,24 @@ int bsync(dmolp_batch *b) {
         int r_ = (x);        \
         if (r_) return r_;   \
     } while (0)
+
+// The kept label counts (up to 64 bytes per vertex), allocated by the first phase 2 of a batch: nothing else needs
+// them.  Without the memory no graph keeps counts, and its decisions count the rows, to the same result.
+int ensure_counts(dmolp_batch *b) {
+    if (b->counts_ready) return DMOLP_OK;
+    if (b->ncnt > 0) {
+        const int st = balloc(b, &b->a.cnt, (size_t)b->ncnt);
+        if (st && st != DMOLP_ERR_NOMEM) return st;
+        if (st) {
+            for (Inst &I : b->h_inst) I.cstride = 0;
+            BCUDA(cudaMemcpyAsync(b->inst, b->h_inst.data(), b->h_inst.size() * sizeof(Inst), cudaMemcpyHostToDevice,
+                                  b->stream));
+            BCUDA(cudaStreamSynchronize(b->stream));
+        }
+    }
+    b->counts_ready = true;
+    return DMOLP_OK;
+}
 
 // Capture (once per shape and configuration) and launch the batch.
 int run_graph(dmolp_batch *b, const dmolp_batch_tuning &t, const dmolp_lp_config &cfg) {
@@ -290,7 +312,6 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
             *col = nullptr, *order = nullptr, *saved = nullptr;
     int64_t *off = nullptr;
     uint64_t *rec0 = nullptr, *rec1 = nullptr;
-    uint16_t *cnt = nullptr;
     Inst *inst = nullptr;
     Out *out = nullptr;
     long long *counts = nullptr;
@@ -370,8 +391,8 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
         return fail(DMOLP_ERR_ARG, "instance " + std::to_string(h_err - 1) + ": neighbour id outside its graph");
     }
     BCUDA(cudaMemcpy(hi.data(), inst, ninst * sizeof(Inst), cudaMemcpyDeviceToHost));
-    // key widths, and a slice of kept label counts for every graph whose decisions can use them: symmetric,
-    // degrees in 16 bits
+    // key widths, and a slice of kept label counts (ensure_counts) for every graph whose decisions can use them:
+    // symmetric, degrees in 16 bits
     int64_t ncnt = 0;
     for (Inst &I : hi) {
         int ib = 1, db = 1;
@@ -383,7 +404,6 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
         I.cstride = I.symmetric && I.maxdeg < 65536 ? (std::min(I.k, 32) + 7) & ~7 : 0;
         ncnt += (int64_t)I.cstride * I.nv;
     }
-    BTRY(balloc(b, &cnt, ncnt));
     BCUDA(cudaMemcpy(inst, hi.data(), ninst * sizeof(Inst), cudaMemcpyHostToDevice));
     a.off = off;
     a.col = col;
@@ -396,7 +416,8 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
     a.l_win1 = w1;
     a.rec0 = rec0;
     a.rec1 = rec1;
-    a.cnt = cnt;
+    a.cnt = nullptr;
+    b->ncnt = ncnt;
     a.inst = inst;
     a.order = order;
     a.ninst = ninst;
@@ -495,6 +516,7 @@ int dmolp_batch_lp_run(dmolp_batch *b, const dmolp_lp_config *cfg, const dmolp_b
     BTRY(check_cfg(cfg));
     BCUDA(cudaSetDevice(b->device));
     const dmolp_batch_tuning t = tune ? *tune : b->tuning;
+    BTRY(ensure_counts(b));
     BCUDA(cudaEventRecord(b->ev0, b->stream));
     BTRY(run_graph(b, t, *cfg));
     BCUDA(cudaEventRecord(b->ev1, b->stream));
