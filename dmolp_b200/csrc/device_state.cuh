@@ -204,6 +204,7 @@ struct dmolp_ctx {
     unsigned int wait_polls = dmolp::kDefaultWaitPolls;  // polls of a grid barrier before it gives up
     int nhot = 0;                         // hot vertices
     bool loop_ordered = false;            // lpasc / lpdesc are built for the resident graph
+    bool lp_steps = false;                // never take the one-launch loop (dmolp_set_lp_steps)
     int lp_runs = 0;                      // dmolp_lp_run calls on the resident graph
     std::vector<int32_t> h_rawdeg;        // host copy for the hub sort
     bool h_rawdeg_valid = false;          // h_rawdeg mirrors the resident raw degrees

@@ -971,6 +971,12 @@ int dmolp_set_symmetry_test(dmolp_ctx *c, int exact) {
     return DMOLP_OK;
 }
 
+int dmolp_set_lp_steps(dmolp_ctx *c, int on) {
+    if (!c) return fail(DMOLP_ERR_ARG, "null context");
+    c->lp_steps = on != 0;
+    return DMOLP_OK;
+}
+
 int dmolp_set_profiling(dmolp_ctx *c, int enable) {
     if (!c) return fail(DMOLP_ERR_ARG, "null context");
     c->profiling = enable != 0;
@@ -1273,9 +1279,10 @@ int dmolp_phase1(dmolp_ctx *c, int k, int theta, int32_t *seeds_out, int64_t *ve
 // 2.83 -> 1.91 ms; a skewed graph of 7.5 M arcs, 64 parts 1.36 -> 1.10 ms.  Above it the launch per step wins, with
 // its pulled candidates and hub windows instead of a stamp per arc (a skewed graph of 14 M arcs 1.29 ms, here 1.76).
 // A run of fewer than kLoopMinIters iterations does not earn the slot orders (40 us).  Asymmetric graphs recount from
-// the arcs each iteration, and timed launches (profiling) are those of the launch per step.
+// the arcs each iteration, and timed launches (profiling) are those of the launch per step, which a caller can also ask
+// for (dmolp_set_lp_steps).
 static bool use_loop(const dmolp_ctx *c, int iters) {
-    return c->symmetric && !c->profiling && c->narcs > 0 && c->narcs <= kLoopMaxArcs && iters >= kLoopMinIters;
+    return c->symmetric && !c->profiling && !c->lp_steps && c->narcs > 0 && c->narcs <= kLoopMaxArcs && iters >= kLoopMinIters;
 }
 
 int dmolp_lp_run(dmolp_ctx *c, int k, const dmolp_lp_config *cfg, dmolp_lp_result *res, dmolp_lp_record *records,

@@ -183,6 +183,11 @@ class Partitioner:
         """exact=False (default): keyed multiset sums in one pass; exact=True: every reverse arc looked up."""
         self._check(self.lib.dmolp_set_symmetry_test(self.ctx, 1 if exact else 0))
 
+    def set_lp_steps(self, on: bool) -> None:
+        """on=False (default): small symmetric graphs run phase 2's iterations in one launch; on=True: a launch per
+        step, as large ones do.  The results are the same."""
+        self._check(self.lib.dmolp_set_lp_steps(self.ctx, 1 if on else 0))
+
     def kernel_launches(self) -> int:
         return int(self.lib.dmolp_kernel_launches(self.ctx))
 

@@ -219,7 +219,8 @@ int dmolp_labels_restore(dmolp_ctx *ctx);
  * CUDA events and accumulates their device time and algorithmic bytes (read with dmolp_kernel_profile).
  * kernel: 0 = boundary test, 1 = LP decisions, 2 = window marking, 3 = incremental cut/balance update,
  * 4 = per-label window selection (all radix-select launches of an iteration).
- * No reference counterpart. */
+ * The times are those of a launch per step: while timing is enabled, every run takes that form, also on graphs whose
+ * iterations otherwise run in one launch (dmolp_set_lp_steps).  No reference counterpart. */
 int dmolp_set_profiling(dmolp_ctx *ctx, int enable);
 int dmolp_kernel_profile(dmolp_ctx *ctx, int kernel, double *total_ms, int64_t *launches, double *bytes);
 
@@ -240,6 +241,11 @@ int dmolp_set_symmetry_test(dmolp_ctx *ctx, int exact);
 /* The test's answer for the resident graph (runs it now if the loop has not yet): 1 = symmetric with rows
  * strictly increasing (incremental statistics apply), else 0. */
 int dmolp_graph_symmetric(dmolp_ctx *ctx, int *symmetric);
+
+/* Which form phase 2's iterations take.  on = 0 (default): symmetric graphs of at most 8 M arcs run all their
+ * iterations in one cooperative launch, others in a launch per step.  on = 1: every run takes a launch per step.
+ * The results are the same, bit for bit; this is for comparing and testing the two forms. */
+int dmolp_set_lp_steps(dmolp_ctx *ctx, int on);
 
 /* ---- phase-1 hubs on the host (no device work) ----
  * dmolp_find_hubs_pairs: find_hub_nodes (src/phase1/init.cpp:139-177) on n (id, degree) pairs given in the
