@@ -75,6 +75,23 @@ __device__ __forceinline__ void block_atomic_add(unsigned long long v, T *dst) {
     }
 }
 
+// A block's arrival at a barrier of n blocks that are all resident, and its wait for the others; called by one thread
+// between block barriers of its block.  The scheme is that of the grid barrier of CUDA's cooperative groups, with a
+// bounded wait: one word, to which the leading block adds 2^31 - (n - 1) and every other one 1, so that the arrivals
+// together flip the top bit and leave the rest as it was; each block waits for the flip.  One atomic and the polls, no
+// reset.  The fences order the whole block's accesses: the block barriers around the call make them cumulative.
+// False when the wait ran past `polls` polls, or *gave_up was found set: another block's wait has ended that way.
+__device__ __forceinline__ bool arrive_and_wait(unsigned int *word, unsigned int n, bool leads, unsigned int polls,
+                                                const int *gave_up) {
+    __threadfence();
+    const unsigned int old = atomicAdd(word, leads ? 0x80000000u - (n - 1u) : 1u);
+    const volatile unsigned int *const w = word;
+    for (unsigned int i = 0; ((*w ^ old) & 0x80000000u) == 0u; ++i)
+        if (i >= polls || ((i & 63u) == 63u && *(const volatile int *)gave_up)) return false;
+    __threadfence();
+    return true;
+}
+
 // Read-only, streaming load of a neighbour id (bypasses L1 allocation; CSR is read once per pass).
 __device__ __forceinline__ int32_t ld_stream(const int32_t *p) { return __ldcs(p); }
 

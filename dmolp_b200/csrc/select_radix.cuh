@@ -52,11 +52,8 @@ struct SelArgs {
     unsigned int polls;  // grid barrier wait limit
 };
 
-// Grid barrier (all blocks are resident: cooperative launch) on one word: block 0 adds 2^31 - (blocks - 1), every
-// other block 1, so the arrivals together flip the top bit and leave the rest as it was; each block waits for the
-// flip.  One atomic and the polls, no reset (arrival count, its reset and a generation word took two more round trips
-// to L2).  Thread 0's fences order the whole block's accesses: the block barriers around them make them cumulative.
-// Returns false when the wait ran past `polls` polls, or another block's barrier already gave up: then
+// Grid barrier (all blocks are resident: cooperative launch) on one word, arrive_and_wait; an arrival count, its reset
+// and a generation word took two more round trips to L2.  Returns false when the wait ran past `polls` polls, or another block's barrier already gave up: then
 // ctl->wait_timeout holds 1 + the id of the first barrier that gave up, the loop is stopped, and the caller's
 // block leaves the kernel at once (every block that waits at a later barrier leaves too), so the kernel
 // always ends; the host reports the timeout and clears the barrier state.
@@ -64,20 +61,11 @@ __device__ __forceinline__ bool grid_sync(LpControl *ctl, unsigned int polls, in
     __shared__ int s_pass;
     __syncthreads();
     if (threadIdx.x == 0) {
-        int pass = 1;
-        volatile unsigned int *word = &ctl->bar_count;
-        volatile int *gave_up = &ctl->wait_timeout;
-        __threadfence();
-        const unsigned int old = atomicAdd(&ctl->bar_count, blockIdx.x == 0 ? 0x80000000u - (gridDim.x - 1u) : 1u);
-        for (unsigned int i = 0; ((*word ^ old) & 0x80000000u) == 0u; ++i) {
-            if (i >= polls || ((i & 63u) == 63u && *gave_up)) {
-                atomicCAS(&ctl->wait_timeout, 0, 1 + id);
-                atomicExch(&ctl->stopped, 1);  // the LP iteration's later kernels return at once
-                pass = 0;
-                break;
-            }
+        const bool pass = arrive_and_wait(&ctl->bar_count, gridDim.x, blockIdx.x == 0, polls, &ctl->wait_timeout);
+        if (!pass) {
+            atomicCAS(&ctl->wait_timeout, 0, 1 + id);
+            atomicExch(&ctl->stopped, 1);  // the LP iteration's later kernels return at once
         }
-        __threadfence();
         s_pass = pass;
     }
     __syncthreads();

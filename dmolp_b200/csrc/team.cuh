@@ -63,10 +63,9 @@ struct ClusterTeam {
 
 // Some of the CTAs of a cooperative launch (all resident), for graphs that are worth more CTAs than a cluster has.
 // They share no shared memory: the team's counters are one object in global memory, which first(p) leaves as it is,
-// and code for this team keeps nothing else per CTA in it.  sync() is a barrier on one word: the first CTA adds
-// 2^31 - (n - 1), every other CTA 1, so the arrivals flip the top bit and leave the rest; the fences of thread 0,
-// between barriers of the block, order the whole block's accesses.  It returns false when the wait gave up after
-// `polls` polls, or another CTA's did (*err is then set): the caller leaves the kernel at once.
+// and code for this team keeps nothing else per CTA in it.  sync() is a barrier on one word (arrive_and_wait).  It
+// returns false when the wait gave up after `polls` polls, or another CTA's did (*err is then set): the caller leaves
+// the kernel at once.
 template <int NT>
 struct GridTeam {
     unsigned int *word;
@@ -83,18 +82,8 @@ struct GridTeam {
         bool pass = true;
         __syncthreads();
         if (threadIdx.x == 0) {
-            __threadfence();
-            const unsigned int old = atomicAdd(word, rank == 0 ? 0x80000000u - ((unsigned int)n - 1u) : 1u);
-            volatile unsigned int *w = word;
-            volatile int *gave_up = err;
-            for (unsigned int i = 0; ((*w ^ old) & 0x80000000u) == 0u; ++i) {
-                if (i >= polls || ((i & 63u) == 63u && *gave_up)) {
-                    atomicExch(err, 1);
-                    pass = false;
-                    break;
-                }
-            }
-            __threadfence();
+            pass = arrive_and_wait(word, (unsigned int)n, rank == 0, polls, err);
+            if (!pass) atomicExch(err, 1);
         }
         return __syncthreads_and(pass);
     }
