@@ -33,7 +33,7 @@ constexpr int kLoopMinIters = 4;
 constexpr size_t kLoopCntBytes = 256;
 inline size_t loop_pieces(int64_t narcs) { return (size_t)narcs / kLoopShort + 2; }
 
-// Polls of a grid-barrier generation word before the barrier gives up (about a second on B200).
+// Polls of a grid barrier's word before the barrier gives up (about a second on B200).
 constexpr unsigned int kDefaultWaitPolls = 1u << 22;
 
 // Per-iteration counters of the LP loop (reset by the first kernel of each iteration).
@@ -41,7 +41,6 @@ struct LpCounters {
     int ncand;        // candidates this iteration (t >= 2)
     int nbnd;         // boundary candidates (selection records)
     int nwin[2];      // window (selected set) sizes, double-buffered by iteration parity
-    int nactive[2];   // radix-select active lists
     int napply, apply_iter;  // movers of the iteration whose labels are due, and that iteration (k_update)
     int nchanged;     // selected vertices whose label changed (movers)
     int ndec[3];      // selected vertices per decision class
@@ -66,7 +65,6 @@ struct LpControl {
     int error;          // 1 = odd cut-arc count or invalid label (the reference aborts)
     int mode;           // DMOLP_LP_MODE_*
     int pull;           // next iteration finds candidates by pulling (rows scanned for a window member)
-    int sel_open[2];    // radix select: segments still needing records after a pass (by pass parity)
     unsigned int bar_count;  // grid barrier of the cooperative kernels
     int wait_timeout;   // a grid barrier gave up waiting (1 + the barrier's index in the kernel)
     int sel_tail;       // radix select: records appended to the list that block 0 finishes alone
@@ -108,9 +106,10 @@ struct Buffers {
     int32_t *stamp = nullptr;  // [nv] iteration stamp of candidate marking (push)
     int32_t *sstamp = nullptr; // [nv] iteration stamp of the selected window (pull)
     int32_t *ndiff = nullptr;  // [nv] neighbours with another label (the boundary test is ndiff > 0)
-    int32_t *cand = nullptr;   // [nv] phase-1 claimed list / stand-alone window list
+    int32_t *cand = nullptr;   // [nv] stand-alone window list; scratch of the hub sort and the slot orders
     int32_t *win[2] = {nullptr, nullptr};  // [nv] each: selected window of the iteration (by parity)
-    int32_t *bv = nullptr, *bnew = nullptr;  // [nv] mover pairs of dmolp_lp_apply; phase-1 records
+    int32_t *bv = nullptr, *bnew = nullptr;  // [nv] mover pairs of dmolp_lp_apply; scratch (bv as cand,
+                                             // bnew: slot labels of the one-launch loop)
     int32_t *bown = nullptr;   // [nv] record slot: own label of a boundary vertex, -1 otherwise
     uint64_t *bkey = nullptr;  // [nv] record slot: selection key
     uint8_t *bsel = nullptr;   // [nv] record slot: selected
@@ -131,7 +130,7 @@ struct Buffers {
     int32_t *colh = nullptr;   // [narcs] col with a hot neighbour u written as -(hrank[u] + 2)
     int32_t *hrank = nullptr;  // [nv] rank of a hot vertex, else -1
     int32_t *hotid = nullptr;  // [kHotMax] vertex of each rank
-    uint8_t *hotlab = nullptr; // [kHotMax] label of each hot vertex, clamped to 255 (kept current by k_apply)
+    uint8_t *hotlab = nullptr; // [kHotMax] label of each hot vertex, clamped to 255 (kept current by apply_movers)
     unsigned int *degh = nullptr;  // [65536] degree histogram (hot-set threshold)
     // kept label counts (symmetric graphs, eff <= 32): vcnt[v * 32 + c] = neighbours of v with label c, for
     // every vertex with at most kLargeDeg arcs (hubs: hh); built by the run's first statistics pass and

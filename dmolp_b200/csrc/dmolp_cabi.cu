@@ -99,7 +99,7 @@ int clear_select_bins(dmolp_ctx *c) {
     return DMOLP_OK;
 }
 
-// A grid barrier of a cooperative selection that gave up waiting (its blocks are co-resident, so only a
+// A grid barrier of a cooperative kernel that gave up waiting (its blocks are co-resident, so only a
 // wait limit far below the default makes this happen): report it, and clear the barrier state and the
 // selections' counts for the next launch.
 int report_waits(dmolp_ctx *c, int to) {
@@ -107,7 +107,7 @@ int report_waits(dmolp_ctx *c, int to) {
         const cudaError_t e = c->launch_error;
         c->launch_error = cudaSuccess;
         cudaGetLastError();
-        return fail(DMOLP_ERR_CUDA, std::string("window selection launch: ") + cudaGetErrorString(e));
+        return fail(DMOLP_ERR_CUDA, std::string("cooperative launch: ") + cudaGetErrorString(e));
     }
     if (!to) return DMOLP_OK;
     // bar_count and wait_timeout are adjacent
@@ -118,7 +118,7 @@ int report_waits(dmolp_ctx *c, int to) {
     if (st2) return st2;
     sync(c);
     return fail(DMOLP_ERR_CUDA, "grid barrier " + std::to_string(to - 1) +
-                                    " of a window selection gave up waiting (wait limit " +
+                                    " of a cooperative kernel gave up waiting (wait limit " +
                                     std::to_string(c->wait_polls) + " polls)");
 }
 
@@ -1278,6 +1278,11 @@ int dmolp_phase1(dmolp_ctx *c, int k, int theta, int32_t *seeds_out, int64_t *ve
 // what counts: a mesh of 0.76 M arcs, 20 iterations 1.17 -> 0.49 ms; preferential attachment of 6.4 M arcs, 48 labels
 // 2.83 -> 1.91 ms; a skewed graph of 7.5 M arcs, 64 parts 1.36 -> 1.10 ms.  Above it the launch per step wins, with
 // its pulled candidates and hub windows instead of a stamp per arc (a skewed graph of 14 M arcs 1.29 ms, here 1.76).
+// Meshes meet the line earlier when at most 32 labels are scored: of 6.5 and 6.9 M arcs, 8 parts, 20 iterations from
+// phase-1 labels, 0.96 and 1.26 ms as launches, here 0.95 and 1.22, on a graph's first run 1.19 and 1.45, here 0.98 and
+// 1.25; from random labels, whose windows are large, 1.64 and 1.75, here 1.99 and 1.87 (first run 1.86 and 1.97, here
+// 2.03 and 1.90).  A run starts from phase-1 labels as a rule, and once per graph, so one line serves both families.
+// With 64 labels scored they take 30 to 45 % less here, from either start.
 // A run of fewer than kLoopMinIters iterations does not earn the slot orders (40 us).  Asymmetric graphs recount from
 // the arcs each iteration, and timed launches (profiling) are those of the launch per step, which a caller can also ask
 // for (dmolp_set_lp_steps).
@@ -1346,7 +1351,8 @@ int dmolp_lp_run(dmolp_ctx *c, int k, const dmolp_lp_config *cfg, dmolp_lp_resul
         if (st) return st;
         int stopped = 0;
         // Iterations in blocks: FIXED mode one block of all iterations, REF mode blocks of 8 with a check of
-        // the stop flag in between.  Each block is captured into a CUDA graph once and replayed afterwards.
+        // the stop flag in between.  A block is launched the first time, captured the second, then replayed
+        // (run_block_graph).
         const int block = cfg->mode == DMOLP_LP_MODE_REF ? 8 : std::max(1, max_iter);
         for (int t0 = 1; t0 <= max_iter; t0 += block) {
             const int cnt = std::min(block, max_iter - t0 + 1);

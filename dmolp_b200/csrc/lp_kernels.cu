@@ -1,8 +1,9 @@
 // Phase-2 label propagation on the resident CSR.  One iteration t (1-based) is a fixed sequence of
-// launches with device-side counts, so a whole run is captured once into a CUDA graph and replayed:
+// launches with device-side counts, so the second run on a graph is captured into CUDA graphs, replayed from then on
+// (the first is launched as it is; small symmetric graphs run in one launch instead, lp_loop.cu):
 //
 //   begin    penalties from the current statistics (calculatePenalties, src/phase2/phase2.cpp:158-209);
-//            counter reset (with the previous iteration's end: one k_lp_turn between iterations)
+//            counter reset (with the previous iteration's end: one turn between iterations, lp_turn)
 //   mark     stamp the previous window and its neighbours with t (expandBoundaryNodes' candidate set,
 //            src/phase2/gpu_lp_boundary.cu:195-240): thread per short row, warp per longer row; a hub's
 //            row is walked only when the hub enters or leaves the window, keeping hubwin[u] (window hubs
@@ -24,7 +25,7 @@
 //            the neighbour stays (its reverse arc is not visited) and 1 when it moves too.  Asymmetric
 //            graphs run the full statistics pass instead (computePartitionStats / computeEdgeCut,
 //            phase2.cpp:55-117, 214-253).
-//   apply    movers take their new labels
+//   apply    movers take their new labels (in the turn's launch)
 //   end      the stopping rules of run_phase2 (phase2.cpp:309-415) and the iteration record
 //
 // Floating point: penalties and scores use __d*_rn intrinsics, which the compiler never contracts into

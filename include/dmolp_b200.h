@@ -224,11 +224,11 @@ int dmolp_labels_restore(dmolp_ctx *ctx);
 int dmolp_set_profiling(dmolp_ctx *ctx, int enable);
 int dmolp_kernel_profile(dmolp_ctx *ctx, int kernel, double *total_ms, int64_t *launches, double *bytes);
 
-/* How long a grid barrier of the cooperative window selections waits before it gives up: `polls` reads of
- * its generation word (0 = the default, 2^22, about a second).  Its blocks are co-resident (cooperative
- * launch), so the default is never reached; a barrier that gives up stops the loop and every block leaves the
- * kernel, and the call returns DMOLP_ERR_CUDA naming the barrier, with the context ready for the next call.
- * No reference counterpart (the reference's kernel has no barrier).  Mainly for testing that path. */
+/* How long a grid barrier of the cooperative kernels (hub list, phase 1, slot orders, the one-launch loop, window
+ * selections) waits before it gives up: `polls` reads of its word (0 = the default, 2^22, about a second).  Its
+ * blocks are co-resident (cooperative launch), so the default is never reached; a barrier that gives up makes every
+ * block leave the kernel, and the call returns DMOLP_ERR_CUDA naming the barrier, with the context ready for the next
+ * call.  No reference counterpart (the reference's kernel has no barrier).  Mainly for testing that path. */
 int dmolp_set_wait_limit(dmolp_ctx *ctx, uint32_t polls);
 
 /* How the LP loop tests whether the resident graph is symmetric (every arc's reverse present, with the same
