@@ -30,7 +30,7 @@ struct dmolp_batch {
     std::vector<void *> allocations;
     Args a{};
     int64_t ncnt = 0;           // 16-bit label counts of the graphs that can keep them
-    bool counts_ready = false;  // allocated, or given up, by a phase 2 of the resident batch
+    bool counts_ready = false;  // allocated, or given up by a phase 2 of the resident batch
     Inst *inst = nullptr;
     int32_t *order = nullptr, *saved = nullptr, *longrow = nullptr;
     int nlong = 0;
@@ -107,10 +107,19 @@ int bsync(dmolp_batch *b) {
         if (r_) return r_;   \
     } while (0)
 
-// The kept label counts (up to 64 bytes per vertex), allocated by the first phase 2 of a batch: nothing else needs
-// them.  Without the memory no graph keeps counts, and its decisions count the rows, to the same result.
-int ensure_counts(dmolp_batch *b) {
+// The kept label counts (up to 64 bytes per vertex), which phase 2 alone needs.  The upload allocates them where memory
+// is plentiful: kCountsRoom bytes per vertex stay free, what the proposal network takes in training and to spare (on
+// 100 MB of counts an allocation in the first phase 2 cost that call 1 ms).  Otherwise they wait for the first phase 2,
+// so that a batch that is only seeded or proposed for does without them; and when they do not fit then, no graph keeps
+// counts, and its decisions count the rows, to the same result.
+constexpr size_t kCountsRoom = 4096;
+int ensure_counts(dmolp_batch *b, bool upload) {
     if (b->counts_ready) return DMOLP_OK;
+    if (upload) {
+        size_t avail = 0, total = 0;
+        BCUDA(cudaMemGetInfo(&avail, &total));
+        if (avail < (size_t)b->ncnt * sizeof(uint16_t) + kCountsRoom * (size_t)b->nv) return DMOLP_OK;
+    }
     if (b->ncnt > 0) {
         const int st = balloc(b, &b->a.cnt, (size_t)b->ncnt);
         if (st && st != DMOLP_ERR_NOMEM) return st;
@@ -467,6 +476,7 @@ int dmolp_batch_upload(dmolp_batch *b, int32_t ninst, const int64_t *vstart, con
     q.seeds_out = seeds_out;
     q.out = p1out;
     b->h_p1.assign(ninst, P1Out());
+    BTRY(ensure_counts(b, true));
     b->has_graph = true;
     return DMOLP_OK;
 }
@@ -516,7 +526,7 @@ int dmolp_batch_lp_run(dmolp_batch *b, const dmolp_lp_config *cfg, const dmolp_b
     BTRY(check_cfg(cfg));
     BCUDA(cudaSetDevice(b->device));
     const dmolp_batch_tuning t = tune ? *tune : b->tuning;
-    BTRY(ensure_counts(b));
+    BTRY(ensure_counts(b, false));
     BCUDA(cudaEventRecord(b->ev0, b->stream));
     BTRY(run_graph(b, t, *cfg));
     BCUDA(cudaEventRecord(b->ev1, b->stream));

@@ -371,9 +371,10 @@ typedef struct dmolp_mpnn dmolp_mpnn;
 int64_t dmolp_mpnn_num_params(void);           /* length of the flat FP32 parameter vector */
 int dmolp_mpnn_create(int device, dmolp_mpnn **out);  /* fixed-seed Glorot hidden layers, zero output layer */
 int dmolp_mpnn_destroy(dmolp_mpnn *m);
-/* Polls of a GEMM's MMA completion barrier before the GEMM gives up (0 = the default, 2^24 non-blocking
- * checks, a fraction of a second; far above any real MMA).  A GEMM that gives up waits (bounded) for the MMA in flight, frees its tensor memory and sets an
- * error flag: the call returns DMOLP_ERR_CUDA and the network stays usable.  Mainly for testing that path. */
+/* Polls of a GEMM's MMA completion barrier, or of the team barrier of a large graph's anchor searches, before the wait
+ * gives up (0 = the default, 2^24 non-blocking checks, a fraction of a second; far above any real wait).  A GEMM that
+ * gives up waits (bounded) for the MMA in flight and frees its tensor memory; either sets an error flag: the call
+ * returns DMOLP_ERR_CUDA and the network stays usable.  Mainly for testing that path. */
 int dmolp_mpnn_set_wait_limit(dmolp_mpnn *m, uint32_t polls);
 /* Parameters, flat FP32: per layer W [K x N] row-major then b [N]; K = 32, 128, 128; N = 64, 64, 16.
  * Setting them resets the optimiser state. */
