@@ -10,13 +10,13 @@
 // part's size alone (segment_length).  A warp sums a segment at a time in registers, to the segment's record in global
 // memory, and one warp per part adds the records in order.  So the sums' order, and with it the result, depends neither
 // on scheduling nor on the team, that is on what else is in the batch.  (Sums over whatever vertices a warp held did:
-// the team's size moved the last bits of mean and axis.)  The selection is an MSD radix select over keys (orderable float bits of the
-// projection, id) with 6-bit digits and no lists: a record is open while its leading digits are its part's
-// prefix.  A stable partition of the permutation by the part's threshold key then forms the children.
+// the team's size moved the last bits of mean and axis.)  The selection is an MSD radix select over keys (orderable
+// float bits of the projection, id) with 6-bit digits and no lists: a record is open while its leading digits are its
+// part's prefix.  A stable partition of the permutation by the part's threshold key then forms the children.
 //
 // What bounds it: passes over 32 bytes per vertex at the level's start, and the chain of about 20 barriers per
 // level.  One CTA that walked all vertices once per part took 229 ms for a skewed graph of a million vertices and
-// 32 parts; 16 CTAs over the permutation take 2.7 ms.
+// 32 parts; 16 CTAs over the permutation take 2.8 ms (2.7 with sums over whatever a warp held).
 #include <algorithm>
 #include <vector>
 
