@@ -53,10 +53,10 @@ struct SelArgs {
 };
 
 // Grid barrier (all blocks are resident: cooperative launch) on one word, arrive_and_wait; an arrival count, its reset
-// and a generation word took two more round trips to L2.  Returns false when the wait ran past `polls` polls, or another block's barrier already gave up: then
-// ctl->wait_timeout holds 1 + the id of the first barrier that gave up, the loop is stopped, and the caller's
-// block leaves the kernel at once (every block that waits at a later barrier leaves too), so the kernel
-// always ends; the host reports the timeout and clears the barrier state.
+// and a generation word took two more round trips to L2.  Returns false when the wait ran past `polls` polls, or
+// another block's barrier already gave up: then ctl->wait_timeout holds 1 + the id of the first barrier that gave up,
+// the loop is stopped, and the caller's block leaves the kernel at once (every block that waits at a later barrier
+// leaves too), so the kernel always ends; the host reports the timeout and clears the barrier state.
 __device__ __forceinline__ bool grid_sync(LpControl *ctl, unsigned int polls, int id) {
     __shared__ int s_pass;
     __syncthreads();
