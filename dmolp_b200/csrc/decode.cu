@@ -6,9 +6,10 @@
 // axis.  The axis: mean and covariance of the part in double, cyclic Jacobi on the 8x8 covariance, the
 // eigenvector of the largest eigenvalue signed so that its largest-magnitude component is positive.
 //
-// A part's vertices stay contiguous in a permutation (ascending ids), cut into segments whose length depends on the
-// part's size alone (segment_length).  A warp sums a segment at a time in registers, to the segment's record in global
-// memory, and one warp per part adds the records in order.  So the sums' order, and with it the result, depends neither
+// A part's vertices stay contiguous in a permutation (ascending ids), so each warp owns a run of it.  For the sums the
+// parts are cut into segments whose length the graph and the level alone decide (segment_length).  A warp sums a segment
+// at a time in registers, to the segment's record in global memory, and one warp per part adds the records in order.
+// So the sums' order, and with it the result, depends neither
 // on scheduling nor on the team, that is on what else is in the batch.  (Sums over whatever vertices a warp held did:
 // the team's size moved the last bits of mean and axis.)  The selection is an MSD radix select over keys (orderable
 // float bits of the projection, id) with 6-bit digits and no lists: a record is open while its leading digits are its
@@ -16,7 +17,7 @@
 //
 // What bounds it: passes over 32 bytes per vertex at the level's start, and the chain of about 20 barriers per
 // level.  One CTA that walked all vertices once per part took 229 ms for a skewed graph of a million vertices and
-// 32 parts; 16 CTAs over the permutation take 2.8 ms (2.7 with sums over whatever a warp held).
+// 32 parts; 16 CTAs over the permutation take 2.7 ms.
 #include <algorithm>
 #include <vector>
 
@@ -37,13 +38,29 @@ constexpr int kWarps = kDecThreads / 32;
 constexpr int kParts = batch::kBatchMaxK;
 constexpr int kDims = 8;
 constexpr int kTri = kDims * (kDims + 1) / 2;
-constexpr int kSeg = 512;      // vertices of a segment of a small part; multiples of it in parts of more than ...
-constexpr int kMaxSegs = 256;  // ... this many such (one per warp of the largest team)
+constexpr int kRun = 128;             // granularity of the warps' runs, in vertices; the shortest segment
 constexpr int kRecs = kWarps + kParts;  // a CTA's warps meet at most this many (warp, part) pairs
-static_assert(kSeg == kDecSeg && kTri == kDecRecord && kParts / 2 == kDecSplits, "the records' workspace");
+static_assert(kRun == kDecSeg && kTri == kDecRecord && kParts / 2 == kDecSplits, "the records' workspace");
 
-// Vertices per segment of a part of n.
-__device__ __forceinline__ int segment_length(int n) { return ((n - 1) / (kSeg * kMaxSegs) + 1) * kSeg; }
+// Vertices per segment where `split` parts of n vertices together split.  For t segments per warp of the largest team
+// the length is the shortest that leaves at most so many (a part's last segment may be short); t is chosen by the
+// level's time, t x (length / 32 + kReduce), in steps of 32 vertices: a segment's sums over the lanes cost about
+// kReduce of them.  So a large graph takes one or two segments per warp at every level, a small one segments of kRun.
+// (Lengths of 512 and more by the part's size: a graph of 28 K vertices left three of four warps without a segment of
+// the first part, its decoder 0.53 -> 0.58 ms; one length per graph: 2.76 -> 3.07 ms for a million vertices.)
+constexpr int kReduce = 6;
+__device__ __forceinline__ int segment_length(int n, int split) {
+    int best = 0x7fffffff, len = kRun;
+    for (int t = 1; t <= 4; ++t) {
+        const int m = t * kWarps * batch::kMaxTeam - split;
+        const int steps = ((n - 1) / m + 32) / 32, cost = t * (steps + kReduce);
+        if (cost < best) {
+            best = cost;
+            len = steps * 32;
+        }
+    }
+    return len < kRun ? kRun : len;
+}
 
 struct DecSmem {
     double mean[kParts][kDims], axis[kParts][kDims];
@@ -52,8 +69,8 @@ struct DecSmem {
     int hist[2][kParts * kDigits];         // zero between selections
     int lrec[kRecs];                       // selected vertices per (warp, part)
     int kp[kParts], beg[kParts], cnt[kParts], need[kParts], below[kParts], keep[kParts], fin[kParts];
-    int part[kParts], len[kParts], seg0[kParts + 1];  // splitting parts by ordinal, segment lengths, first segments
-    int nsplit, bad, inst;
+    int part[kParts], run0[kParts + 1], seg0[kParts + 1];  // splitting parts by ordinal, their first runs and segments
+    int len, nsplit, bad, inst;  // len: vertices per segment
 };
 
 __device__ __forceinline__ unsigned orderable(float x) {
@@ -102,30 +119,31 @@ __device__ void jacobi8(double (*A)[kDims], double (*V)[kDims]) {
     __syncwarp();
 }
 
-// A warp's share of a level: the segments [a, b) of the splitting parts, whose segments follow each other by ordinal.
+// A warp's share of a level: the runs [a, b) of the splitting parts, whose runs follow each other by ordinal.
 // f(ordinal, first position, last position) for each part it meets, positions in the permutation.
 template <typename F>
 __device__ __forceinline__ void for_parts(const DecSmem &sm, int a, int b, F f) {
     int o = 0;
-    while (o < sm.nsplit && sm.seg0[o + 1] <= a) ++o;
+    while (o < sm.nsplit && sm.run0[o + 1] <= a) ++o;
     for (; a < b; ++o) {
-        const int p = sm.part[o], s0 = sm.seg0[o], end = sm.beg[p] + sm.cnt[p];
-        const int z = b < sm.seg0[o + 1] ? b : sm.seg0[o + 1];
-        const int i0 = sm.beg[p] + (a - s0) * sm.len[o];
-        f(o, i0, z == sm.seg0[o + 1] ? end : sm.beg[p] + (z - s0) * sm.len[o]);
+        const int p = sm.part[o], r0 = sm.run0[o];
+        const int z = b < sm.run0[o + 1] ? b : sm.run0[o + 1];
+        const int i0 = sm.beg[p] + (a - r0) * kRun;
+        const int i1 = z == sm.run0[o + 1] ? sm.beg[p] + sm.cnt[p] : sm.beg[p] + (z - r0) * kRun;
+        f(o, i0, i1);
         a = z;
     }
 }
 
-// The same segment by segment: f(ordinal, segment, first position, last position).
+// The segments [a, b) one by one, numbered alike: f(ordinal, segment, first position, last position).
 template <typename F>
 __device__ __forceinline__ void for_segments(const DecSmem &sm, int a, int b, F f) {
     int o = 0;
     for (; a < b; ++a) {
         while (sm.seg0[o + 1] <= a) ++o;
         const int p = sm.part[o], end = sm.beg[p] + sm.cnt[p];
-        const int i0 = sm.beg[p] + (a - sm.seg0[o]) * sm.len[o];
-        f(o, a, i0, end - i0 < sm.len[o] ? end : i0 + sm.len[o]);
+        const int i0 = sm.beg[p] + (a - sm.seg0[o]) * sm.len;
+        f(o, a, i0, end - i0 < sm.len ? end : i0 + sm.len);
     }
 }
 
@@ -215,32 +233,45 @@ __device__ void run_decode(const DecodeWork &w, int ii, const Tm &tm, DecSmem &s
     }
     int cur = 0;
     for (int level = 0; level < 7; ++level, cur ^= 1) {
-        // ---- the splitting parts and their segments (by every CTA alike) ----
+        // ---- the splitting parts, their runs and segments (by every CTA alike) ----
         __syncthreads();
         if (wib == 0) {
-            int nsplit = 0, segs = 0;
+            int nsplit = 0, total = 0, runs = 0, segs = 0;
+            for (int p0 = 0; p0 < kParts; p0 += 32) {
+                const int n = sm.kp[p0 + lane] >= 2 ? sm.cnt[p0 + lane] : 0;
+                nsplit += __popc(__ballot_sync(DMOLP_FULL_MASK, n > 0));
+                total += __reduce_add_sync(DMOLP_FULL_MASK, n);
+            }
+            const int len = segment_length(total, nsplit);
+            nsplit = 0;
             for (int p0 = 0; p0 < kParts; p0 += 32) {
                 const int p = p0 + lane;
                 const bool split = sm.kp[p] >= 2 && sm.cnt[p] > 0;
-                const int len = split ? segment_length(sm.cnt[p]) : 1, r = split ? (sm.cnt[p] - 1) / len + 1 : 0;
-                int incl = r;
+                const int r = split ? (sm.cnt[p] - 1) / kRun + 1 : 0, g = split ? (sm.cnt[p] - 1) / len + 1 : 0;
+                int ir = r, ig = g;
                 for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(DMOLP_FULL_MASK, incl, o);
-                    if (lane >= o) incl += y;
+                    const int yr = __shfl_up_sync(DMOLP_FULL_MASK, ir, o), yg = __shfl_up_sync(DMOLP_FULL_MASK, ig, o);
+                    if (lane >= o) {
+                        ir += yr;
+                        ig += yg;
+                    }
                 }
                 const unsigned m = __ballot_sync(DMOLP_FULL_MASK, split);
                 if (split) {
                     const int o = nsplit + __popc(m & ((1u << lane) - 1));
                     sm.part[o] = p;
-                    sm.len[o] = len;
-                    sm.seg0[o] = segs + incl - r;
+                    sm.run0[o] = runs + ir - r;
+                    sm.seg0[o] = segs + ig - g;
                 }
                 nsplit += __popc(m);
-                segs += __shfl_sync(DMOLP_FULL_MASK, incl, 31);
+                runs += __shfl_sync(DMOLP_FULL_MASK, ir, 31);
+                segs += __shfl_sync(DMOLP_FULL_MASK, ig, 31);
             }
             if (lane == 0) {
                 sm.nsplit = nsplit;
+                sm.run0[nsplit] = runs;
                 sm.seg0[nsplit] = segs;
+                sm.len = len;
             }
         }
         for (int p = threadIdx.x; p < kParts; p += kDecThreads) {
@@ -254,12 +285,14 @@ __device__ void run_decode(const DecodeWork &w, int ii, const Tm &tm, DecSmem &s
         any = __any_sync(DMOLP_FULL_MASK, any);
         __syncthreads();
         if (!any) break;
-        const int nsplit = sm.nsplit, segs = sm.seg0[nsplit];
-        const int per = segs > 0 ? (segs + team_warps - 1) / team_warps : 1;
-        const int a = min(wid * per, segs), b = min(a + per, segs);
+        const int nsplit = sm.nsplit, runs = sm.run0[nsplit], segs = sm.seg0[nsplit];
+        const int per = runs > 0 ? (runs + team_warps - 1) / team_warps : 1;
+        const int a = min(wid * per, runs), b = min(a + per, runs);
+        const int sper = (segs + team_warps - 1) / team_warps;
+        const int sa = min(wid * sper, segs), sb = min(sa + sper, segs);
         const int32_t *const pm = perm[cur];
         // ---- means ----
-        for_segments(sm, a, b, [&](int, int seg, int i0, int i1) {
+        for_segments(sm, sa, sb, [&](int, int seg, int i0, int i1) {
             double acc[kDims];
 #pragma unroll
             for (int d = 0; d < kDims; ++d) acc[d] = 0.0;
@@ -280,7 +313,7 @@ __device__ void run_decode(const DecodeWork &w, int ii, const Tm &tm, DecSmem &s
         }
         tm.sync();
         // ---- covariances (upper triangles), principal axes ----
-        for_segments(sm, a, b, [&](int o, int seg, int i0, int i1) {
+        for_segments(sm, sa, sb, [&](int o, int seg, int i0, int i1) {
             double acc[kTri], mu[kDims];
 #pragma unroll
             for (int i = 0; i < kTri; ++i) acc[i] = 0.0;
@@ -390,7 +423,7 @@ __device__ void run_decode(const DecodeWork &w, int ii, const Tm &tm, DecSmem &s
             const uint64_t cut = sm.cut[p];
             // selected vertices of the part in front of this share: its earlier warps' counts
             int left = 0;
-            for (int x = sm.seg0[o] / per + lane; x < wid; x += 32)
+            for (int x = sm.run0[o] / per + lane; x < wid; x += 32)
                 left += *tm.at(&sm.lrec[x % kWarps + o], x / kWarps);
             left = __reduce_add_sync(DMOLP_FULL_MASK, left);
             const int nl = (int)(((long long)sm.cnt[p] * kl) / sm.kp[p]);

@@ -96,9 +96,9 @@ struct FeatWork {
 int features(const FeatWork &w, const batch::View &b, cudaStream_t s);  // returns a CUDA error code (0 = ok)
 void features_to_input(const float *Xf, int nv, __nv_bfloat16 *X, int ldx, int num_sms, cudaStream_t s);
 
-// The decoder's records: kDecRecord sums per segment of at least kDecSeg vertices of a part that splits, at most
-// kDecSplits such parts at once.  A graph's records start at decode_record of its first vertex and its index.
-constexpr int kDecSeg = 512, kDecRecord = 36, kDecSplits = batch::kBatchMaxK / 2;
+// The decoder's records: kDecRecord sums per segment of a part that splits, all but a part's last of at least kDecSeg
+// vertices, at most kDecSplits such parts at once.  A graph's records start at decode_record of its first vertex and its index.
+constexpr int kDecSeg = 128, kDecRecord = 36, kDecSplits = batch::kBatchMaxK / 2;
 __host__ __device__ __forceinline__ size_t decode_record(int64_t vbase, int inst) {
     return (size_t)(vbase / kDecSeg) + (size_t)kDecSplits * inst;
 }

@@ -1,5 +1,5 @@
 """The decoder's labels of a graph depend on the graph and its coordinates, not on the batch it is in: a team of CTAs
-sums a part's mean and covariance in an order that the part's size alone decides.  The coordinates are closed under
+sums a part's mean and covariance in an order that the graph and the part alone decide.  The coordinates are closed under
 exchange and signs of two axes, so the principal axis is decided by the last bits of the sums."""
 import numpy as np
 import pytest
